@@ -19,7 +19,7 @@ constexpr int kProfPad = 32;
 // many column steps (strips x (width + R - 1)) is swept as paired strips.
 constexpr uint32_t kPairStepsDefault = 2048;
 constexpr uint32_t kLongStepsNever = 0xFFFFFFFFu;
-constexpr uint32_t kLongStepsAuto = 0xFFFFFFFEu;  // from the batch's cells per lane, at least kLongStepsSmall
+constexpr uint32_t kLongStepsAuto = 0xFFFFFFFEu;  // from the batch's cells per lane (long_steps_for)
 constexpr uint32_t kLongStepsSmall = 2048;
 constexpr uint32_t kLongStepsDefault = kLongStepsAuto;
 // Residue code used for positions outside a window or a query: its profile
@@ -102,6 +102,36 @@ struct GenericArgs {
     int go, ge;
     int32_t* scores;
 };
+// The anti-diagonal kernel (band_wave.cu): classes of jobs by lanes and band
+// indices per lane, widest first.
+constexpr int kWaveClasses = 7;
+constexpr int kWaveMaxWidth = 1024;  // 32 lanes x 32 band indices
+constexpr int kWaveRowBytes = 52;    // row pitch of its score table (QuerySet::qrow holds row offsets)
+// Class of a band of width w <= kWaveMaxWidth: 32 lanes of 32, 16, 8 and 4
+// band indices, then 16, 9 and 8 lanes of 4.  Nine lanes (three jobs per
+// warp) take the prefilter band of a seed hit, 2 x 16 + 1 wide, which sixteen
+// would leave half empty.
+__host__ __device__ inline int wave_class(int64_t w) {
+    return w > 512 ? 0 : w > 256 ? 1 : w > 128 ? 2 : w > 64 ? 3 : w > 36 ? 4 : w > 32 ? 5 : 6;
+}
+struct WaveArgs {
+    const uint8_t* res;
+    const uint32_t* qrow;    // per batch position: table row offset | bias << 16
+    const int32_t* matrix;   // 24 x 24
+    const uint64_t* qoffs;
+    const saber_band_job* jobs;
+    const uint32_t* order;   // sorted job indices
+    const uint32_t* skip0;   // device counts of leading entries of order to skip, or null
+    const uint32_t* skip1;
+    const uint32_t* counts;  // jobs per class
+    uint32_t* task_counter;
+    int go, ge;
+    int32_t* scores;
+    uint32_t* rescue;
+    uint32_t* rescue_count;
+};
+cudaError_t launch_band_wave(unsigned sm_count, cudaStream_t s, const WaveArgs& a);
+
 // Allocation-free entry point (noalloc.cu).
 constexpr int32_t kNoAllocMaxBandWidth = 4096;
 struct NoAllocArgs {

@@ -1,0 +1,269 @@
+// Banded affine-gap Smith-Waterman, one job on 8, 9, 16 or 32 lanes (int16
+// pairs): the jobs whose sweep in one lane of k_band_fast would outlast the
+// rest of the batch, and narrow bands.  Semantics as in band_kernels.cu.
+//
+// The band is swept along anti-diagonals s = 2 i + k of its (row i, band
+// index k = j - i - lo) coordinates.  A lane holds 4 J consecutive band
+// indices k0 = 4 J l ..: the even ones in J registers of pairs (k, k + 2),
+// the odd ones in J more.  The cells of one anti-diagonal have the parity of
+// s, so an even step updates the even registers from the odd ones and the
+// other way round:
+//   left neighbour (i, k - 1)    at s - 1, the other parity
+//   upper neighbour (i - 1, k + 1) at s - 1, the other parity
+//   diagonal (i - 1, k)          at s - 2, the same register
+// so every lane works on every step whatever the band's width, one warp
+// shuffle per step crosses lanes, and nothing goes through memory.  A job
+// takes 2 rows + w steps, against (strips x (w + 15)) steps of 16 dependent
+// rows in one lane of the strip kernel.
+//
+// A lane's rows at one step are i0, i0 - 1, ..., i0 - 2J + 1 and its columns
+// c0 .. c0 + 2J; both windows advance by one per two steps, so one query
+// letter and one subject letter enter per lane and two steps (fetched four
+// pairs of steps ahead).  Scores come from the 24 x 24 matrix in shared
+// memory (int16, S + go) plus the packed query bias of the row pair.
+//
+// Bound: L1 wavefronts of the score gathers (95 % busy at 100 k jobs, 2.75
+// wavefronts per gather; ALU pipe 68 %), 1.3e12 cells/s, half the strip
+// kernel's rate at a full device but reached from a few thousand jobs on.
+// One GB300: 3,001 host jobs (half-widths 4..64) 1.78 -> 0.28 ms a call, 40
+// full windows of a 310-residue query 0.86 -> 0.38 ms, 2 x 3,662 kilobase DNA
+// bands 16.5 -> 5.4 ms of scoring.
+//
+// Cells left of column 0 or above row 0 hold H = 0 and E, F <= 0 from the
+// initial state on (their score is the sentinel), which is what the
+// recurrence reads there; cells past the last row or column hold values below
+// the optimum and feed no cell of the window; cells past the band (k >= w in
+// the last lanes) are held at H = 0 by a mask, so that neither E nor F carries
+// a score across the band's edge.
+#include "band_common.cuh"
+
+#include <cuda_runtime.h>
+
+namespace saber {
+
+constexpr int kWaveRow = kWaveRowBytes;   // bytes per row of the score table (26 entries)
+constexpr int kWaveSent = 24;             // row / column of the sentinel score
+constexpr unsigned kWaveThreads = 128;
+constexpr int kWaveAhead = 4;             // pairs of steps between a letter's load and its use
+
+__device__ __forceinline__ uint32_t wv_prmt(uint32_t x, uint32_t y, uint32_t sel) { return __byte_perm(x, y, sel); }
+__device__ __forceinline__ uint32_t wv_pk2(int v) { return (uint32_t)(uint16_t)(int16_t)v * 0x10001u; }
+
+// Row word of query position i: byte offset of its table row | bias << 16;
+// the sentinel row outside [0, m).
+__device__ __forceinline__ uint32_t wv_row(const uint32_t* __restrict__ qrow, int i, int m) {
+    return (unsigned)i < (unsigned)m ? __ldg(qrow + i) : (uint32_t)(kWaveSent * kWaveRow);
+}
+// Residue code of window column c, the sentinel code outside [0, n).
+__device__ __forceinline__ uint32_t wv_col(const uint8_t* __restrict__ win, int c, int n) {
+    return (unsigned)c < (unsigned)n ? (uint32_t)__ldg(win + c) : (uint32_t)kWaveSent;
+}
+
+// Jobs [task * 32 / L, ...) of one (L, J) class of the sorted list, one per
+// group of L lanes.
+template <int L, int J>
+__device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __restrict__ list, uint32_t njobs,
+                                          uint32_t task, int lane, const uint8_t* tab) {
+    constexpr int G = 32 / L;
+    const int gl = lane % L;
+    const uint32_t pos = task * G + (uint32_t)(lane / L);
+    const bool has = pos < njobs && lane < G * L;
+    uint32_t jid = 0;
+    int m = 0, n = 0, lo = 0, w = 0, s0 = 0, nit = 0;
+    const uint32_t* qrow = a.qrow;
+    const uint8_t* win = a.res;
+    if (has) {
+        jid = list[pos];
+        const saber_band_job jj = a.jobs[jid];
+        const uint64_t q0 = a.qoffs[jj.query];
+        const int64_t mm = (int64_t)(a.qoffs[jj.query + 1] - q0);
+        int64_t l64 = jj.band_lo, h64 = jj.band_hi;
+        w = (int)clip_band(mm, jj.win_len, l64, h64);
+        m = (int)mm;
+        n = (int)jj.win_len;
+        lo = (int)l64;
+        qrow += q0;
+        win += jj.win_begin;
+        // anti-diagonals of the cells inside the window
+        const int first = h64 < 0 ? (int)-h64 : 0;
+        int last = n - 1 - lo;
+        if (last > m - 1) last = m - 1;
+        const int s_min = 2 * first + (-lo - first > 0 ? -lo - first : 0);
+        const int k_end = n - 1 - lo - last;
+        const int s_max = 2 * last + (k_end < w - 1 ? k_end : w - 1);
+        s0 = s_min & ~1;
+        nit = (s_max - s0) / 2 + 1;
+    }
+    const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)nit);
+    const int go = a.go;
+    const uint32_t ngo2 = wv_pk2(-go), nge2 = wv_pk2(-a.ge), neg2 = wv_pk2(kNeg16);
+    int i0 = s0 / 2 - 2 * J * gl;
+    int c0 = s0 / 2 + 2 * J * gl + lo;
+
+    uint32_t Ge[J], Go[J], E[J], F[J], keep_e[J], keep_o[J], R[2 * J], C[2 * J + 1], B[J];
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+        Ge[j] = Go[j] = ngo2;
+        E[j] = F[j] = neg2;
+        const int k = 4 * J * gl + 4 * j;
+        keep_e[j] = (k < w ? 0xFFFFu : 0u) | (k + 2 < w ? 0xFFFF0000u : 0u);
+        keep_o[j] = (k + 1 < w ? 0xFFFFu : 0u) | (k + 3 < w ? 0xFFFF0000u : 0u);
+        const uint32_t ra = wv_row(qrow, i0 - 2 * j, m), rb = wv_row(qrow, i0 - 2 * j - 1, m);
+        R[2 * j] = ra & 0xFFFFu;
+        R[2 * j + 1] = rb & 0xFFFFu;
+        B[j] = wv_prmt(ra, rb, 0x7632);
+    }
+#pragma unroll
+    for (int r = 0; r <= 2 * J; r++) C[r] = 2 * wv_col(win, c0 + r, n);
+    // letters of the next kWaveAhead pairs of steps
+    uint32_t qn[kWaveAhead], sn[kWaveAhead];
+#pragma unroll
+    for (int t = 0; t < kWaveAhead; t++) {
+        qn[t] = wv_row(qrow, i0 + 1 + t, m);
+        sn[t] = wv_col(win, c0 + 2 * J + 1 + t, n);
+    }
+    i0 += kWaveAhead;
+    c0 += 2 * J + kWaveAhead;
+    uint32_t best = 0;
+    auto sub = [&](uint32_t ra, uint32_t ca, uint32_t rb, uint32_t cb, uint32_t bias) {
+        const uint32_t x = *reinterpret_cast<const uint16_t*>(tab + ra + ca);
+        const uint32_t y = *reinterpret_cast<const uint16_t*>(tab + rb + cb);
+        return __vadd2(wv_prmt(x, y, 0x5410), bias);
+    };
+    for (int it = 0; it < nmax; it += kWaveAhead) {
+#pragma unroll
+        for (int t = 0; t < kWaveAhead; t++) {
+            // even step: E, F come in from the odd band indices
+            uint32_t left = __shfl_up_sync(0xffffffffu, E[J - 1], 1);
+            if (gl == 0) left = neg2;
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                const uint32_t own = E[j];
+                const uint32_t Ein = wv_prmt(left, own, 0x5432);
+                left = own;
+                const uint32_t Fin = F[j];
+                const uint32_t ds = __vadd2(Ge[j], sub(R[2 * j], C[2 * j], R[2 * j + 1], C[2 * j + 1], B[j]));
+                const uint32_t H = __vimax3_s16x2_relu(Ein, Fin, ds) & keep_e[j];
+                const uint32_t Gv = __vadd2(H, ngo2);
+                Ge[j] = Gv;
+                E[j] = __viaddmax_s16x2(Ein, nge2, Gv);
+                F[j] = __viaddmax_s16x2(Fin, nge2, Gv);
+                best = __vmaxs2(best, H);
+            }
+            // odd step: from the even ones
+            uint32_t down = __shfl_down_sync(0xffffffffu, F[0], 1);
+            if (gl == L - 1) down = neg2;
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                const uint32_t Ein = E[j];
+                const uint32_t Fin = wv_prmt(F[j], j + 1 < J ? F[j + 1 < J ? j + 1 : j] : down, 0x5432);
+                const uint32_t ds = __vadd2(Go[j], sub(R[2 * j], C[2 * j + 1], R[2 * j + 1], C[2 * j + 2], B[j]));
+                const uint32_t H = __vimax3_s16x2_relu(Ein, Fin, ds) & keep_o[j];
+                const uint32_t Gv = __vadd2(H, ngo2);
+                Go[j] = Gv;
+                E[j] = __viaddmax_s16x2(Ein, nge2, Gv);
+                F[j] = __viaddmax_s16x2(Fin, nge2, Gv);
+                best = __vmaxs2(best, H);
+            }
+            // the windows advance by one row and one column
+#pragma unroll
+            for (int j = J - 1; j > 0; j--) B[j] = wv_prmt(B[j - 1], B[j], 0x5432);
+            B[0] = wv_prmt(qn[t], B[0], 0x5432);
+#pragma unroll
+            for (int r = 2 * J - 1; r > 0; r--) R[r] = R[r - 1];
+            R[0] = qn[t] & 0xFFFFu;
+#pragma unroll
+            for (int r = 0; r < 2 * J; r++) C[r] = C[r + 1];
+            C[2 * J] = 2 * sn[t];
+            i0++;
+            c0++;
+            qn[t] = wv_row(qrow, i0, m);
+            sn[t] = wv_col(win, c0, n);
+        }
+    }
+    int sc = max((int)(best & 0xFFFFu), (int)(best >> 16));  // H >= 0
+    // the group's maximum in its first lane (lanes past the group's end add
+    // nothing: their values are masked out)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const int v = __shfl_down_sync(0xffffffffu, sc, o);
+        if (o < L && gl + o < L) sc = max(sc, v);
+    }
+    if (has && gl == 0) {
+        if (sc >= kLimit16) a.rescue[atomicAdd(a.rescue_count, 1u)] = jid;
+        else a.scores[jid] = sc;
+    }
+}
+
+// Persistent warps over warp tasks of the classes, widest bands first; within
+// a class the list is largest first.
+__global__ void __launch_bounds__(kWaveThreads, 4) k_band_wave(WaveArgs a) {
+    __shared__ __align__(4) int16_t tab[25 * kWaveRow / 2];
+    for (int t = threadIdx.x; t < 25 * (kWaveRow / 2); t += blockDim.x) {
+        const int r = t / (kWaveRow / 2), c = t - r * (kWaveRow / 2);
+        tab[t] = r < 24 && c < 24 ? (int16_t)(a.matrix[r * 24 + c] + a.go) : (int16_t)kSent16;
+    }
+    __syncthreads();
+    const uint8_t* tb = reinterpret_cast<const uint8_t*>(tab);
+    const int lane = threadIdx.x & 31;
+    uint32_t n[kWaveClasses], tasks[kWaveClasses], total = 0;
+#pragma unroll
+    for (int c = 0; c < kWaveClasses; c++) {
+        n[c] = a.counts[c];
+        const uint32_t per = c < 4 ? 1u : c - 2u;  // jobs per warp
+        tasks[c] = (n[c] + per - 1) / per;
+        total += tasks[c];
+    }
+    const uint32_t* list = a.order + (a.skip0 ? *a.skip0 : 0u) + (a.skip1 ? *a.skip1 : 0u);
+    for (;;) {
+        uint32_t t = 0;
+        if (lane == 0) t = atomicAdd(a.task_counter, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= total) break;
+        const uint32_t* l = list;
+        if (t < tasks[0]) {
+            wave_task<32, 8>(a, l, n[0], t, lane, tb);
+            continue;
+        }
+        t -= tasks[0];
+        l += n[0];
+        if (t < tasks[1]) {
+            wave_task<32, 4>(a, l, n[1], t, lane, tb);
+            continue;
+        }
+        t -= tasks[1];
+        l += n[1];
+        if (t < tasks[2]) {
+            wave_task<32, 2>(a, l, n[2], t, lane, tb);
+            continue;
+        }
+        t -= tasks[2];
+        l += n[2];
+        if (t < tasks[3]) {
+            wave_task<32, 1>(a, l, n[3], t, lane, tb);
+            continue;
+        }
+        t -= tasks[3];
+        l += n[3];
+        if (t < tasks[4]) {
+            wave_task<16, 1>(a, l, n[4], t, lane, tb);
+            continue;
+        }
+        t -= tasks[4];
+        l += n[4];
+        if (t < tasks[5]) {
+            wave_task<9, 1>(a, l, n[5], t, lane, tb);
+            continue;
+        }
+        t -= tasks[5];
+        l += n[5];
+        wave_task<8, 1>(a, l, n[6], t, lane, tb);
+    }
+}
+
+cudaError_t launch_band_wave(unsigned sm_count, cudaStream_t s, const WaveArgs& a) {
+    k_band_wave<<<sm_count * 4, kWaveThreads, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+}  // namespace saber

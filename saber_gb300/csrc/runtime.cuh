@@ -82,6 +82,7 @@ struct QuerySet {
     std::vector<uint32_t> pmpad; // host copy of the profile row strides
     DevBuf codes, offsets, bias, prof, prof_off, prof_mpad;
     DevBuf prof8;              // int8 copy of prof, valid when p8
+    DevBuf qrow;               // the anti-diagonal kernel's row words, one per position
     uint64_t prof_elems = 0;   // entries of prof
     int bias_min = 0, bias_max = 0;
     bool has = false;
@@ -106,6 +107,7 @@ struct GraphKey {
     uint32_t pair_steps, nq, long_steps;
     const void* ptrs[16];
     const void* prof8;
+    const void *qrow, *matrix;
     bool operator==(const GraphKey& o) const { return std::memcmp(this, &o, sizeof(GraphKey)) == 0; }
 };
 struct GraphEntry {

@@ -56,7 +56,8 @@ __global__ void k_canon(uint8_t* __restrict__ r, uint64_t n) {
 __global__ void k_profile(const uint8_t* __restrict__ codes, const uint64_t* __restrict__ qoffs,
                           const int8_t* __restrict__ bias, const int32_t* __restrict__ matrix,
                           const uint64_t* __restrict__ prof_off, const uint32_t* __restrict__ prof_mpad,
-                          int go, int16_t* __restrict__ prof, int8_t* __restrict__ prof8) {
+                          int go, int16_t* __restrict__ prof, int8_t* __restrict__ prof8,
+                          uint32_t* __restrict__ qrow) {
     const uint32_t q = blockIdx.x;
     const uint64_t q0 = qoffs[q];
     const int m = (int)(qoffs[q + 1] - q0);
@@ -73,6 +74,12 @@ __global__ void k_profile(const uint8_t* __restrict__ codes, const uint64_t* __r
         }
         P[t] = (int16_t)(v + go);
         if (prof8) prof8[prof_off[q] + t] = real ? (int8_t)(v + go) : (int8_t)-128;
+    }
+    // the anti-diagonal kernel's row words: table row offset | bias << 16
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const int qc = codes[q0 + i];
+        qrow[q0 + i] = (uint32_t)(kWaveRowBytes * (qc < 24 ? qc : 22)) |
+                       ((uint32_t)(uint16_t)(int16_t)(bias ? (int)bias[q0 + i] : 0) << 16);
     }
 }
 
@@ -101,19 +108,25 @@ __global__ void k_job_wmax(const saber_band_job* __restrict__ jobs, uint64_t njo
     }
 }
 
+constexpr int kCounts = 32;  // words of the counts buffer
+
 // stats layout (uint64): 0 cells, 1 wmax of the R-row class, 2 wmax of the
 //   int32 class, 3 bad job count, 4 cells of the packed classes, 5 wmax of
 //   the 8-row class
 // counts layout (uint32): 0 jobs in the R-row class (paired ones included),
 //   1 int32 class, 4 empty, 5 int32 list length (class + rescued), 6 task
 //   counter of the R-row launch, 7 jobs in the 8-row class, 8 task counter of
-//   the 8-row launch, 9 paired jobs of the R-row class
+//   the 8-row launch, 9 paired jobs of the R-row class, 10..16 jobs in the
+//   anti-diagonal kernel's classes, 17 their sum, 18 its task counter, 19 the
+//   narrow bands among its jobs
 //
 // Classes (the top two key bits, so the sort makes them contiguous):
 //   0: width >= R (R = the handle's strip rows), packed int16 kernel with R rows
 //   1: 8 <= width < R when R = 16, packed int16 kernel with 8 rows
 //   2: narrower bands, out-of-range sizes and sweeps longer than long_steps
-//      column steps in one lane: the warp-per-job int32 kernel, largest first
+//      column steps in one lane: the anti-diagonal int16 kernel by its classes
+//      (bits 58..60), then (bit 61) the bands too wide for it: the
+//      warp-per-job int32 kernel; largest first
 //   3: empty jobs (score 0, written here)
 // Packed-class keys order jobs by (strips, width, query) so that the 64
 // consecutive jobs of a warp task share their loop counts and widths; within
@@ -126,7 +139,7 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
                            unsigned long long* __restrict__ stats) {
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint64_t cells = 0, fcells = 0;
-    uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, cp = 0, bad = 0;
+    uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, cp = 0, bad = 0, cw[kWaveClasses] = {}, cn = 0;
     unsigned long long w0 = 0, w1 = 0, w2 = 0;
     // padded launches (captured graphs): entries past the real job count sort
     // last as empty jobs and are neither scored nor counted
@@ -180,10 +193,19 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
             if ((uint64_t)ns * (uint64_t)span > long_steps) cls = 2;
         }
         if (cls == 2) {
-            // largest first, so that the warps' static share ends together
-            const uint64_t sz = jc >> 4 < 0x7FFFFFFFull ? jc >> 4 : 0x7FFFFFFFull;
-            keys[t] = (2ull << 62) | ((0x7FFFFFFFull - sz) << 31) | t;
-            c2++;
+            const uint64_t sz = jc >> 4 < 0x7FFFFFFull ? jc >> 4 : 0x7FFFFFFull;
+            const uint64_t low = ((0x7FFFFFFull - sz) << 31) | t;
+            if (w <= kWaveMaxWidth && m < (1 << 28) && j.win_len < (1u << 28)) {
+                const int wc = wave_class(w);
+#pragma unroll
+                for (int k = 0; k < kWaveClasses; k++) cw[k] += wc == k;
+                if (w < kStripRowsMin) cn++;
+                else fcells += jc;
+                keys[t] = (2ull << 62) | ((uint64_t)wc << 58) | low;
+            } else {
+                keys[t] = (2ull << 62) | (1ull << 61) | low;
+                c2++;
+            }
             w2 = max(w2, (unsigned long long)w);
         } else {
             // within (strips, width): jobs ordered by the first strip's
@@ -210,8 +232,8 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
     // block totals in shared memory, then one global atomic per counter and block
     __shared__ unsigned long long b_sum[4];  // cells, bad, fast cells, unused
     __shared__ unsigned long long b_max[3];  // w0, w2, w1
-    __shared__ uint32_t b_cnt[5];            // c0, c1, c2, c3, paired
-    if (threadIdx.x < 5) b_cnt[threadIdx.x] = 0;
+    __shared__ uint32_t b_cnt[6 + kWaveClasses];  // c0, c1, c2, c3, paired, narrow, anti-diagonal classes
+    if (threadIdx.x < 6 + kWaveClasses) b_cnt[threadIdx.x] = 0;
     if (threadIdx.x < 4) {
         b_sum[threadIdx.x] = 0;
         if (threadIdx.x < 3) b_max[threadIdx.x] = 0;
@@ -222,6 +244,9 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
     c2 = __reduce_add_sync(0xffffffffu, c2);
     c3 = __reduce_add_sync(0xffffffffu, c3);
     cp = __reduce_add_sync(0xffffffffu, cp);
+    cn = __reduce_add_sync(0xffffffffu, cn);
+#pragma unroll
+    for (int k = 0; k < kWaveClasses; k++) cw[k] = __reduce_add_sync(0xffffffffu, cw[k]);
     bad = __reduce_add_sync(0xffffffffu, bad);
     for (int o = 16; o > 0; o >>= 1) {
         cells += __shfl_xor_sync(0xffffffffu, cells, o);
@@ -236,6 +261,10 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
         atomicAdd(&b_cnt[2], c2);
         atomicAdd(&b_cnt[3], c3);
         atomicAdd(&b_cnt[4], cp);
+        atomicAdd(&b_cnt[5], cn);
+#pragma unroll
+        for (int k = 0; k < kWaveClasses; k++)
+            if (cw[k]) atomicAdd(&b_cnt[6 + k], cw[k]);
         atomicAdd(&b_sum[0], (unsigned long long)cells);
         atomicAdd(&b_sum[1], (unsigned long long)bad);
         atomicAdd(&b_sum[2], (unsigned long long)fcells);
@@ -250,6 +279,13 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
         atomicAdd(&counts[1], b_cnt[2]);
         atomicAdd(&counts[4], b_cnt[3]);
         atomicAdd(&counts[9], b_cnt[4]);
+        atomicAdd(&counts[19], b_cnt[5]);
+        uint32_t nw = 0;
+        for (int k = 0; k < kWaveClasses; k++) {
+            if (b_cnt[6 + k]) atomicAdd(&counts[10 + k], b_cnt[6 + k]);
+            nw += b_cnt[6 + k];
+        }
+        if (nw) atomicAdd(&counts[17], nw);
         atomicAdd(&stats[0], b_sum[0]);
         atomicMax(&stats[1], b_max[0]);
         atomicMax(&stats[2], b_max[1]);
@@ -264,22 +300,31 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
 // the scoring pipeline (device-resident jobs and scores)
 // ---------------------------------------------------------------------------
 // The long-job threshold of a call.  In the automatic mode a one-lane sweep
-// goes to the warp-pipelined int32 kernel when it is longer than about four
-// times the sweep steps each int16 lane gets if the batch's cells were
-// spread evenly (a lane sweeps 32 cells per step), as a power of two, at
-// least kLongStepsSmall: such a job would otherwise set the launch's length
-// while most lanes are done.  Measured on one GB300 (threshold -> result):
-// the blastn batch (26.8 k kilobase regions, about 6.9 k steps per lane)
-// 2048 / 16384 / 32768 / none -> scoring 80 / 61 / 56 / 82 ms; the 1 M-job
-// microbench (about 11.6 k) 16384 / 65536 / none -> 8.66 / 8.71 / 8.67 ms;
-// the 11,000-query protein search (about 60 k) 32768 / none -> 64.1 /
-// 64.1 ms of device scoring.
+// goes to the anti-diagonal kernel when it is longer than 1.25 times the
+// sweep steps each lane of the strip kernel gets if the batch's cells were
+// spread evenly (a lane sweeps 32 cells per step), rounded up to a power of
+// two: such a job would set the launch's length while most lanes are done.
+// A batch of fewer than kLoadSmall steps per lane cannot keep the strip
+// kernel's lanes busy (its longest sweeps take as long as the whole batch)
+// and goes to the anti-diagonal kernel as a whole.  Scoring time on one GB300
+// by threshold 0 / 2048 / 4096 / 8192 / 16384 / none, bands half 8..128 wide,
+// by steps per lane:
+//      84 (10 k jobs)    0.28 / 1.13 / 1.79 / 3.24 / 3.30 / 3.35 ms
+//     883 (100 k)        1.69 / 2.05 / 2.34 / 3.24 / 3.85 / 3.89
+//    1751 (200 k)        3.21 / 2.85 / 2.66 / 3.56 / 4.06 / 4.19
+//    2641 (300 k)        4.77 / 3.87 / 3.58 / 3.89 / 4.59 / 4.50
+//    4374 (500 k)        7.82 / 5.87 / 4.94 / 4.84 / 5.29 / 5.27
+//    8750 (1 M)         15.48 / 10.8 / 8.80 / 8.59 / 8.16 / 8.21
+// and 11,000-query searches (30 k steps per lane) 131 / 65.0 / 64.1 / 64.1 /
+// 63.7 / 63.8 ms.
+constexpr uint64_t kLoadSmall = 1500;
 static uint32_t long_steps_for(const saber_gpu* h, uint64_t cells) {
     if (h->long_steps != kLongStepsAuto) return h->long_steps;
     const uint64_t lanes = (uint64_t)h->sm_count * band_fast_blocks_per_sm(h->strip_rows, false) * 256;
     const uint64_t load = cells / 32 / (lanes ? lanes : 1);
+    if (load < kLoadSmall) return 0;
     uint64_t t = kLongStepsSmall;
-    while (t < 4 * load && t < (1ull << 30)) t <<= 1;
+    while (t < load + load / 4 && t < (1ull << 30)) t <<= 1;
     return (uint32_t)t;
 }
 
@@ -301,6 +346,27 @@ static int jobs_cells(saber_gpu* h, const QuerySet& qs, const saber_band_job* d_
     return SABER_OK;
 }
 
+static WaveArgs wave_args(const Scheme& sch, const Dataset& ds, const saber_band_job* d_jobs, const uint32_t* order,
+                          uint32_t* counts, int32_t* d_scores, uint32_t* list) {
+    WaveArgs a;
+    a.res = ds.res.as<uint8_t>();
+    a.qrow = ds.qs.qrow.as<uint32_t>();
+    a.matrix = sch.d_matrix.as<int32_t>();
+    a.qoffs = ds.qs.offsets.as<uint64_t>();
+    a.jobs = d_jobs;
+    a.order = order;
+    a.skip0 = counts + 0;
+    a.skip1 = counts + 7;
+    a.counts = counts + 10;
+    a.task_counter = counts + 18;
+    a.go = sch.go;
+    a.ge = sch.ge;
+    a.scores = d_scores;
+    a.rescue = list;
+    a.rescue_count = counts + 5;
+    return a;
+}
+
 static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, const saber_band_job* d_jobs,
                           uint64_t njobs, int32_t* d_scores, saber_score_stats* st) {
     if (!sch.has) return fail(h, SABER_ERR_STATE, "no scoring scheme set");
@@ -319,12 +385,12 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     CUALLOC(h, h->keys_out, njobs * 8);
     CUALLOC(h, h->vals_in, njobs * 4);
     CUALLOC(h, h->vals_out, njobs * 4);
-    CUALLOC(h, h->counts, 16 * 4);
+    CUALLOC(h, h->counts, kCounts * 4);
     CUALLOC(h, h->stats, 8 * 8);
     CUALLOC(h, h->list, njobs * 4);
     uint32_t* counts = h->counts.as<uint32_t>();
     unsigned long long* stats = h->stats.as<unsigned long long>();
-    CU(h, cudaMemsetAsync(counts, 0, 16 * 4, s));
+    CU(h, cudaMemsetAsync(counts, 0, kCounts * 4, s));
     CU(h, cudaMemsetAsync(stats, 0, 8 * 8, s));
 
     const QuerySet& qs = ds.qs;
@@ -362,19 +428,19 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     local.library_launches += 9;  // onesweep radix sort: histogram + 8 digit passes
 
     // one small read-back: class counts and widths size the scratch
-    uint32_t hc[10];
+    uint32_t hc[20];
     unsigned long long hs[6];
-    CU(h, cudaMemcpyAsync(hc, counts, 10 * 4, cudaMemcpyDeviceToHost, s));
+    CU(h, cudaMemcpyAsync(hc, counts, 20 * 4, cudaMemcpyDeviceToHost, s));
     CU(h, cudaMemcpyAsync(hs, stats, 6 * 8, cudaMemcpyDeviceToHost, s));
     CU(h, cudaStreamSynchronize(s));
     if (hs[3] != 0)
         return fail(h, SABER_ERR_ARG, "%llu job(s) reference a query or window outside the loaded data", hs[3]);
-    const uint32_t n_fast = hc[0], n_gen = hc[1], n_fast8 = hc[7];
+    const uint32_t n_fast = hc[0], n_gen = hc[1], n_fast8 = hc[7], n_wave = hc[17];
     local.jobs = njobs;
     local.banded_cells = hs[0];
     local.fast_cells = hs[4];
-    local.fast_jobs = n_fast + n_fast8;
-    local.generic_jobs = n_gen;
+    local.fast_jobs = n_fast + n_fast8 + n_wave - hc[19];
+    local.generic_jobs = n_gen + hc[19];
     local.empty_jobs = hc[4];
     const uint64_t wmax_fast = std::max<uint64_t>(hs[1], hs[5]);
     const uint64_t wmax_all = std::max<uint64_t>(wmax_fast, hs[2]);
@@ -382,7 +448,7 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     const uint32_t* order = h->vals_out.as<uint32_t>();
     // generic list: class-1 jobs, then int16 overflows appended by the fast kernel
     if (n_gen)
-        CU(h, cudaMemcpyAsync(h->list.as<uint32_t>(), order + n_fast + n_fast8, (size_t)n_gen * 4,
+        CU(h, cudaMemcpyAsync(h->list.as<uint32_t>(), order + n_fast + n_fast8 + n_wave, (size_t)n_gen * 4,
                               cudaMemcpyDeviceToDevice, s));
     CU(h, cudaMemcpyAsync(counts + 5, &n_gen, 4, cudaMemcpyHostToDevice, s));
 
@@ -421,6 +487,11 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
         a.rescue_count = counts + 5;
         a.strip_rows = rows;
         CU(h, launch_band_fast(grid, s, a));
+        local.kernel_launches++;
+    }
+    if (n_wave) {
+        WaveArgs wa = wave_args(sch, ds, d_jobs, order, counts, d_scores, h->list.as<uint32_t>());
+        CU(h, launch_band_wave((unsigned)h->sm_count, s, wa));
         local.kernel_launches++;
     }
     CU(h, cudaEventRecord(ev[2], s));
@@ -469,9 +540,9 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
 // the R-row and 8-row classes in the sorted order), counts read on the device.
 __global__ void k_copy_generic(const uint32_t* __restrict__ order, uint32_t* __restrict__ counts,
                                uint32_t* __restrict__ list) {
-    const uint32_t n_fast = counts[0], n_fast8 = counts[7], n_gen = counts[1];
+    const uint32_t n_fast = counts[0], n_fast8 = counts[7], n_gen = counts[1], n_wave = counts[17];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_gen; i += gridDim.x * blockDim.x)
-        list[i] = order[n_fast + n_fast8 + i];
+        list[i] = order[n_fast + n_fast8 + n_wave + i];
     if (blockIdx.x == 0 && threadIdx.x == 0) counts[5] = n_gen;
 }
 
@@ -500,7 +571,7 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     CUALLOC(h, h->keys_out, npad * 8);
     CUALLOC(h, h->vals_in, npad * 4);
     CUALLOC(h, h->vals_out, npad * 4);
-    CUALLOC(h, h->counts, 16 * 4);
+    CUALLOC(h, h->counts, kCounts * 4);
     CUALLOC(h, h->stats, 8 * 8);
     CUALLOC(h, h->list, npad * 4);
     CUALLOC(h, h->g_nreal, 16);
@@ -532,6 +603,8 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
                             h->vals_out.p, h->counts.p, h->stats.p, h->list.p, h->bufs.p, h->slabs.p,
                             h->cub_tmp.p, ds.res.p, qs.prof.p, qs.offsets.p, qs.prof_off.p};
     std::memcpy(key.ptrs, ptrs, sizeof(ptrs));
+    key.qrow = qs.qrow.p;
+    key.matrix = sch.d_matrix.p;
     const void* extra = qs.prof_mpad.p;  // (pointer identity of the last profile table)
     cudaGraphExec_t exec = nullptr;
     for (auto& e : h->graphs)
@@ -546,7 +619,7 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
         auto chk = [&](cudaError_t e) {
             if (e != cudaSuccess) ok = false;
         };
-        chk(cudaMemsetAsync(counts, 0, 16 * 4, s));
+        chk(cudaMemsetAsync(counts, 0, kCounts * 4, s));
         chk(cudaMemsetAsync(stats, 0, 8 * 8, s));
         k_classify<<<nblocks(npad, 256, h->sm_count * 8), 256, 0, s>>>(
             d_jobs, npad, h->g_nreal.as<uint32_t>(), rows0, h->pair_steps, long_steps,
@@ -584,6 +657,8 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
             a.strip_rows = pass == 0 ? rows0 : kStripRowsMin;
             chk(launch_band_fast(pass == 0 ? grid0 : grid8, s, a));
         }
+        chk(launch_band_wave((unsigned)h->sm_count, s,
+                             wave_args(sch, ds, d_jobs, order, counts, d_scores, h->list.as<uint32_t>())));
         GenericArgs g;
         g.res = ds.res.as<uint8_t>();
         g.prof = qs.prof.as<int16_t>();
@@ -624,9 +699,9 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     CU(h, cudaEventRecord(e0, s));
     CU(h, cudaGraphLaunch(exec, s));
     CU(h, cudaEventRecord(e1, s));
-    uint32_t hc[10];
+    uint32_t hc[20];
     unsigned long long hs[6];
-    CU(h, cudaMemcpyAsync(hc, h->counts.p, 10 * 4, cudaMemcpyDeviceToHost, s));
+    CU(h, cudaMemcpyAsync(hc, h->counts.p, 20 * 4, cudaMemcpyDeviceToHost, s));
     CU(h, cudaMemcpyAsync(hs, h->stats.p, 6 * 8, cudaMemcpyDeviceToHost, s));
     CU(h, cudaStreamSynchronize(s));
     float ms = 0;
@@ -642,11 +717,11 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
         local.jobs = njobs;
         local.banded_cells = hs[0];
         local.fast_cells = hs[4];
-        local.fast_jobs = hc[0] + hc[7];
-        local.generic_jobs = hc[1];
+        local.fast_jobs = hc[0] + hc[7] + hc[17] - hc[19];
+        local.generic_jobs = hc[1] + hc[19];
         local.empty_jobs = hc[4];
         local.i16_rescored = hc[5] - hc[1];
-        local.kernel_launches = 5;
+        local.kernel_launches = 6;
         local.library_launches = 9;
         local.t_fast_ms = ms;
         local.prof8 = qs.p8 ? 1 : 0;
@@ -667,10 +742,12 @@ static int build_profiles(saber_gpu* h, const Scheme& sch, QuerySet& q) {
     }
     const bool fits8 = smin + q.bias_min + sch.go >= -127 && smax + q.bias_max + sch.go <= 127;
     if (fits8) CUALLOC(h, q.prof8, q.prof_elems + 64);
+    CUALLOC(h, q.qrow, (q.offs[q.nq] + 16) * 4);
     k_profile<<<q.nq, 256, 0, h->stream>>>(q.codes.as<uint8_t>(), q.offsets.as<uint64_t>(),
                                            q.has_bias ? q.bias.as<int8_t>() : nullptr, sch.d_matrix.as<int32_t>(),
                                            q.prof_off.as<uint64_t>(), q.prof_mpad.as<uint32_t>(), sch.go,
-                                           q.prof.as<int16_t>(), fits8 ? q.prof8.as<int8_t>() : nullptr);
+                                           q.prof.as<int16_t>(), fits8 ? q.prof8.as<int8_t>() : nullptr,
+                                           q.qrow.as<uint32_t>());
     CU(h, cudaGetLastError());
     CU(h, cudaStreamSynchronize(h->stream));
     q.p8 = fits8;
