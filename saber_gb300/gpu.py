@@ -416,13 +416,18 @@ class Device:
         o = np.ascontiguousarray(offsets, dtype=np.uint64)
         m = np.ascontiguousarray(np.asarray(matrix).reshape(576), dtype=np.int32)
         n = int(o[-1]) if o.size else 0
-        mask = np.zeros(max(n, 1), np.uint8)
-        probs = np.zeros(max(n, 1), np.float32) if want_probs else None
+        first = int(o[0]) if o.size else 0
+        # the call writes every residue from the first offset on
+        mask = np.empty(max(n, 1), np.uint8)
+        mask[:first] = 0
+        probs = np.empty(max(n, 1), np.float32) if want_probs else None
+        if want_probs:
+            probs[:first] = 0
         nm, lam = ctypes.c_uint64(), ctypes.c_double()
         self._check(self.lib.saber_gpu_tantan_mask(self.h, ctypes.byref(params), _ptr(m), _ptr(c), _ptr(o),
                                                    max(o.size - 1, 0), _ptr(mask), _ptr(probs), ctypes.byref(nm),
                                                    ctypes.byref(lam)), "tantan_mask")
-        return mask[:n].astype(bool), None if probs is None else probs[:n], int(nm.value), float(lam.value)
+        return mask[:n].view(bool), None if probs is None else probs[:n], int(nm.value), float(lam.value)
 
     def tantan_mask_db(self, params, matrix):
         """Mask the loaded database on the device and install it as its seed mask -> (masked, lambda)."""
@@ -439,11 +444,13 @@ class Device:
         aa = np.ascontiguousarray(codon64, dtype=np.uint8)
         nseq = max(o.size - 1, 0)
         total = int(o[-1] - o[0]) if o.size else 0
-        out = np.zeros(max(2 * total + 6, 1), np.uint8)
+        # six frames of n bases hold at most 2 n residues; the call writes all
+        # that it returns, so the bound costs address space only
+        out = np.empty(max(2 * total, 1), np.uint8)
         offs = np.zeros(6 * nseq + 1, np.uint64)
         self._check(self.lib.saber_gpu_translate6(self.h, _ptr(x) if x.size else None, _ptr(o), nseq, _ptr(aa),
                                                   _ptr(out), out.size, _ptr(offs)), "translate6")
-        return out[:int(offs[-1])].copy(), offs
+        return out[:int(offs[-1])], offs
 
     def scan(self, params, q_mask=None, region_thr=None, out_cap=None):
         """Candidate regions of the loaded query set (REGION_DTYPE, ordered by query and region order)."""
@@ -471,10 +478,16 @@ class Device:
         qc = np.ascontiguousarray(q_codes, dtype=np.uint8)
         qo = np.ascontiguousarray(q_offsets, dtype=np.uint64)
         qm = None if q_mask is None else np.ascontiguousarray(q_mask, dtype=np.uint8)
-        hcap, ocap = 1 << 16, 1 << 20
+        # A full buffer means another search, so the buffers hold the most that
+        # the batch can report (max_target_seqs x max_hsps hits a query, at most
+        # 2 m + 1 runs each) up to a limit; what is not written costs address
+        # space only.
+        nq, per_q = qo.size - 1, int(cparams.max_target_seqs) * int(cparams.max_hsps)
+        hcap = min(max(1 << 16, nq * per_q), 1 << 22)
+        ocap = min(max(1 << 20, per_q * (2 * int(qo[-1]) + nq)), 1 << 26)
         for _ in range(3):
-            hits = np.zeros(hcap, HIT_DTYPE)
-            ops = np.zeros(ocap, np.uint32)
+            hits = np.empty(hcap, HIT_DTYPE)
+            ops = np.empty(ocap, np.uint32)
             nh, no = ctypes.c_uint64(), ctypes.c_uint64()
             st = SearchStats()
             rc = self.lib.saber_gpu_search(self.h, ctypes.byref(cparams), _ptr(db), _ptr(do), do.size - 1, _ptr(qc),
@@ -516,7 +529,7 @@ class Device:
     def triage_predict(self, model, rows):
         m = np.ascontiguousarray(model, dtype=np.float32)
         x = np.ascontiguousarray(rows, dtype=np.float32).reshape(-1, TRIAGE_ROW_FLOATS)
-        out = np.zeros(x.shape[0], np.float32)
+        out = np.empty(x.shape[0], np.float32)
         self._check(self.lib.saber_gpu_triage_predict(self.h, _ptr(m), _ptr(x), x.shape[0], _ptr(out)),
                     "triage_predict")
         return out
