@@ -115,6 +115,12 @@ struct GraphEntry {
     const void* extra;
 };
 
+// Work buffers of the triage network's host entry points (gradients, training,
+// prediction): kept with the handle, sized by the largest call so far.
+struct TriageScratch {
+    DevBuf model, wb, X, Xn, y, H1, H2, z, dz, dH1, part, grad, m, v, loss;
+};
+
 struct Scheme {
     int32_t matrix[576];
     int32_t go = 11, ge = 1;
@@ -160,6 +166,7 @@ struct saber_gpu {
     bool has_db_mask = false;
     // learned triage: installed model, per-call feature buffers, collection
     saber::DevBuf tr_model, tr_wb, tr_sfeat, tr_qfeat, tr_reg, tr_rstat, tr_rq, tr_rrank, tr_qinfo, tr_X, tr_logit;
+    saber::TriageScratch tg;
     bool tr_on = false, tr_sfeat_ok = false;
     uint64_t tr_sfeat_key = 0;
     float tr_threshold = 0.f;

@@ -18,7 +18,6 @@
 #include <cmath>
 #include <cstring>
 #include <random>
-#include <type_traits>
 #include <vector>
 
 #include "runtime.cuh"
@@ -135,70 +134,312 @@ __global__ void k_region_feats(RegionFeatArgs a) {
     }
 }
 
-// ---- generic tiled GEMM: C[m][n] (=|+=) act(sum_k A[m][k] B[k][n] + bias[n]) ----------
-// A[m][k] at A[m * sam + k * sak], B[k][n] at B[k * sbk + n * sbn]; fp32
-// accumulation; ACT 0 none, 1 ReLU; ACC: add into C; MASK: multiply the
-// result by (M[m][n] > 0) (ReLU derivative of a stored activation).
-template <class TA, class TB>
-__device__ __forceinline__ float ld_as_f(const TA* p) {
-    if constexpr (std::is_same<TA, __nv_bfloat16>::value) return __bfloat162float(*p);
-    else return (float)*p;
+// ---- training GEMMs: fp32 FMA on 64 x 64 tiles -----------------------------------
+// C[m][n] = sum_k A[m][k] B[k][n], 256 threads, 4 x 4 outputs each, k in
+// steps of 32: both operands are staged k-major in shared memory (pitch 68:
+// 16-byte rows, so a thread reads its four rows and four columns of a k with
+// two 128-bit loads per 16 FMA), the next step's global loads are in flight
+// while a step computes.  fp32 throughout: the gradients keep the accuracy of
+// a plain fp32 sum (the bf16 tensor path would round the activations).
+// An operand is a loader: ld() reads a thread's 8 values of a step into
+// registers, st() stores them k-major.  Loaders zero what lies outside the
+// matrix.  The weight gradients contract over the batch's rows: the rows are
+// split over blockIdx.z, each split writes its own partial gradient, and
+// k_sum_splits adds them (2,048 rows: 16 splits x 16 tiles instead of 16
+// blocks walking all rows).  A call of 2,048 rows takes six launches and 154
+// us on one GB300 (fourteen launches and 1.49 ms with one block per output
+// tile, separate column sums and buffers allocated per call); its error
+// against 64 bits fell from 6e-7 to 8e-8.
+constexpr int kBT = 64, kBK = 32, kPitch = kBT + 4;
+
+__device__ __forceinline__ float4 bf4(uint2 v) {
+    const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&v.x), b = *reinterpret_cast<const __nv_bfloat162*>(&v.y);
+    return make_float4(__bfloat162float(a.x), __bfloat162float(a.y), __bfloat162float(b.x), __bfloat162float(b.y));
 }
 
-template <class TA, class TB, int ACT, bool ACC, bool MASK>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const TA* __restrict__ A, long sam, long sak,
-                                              const TB* __restrict__ B, long sbk, long sbn, const float* __restrict__ bias,
-                                              const float* __restrict__ Mk, float* __restrict__ C, long ldc) {
-    __shared__ float As[16][64 + 1];
-    __shared__ float Bs[16][64 + 1];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int t = threadIdx.x; t < 16 * 64; t += 256) {
-            const int kk = t / 64, mm = t % 64;
-            const int gm = m0 + mm, gk = k0 + kk;
-            As[kk][mm] = (gm < M && gk < K) ? ld_as_f<TA, TA>(A + (long)gm * sam + (long)gk * sak) : 0.f;
-            const int gn = n0 + mm;
-            Bs[kk][mm] = (gn < N && gk < K) ? ld_as_f<TB, TB>(B + (long)gk * sbk + (long)gn * sbn) : 0.f;
+// rows r0 .. of a row-major [rows][ld] matrix, k along the columns:
+// thread t takes row t / 4 and k = 4 (t % 4) + {0..3, 16..19}
+struct RowsF32 {
+    const float* p;
+    int rows, ld;
+    float4 v[2];
+    __device__ __forceinline__ void load(int r0, int k0, int) {
+        const int r = r0 + (threadIdx.x >> 2), k = k0 + 4 * (threadIdx.x & 3);
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            v[h] = r < rows ? *reinterpret_cast<const float4*>(p + (size_t)r * ld + k + 16 * h)
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __device__ __forceinline__ void store(float (*S)[kPitch]) const {
+        const int r = threadIdx.x >> 2, k = 4 * (threadIdx.x & 3);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            S[k + 16 * h][r] = v[h].x;
+            S[k + 16 * h + 1][r] = v[h].y;
+            S[k + 16 * h + 2][r] = v[h].z;
+            S[k + 16 * h + 3][r] = v[h].w;
         }
+    }
+};
+// the same over a bf16 matrix with all its rows present
+struct RowsBf16 {
+    const __nv_bfloat16* p;
+    int ld;
+    float4 v[2];
+    __device__ __forceinline__ void load(int r0, int k0, int) {
+        const int r = r0 + (threadIdx.x >> 2), k = k0 + 4 * (threadIdx.x & 3);
+#pragma unroll
+        for (int h = 0; h < 2; h++) v[h] = bf4(*reinterpret_cast<const uint2*>(p + (size_t)r * ld + k + 16 * h));
+    }
+    __device__ __forceinline__ void store(float (*S)[kPitch]) const { RowsF32{nullptr, 0, 0, {v[0], v[1]}}.store(S); }
+};
+// the output layer's backward, dH2[i][j] = dz[i] W3[j] (H2[i][j] > 0), rows i
+struct RowsDH2 {
+    const float *H2, *dz;
+    const __nv_bfloat16* w3;
+    int rows;
+    float4 v[2];
+    __device__ __forceinline__ void load(int r0, int k0, int) {
+        const int r = r0 + (threadIdx.x >> 2), k = k0 + 4 * (threadIdx.x & 3);
+        const float d = r < rows ? dz[r] : 0.f;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float4 a = r < rows ? *reinterpret_cast<const float4*>(H2 + (size_t)r * kTHid + k + 16 * h)
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 w = bf4(*reinterpret_cast<const uint2*>(w3 + k + 16 * h));
+            v[h] = make_float4(a.x > 0.f ? d * w.x : 0.f, a.y > 0.f ? d * w.y : 0.f, a.z > 0.f ? d * w.z : 0.f,
+                               a.w > 0.f ? d * w.w : 0.f);
+        }
+    }
+    __device__ __forceinline__ void store(float (*S)[kPitch]) const { RowsF32{nullptr, 0, 0, {v[0], v[1]}}.store(S); }
+};
+// k along the rows of a row-major [..][ld] matrix, columns c0 .. c0 + 63 (those
+// below cols): thread t takes columns 4 (t % 16) .. + 3 of rows t / 16 and + 16
+struct ColsF32 {
+    const float* p;
+    int ld, cols;
+    float4 v[2];
+    __device__ __forceinline__ void load(int c0, int k0, int kend) {
+        const int c = c0 + 4 * (threadIdx.x & 15);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int k = k0 + (threadIdx.x >> 4) + 16 * h;
+            v[h] = k < kend && c < cols ? *reinterpret_cast<const float4*>(p + (size_t)k * ld + c)
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __device__ __forceinline__ void store(float (*S)[kPitch]) const {
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            *reinterpret_cast<float4*>(&S[(threadIdx.x >> 4) + 16 * h][4 * (threadIdx.x & 15)]) = v[h];
+    }
+};
+struct ColsBf16 {
+    const __nv_bfloat16* p;
+    float4 v[2];
+    __device__ __forceinline__ void load(int c0, int k0, int) {
+        const int c = c0 + 4 * (threadIdx.x & 15);
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            v[h] = bf4(*reinterpret_cast<const uint2*>(p + (size_t)(k0 + (threadIdx.x >> 4) + 16 * h) * kTHid + c));
+    }
+    __device__ __forceinline__ void store(float (*S)[kPitch]) const { ColsF32{nullptr, 0, 0, {v[0], v[1]}}.store(S); }
+};
+// dH2 with k along the rows; keeps the column sums of dH2 (db2) and of
+// H2 dz (dW3) of the rows this thread loads
+struct ColsDH2 {
+    const float *H2, *dz;
+    const __nv_bfloat16* w3;
+    float4 v[2];
+    float4 sb, sw;
+    float sz;
+    __device__ __forceinline__ void load(int c0, int k0, int kend) {
+        const int c = c0 + 4 * (threadIdx.x & 15);
+        const float4 w = bf4(*reinterpret_cast<const uint2*>(w3 + c));
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int k = k0 + (threadIdx.x >> 4) + 16 * h;
+            const float d = k < kend ? dz[k] : 0.f;
+            const float4 a = k < kend ? *reinterpret_cast<const float4*>(H2 + (size_t)k * kTHid + c)
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[h] = make_float4(a.x > 0.f ? d * w.x : 0.f, a.y > 0.f ? d * w.y : 0.f, a.z > 0.f ? d * w.z : 0.f,
+                               a.w > 0.f ? d * w.w : 0.f);
+            sb = make_float4(sb.x + v[h].x, sb.y + v[h].y, sb.z + v[h].z, sb.w + v[h].w);
+            sw = make_float4(fmaf(a.x, d, sw.x), fmaf(a.y, d, sw.y), fmaf(a.z, d, sw.z), fmaf(a.w, d, sw.w));
+            sz += d;
+        }
+    }
+    __device__ __forceinline__ void store(float (*S)[kPitch]) const { ColsF32{nullptr, 0, 0, {v[0], v[1]}}.store(S); }
+};
+
+template <class LA, class LB>
+__device__ __forceinline__ void gemm_tile(LA& la, LB& lb, int m0, int n0, int kbeg, int kend, float (*As)[kPitch],
+                                          float (*Bs)[kPitch], float (&acc)[4][4]) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    la.load(m0, kbeg, kend);
+    lb.load(n0, kbeg, kend);
+    for (int k0 = kbeg; k0 < kend; k0 += kBK) {
+        la.store(As);
+        lb.store(Bs);
         __syncthreads();
+        if (k0 + kBK < kend) {
+            la.load(m0, k0 + kBK, kend);
+            lb.load(n0, k0 + kBK, kend);
+        }
 #pragma unroll
-        for (int kk = 0; kk < 16; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
+        for (int k = 0; k < kBK; k++) {
+            const float4 a = *reinterpret_cast<const float4*>(&As[k][4 * ty]);
+            const float4 b = *reinterpret_cast<const float4*>(&Bs[k][4 * tx]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
         }
         __syncthreads();
     }
+}
+
+// H = relu(A W + b), A [rows][lda] fp32, W [K][256] bf16
+__global__ void __launch_bounds__(256) k_layer(const float* __restrict__ A, int rows, int K,
+                                               const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
+                                               float* __restrict__ H) {
+    __shared__ __align__(16) float As[kBK][kPitch], Bs[kBK][kPitch];
+    float acc[4][4];
+    const int n0 = blockIdx.x * kBT, m0 = blockIdx.y * kBT;
+    RowsF32 la{A, rows, K, {}};
+    ColsBf16 lb{W, {}};
+    gemm_tile(la, lb, m0, n0, 0, K, As, Bs, acc);
+    const int n = n0 + 4 * (threadIdx.x & 15);
+    const float4 b = make_float4(bias[n], bias[n + 1], bias[n + 2], bias[n + 3]);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= N) continue;
-            float v = acc[i][j] + (bias ? bias[gn] : 0.f);
-            if (ACT == 1) v = fmaxf(v, 0.f);
-            if (MASK) v = Mk[(long)gm * ldc + gn] > 0.f ? v : 0.f;
-            float* c = C + (long)gm * ldc + gn;
-            *c = ACC ? *c + v : v;
-        }
+        const int m = m0 + 4 * (threadIdx.x >> 4) + i;
+        if (m < rows)
+            *reinterpret_cast<float4*>(H + (size_t)m * kTHid + n) =
+                make_float4(fmaxf(acc[i][0] + b.x, 0.f), fmaxf(acc[i][1] + b.y, 0.f), fmaxf(acc[i][2] + b.z, 0.f),
+                            fmaxf(acc[i][3] + b.w, 0.f));
     }
 }
 
-template <class TA, class TB, int ACT, bool ACC, bool MASK>
-static void gemm(cudaStream_t s, int M, int N, int K, const TA* A, long sam, long sak, const TB* B, long sbk, long sbn,
-                 const float* bias, const float* Mk, float* C, long ldc) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    k_gemm<TA, TB, ACT, ACC, MASK><<<grid, 256, 0, s>>>(M, N, K, A, sam, sak, B, sbk, sbn, bias, Mk, C, ldc);
+// dH1 = (dH2 W2^T) * relu'(H1), dH2 formed from H2, dz and W3 as it is loaded
+__global__ void __launch_bounds__(256) k_back_hidden(const float* __restrict__ H2, const float* __restrict__ dz,
+                                                     const __nv_bfloat16* __restrict__ w3, int rows,
+                                                     const __nv_bfloat16* __restrict__ W2,
+                                                     const float* __restrict__ H1, float* __restrict__ dH1) {
+    __shared__ __align__(16) float As[kBK][kPitch], Bs[kBK][kPitch];
+    float acc[4][4];
+    const int n0 = blockIdx.x * kBT, m0 = blockIdx.y * kBT;
+    RowsDH2 la{H2, dz, w3, rows, {}};
+    RowsBf16 lb{W2, kTHid, {}};
+    gemm_tile(la, lb, m0, n0, 0, kTHid, As, Bs, acc);
+    const int n = n0 + 4 * (threadIdx.x & 15);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int m = m0 + 4 * (threadIdx.x >> 4) + i;
+        if (m >= rows) continue;
+        const float4 h = *reinterpret_cast<const float4*>(H1 + (size_t)m * kTHid + n);
+        *reinterpret_cast<float4*>(dH1 + (size_t)m * kTHid + n) =
+            make_float4(h.x > 0.f ? acc[i][0] : 0.f, h.y > 0.f ? acc[i][1] : 0.f, h.z > 0.f ? acc[i][2] : 0.f,
+                        h.w > 0.f ? acc[i][3] : 0.f);
+    }
+}
+
+// Sum of a per-thread float4 over the 16 threads of a column group (threads
+// t, t + 16, ...), through shared memory; valid in the first 16 threads.
+__device__ __forceinline__ float4 sum_column_group(float4 v, float4* buf) {
+    __syncthreads();
+    buf[threadIdx.x] = v;
+    __syncthreads();
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (threadIdx.x < 16)
+        for (int i = 0; i < 16; i++) {
+            const float4 x = buf[threadIdx.x + 16 * i];
+            s = make_float4(s.x + x.x, s.y + x.y, s.z + x.z, s.w + x.w);
+        }
+    return s;
+}
+
+// Partial weight gradients of the rows of split blockIdx.z into part + split *
+// kOffMu (model layout).  blockIdx.y < 4: tile row blockIdx.y of dW2 = H1^T
+// dH2, the first with db2, dW3 and db3; blockIdx.y == 4: dW1 = Xn^T dH1 with
+// db1.
+__global__ void __launch_bounds__(256) k_weight_grads(const float* __restrict__ Xn, const float* __restrict__ H1,
+                                                      const float* __restrict__ H2, const float* __restrict__ dz,
+                                                      const __nv_bfloat16* __restrict__ w3,
+                                                      const float* __restrict__ dH1, int rows, int per_split,
+                                                      float* __restrict__ part) {
+    __shared__ __align__(16) float As[kBK][kPitch], Bs[kBK][kPitch];
+    const int n0 = blockIdx.x * kBT, kbeg = blockIdx.z * per_split, kend = min(rows, kbeg + per_split);
+    const int n = n0 + 4 * (threadIdx.x & 15);
+    float* g = part + (size_t)blockIdx.z * kOffMu;
+    float acc[4][4];
+    float4* buf = reinterpret_cast<float4*>(&As[0][0]);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto put4 = [](float* p, float4 v) {  // model offsets of W3 and the biases are not all 16-byte aligned
+        p[0] = v.x;
+        p[1] = v.y;
+        p[2] = v.z;
+        p[3] = v.w;
+    };
+    if (blockIdx.y < 4) {
+        const int m0 = blockIdx.y * kBT;
+        ColsF32 la{H1, kTHid, kTHid, {}};
+        ColsDH2 lb{H2, dz, w3, {}, zero, zero, 0.f};
+        gemm_tile(la, lb, m0, n0, kbeg, kend, As, Bs, acc);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            put4(g + kOffW2 + (size_t)(m0 + 4 * (threadIdx.x >> 4) + i) * kTHid + n,
+                 make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
+        if (blockIdx.y == 0) {
+            const float4 b = sum_column_group(lb.sb, buf), w = sum_column_group(lb.sw, buf);
+            const float4 z = sum_column_group(make_float4(lb.sz, 0.f, 0.f, 0.f), buf);
+            if (threadIdx.x < 16) {
+                put4(g + kOffB2 + n, b);
+                put4(g + kOffW3 + n, w);
+                if (n == 0) g[kOffB3] = z.x;
+            }
+        }
+    } else {
+        ColsF32 la{Xn, kTIn, kTIn, {}};
+        ColsF32 lb{dH1, kTHid, kTHid, {}};
+        // column sums of dH1 beside the product: rows of the staged tiles
+        float4 sb = zero;
+        struct Summed {
+            ColsF32& l;
+            float4& s;
+            __device__ __forceinline__ void load(int c0, int k0, int ke) {
+                l.load(c0, k0, ke);
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    s = make_float4(s.x + l.v[h].x, s.y + l.v[h].y, s.z + l.v[h].z, s.w + l.v[h].w);
+            }
+            __device__ __forceinline__ void store(float (*S)[kPitch]) const { l.store(S); }
+        } ls{lb, sb};
+        gemm_tile(la, ls, 0, n0, kbeg, kend, As, Bs, acc);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int m = 4 * (threadIdx.x >> 4) + i;
+            if (m < kTIn) put4(g + kOffW1 + (size_t)m * kTHid + n, make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]));
+        }
+        const float4 b = sum_column_group(sb, buf);
+        if (threadIdx.x < 16) put4(g + kOffB1 + n, b);
+    }
+}
+
+// grad = sum over the splits (zero for the normalisation entries, which are
+// not trained)
+__global__ void k_sum_splits(const float* __restrict__ part, int splits, float* __restrict__ grad) {
+    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < kModelFloats; t += (size_t)gridDim.x * blockDim.x) {
+        float s = 0.f;
+        if (t < kOffMu)
+            for (int k = 0; k < splits; k++) s += part[(size_t)k * kOffMu + t];
+        grad[t] = s;
+    }
 }
 
 // normalised inputs: Xn = (X - mu) * isd
@@ -215,41 +456,46 @@ __global__ void k_to_bf16(const float* __restrict__ src, uint64_t n, __nv_bfloat
         dst[t] = __float2bfloat16_rn(src[t]);
 }
 
-// binary cross-entropy on logits, positives weighted by pos_weight, mean over
-// the batch: dz = w (sigmoid(z) - y) / n; loss accumulated in double
-__global__ void k_bce(const float* __restrict__ z, const uint8_t* __restrict__ y, int n, float pos_weight,
-                      float* __restrict__ dz, double* __restrict__ loss) {
+// Output layer and binary cross-entropy on its logits, positives weighted by
+// pos_weight, mean over the batch: z = H2 W3 + b3, dz = w (sigmoid(z) - y) / n;
+// loss accumulated in double.  A block stages 32 rows in shared memory and a
+// lane sums a row's products in column order (the logit's rounding does not
+// depend on the batch, so neither does the loss).
+constexpr int kBceRows = 32;
+__global__ void __launch_bounds__(256) k_out_bce(const float* __restrict__ H2, const __nv_bfloat16* __restrict__ w3,
+                                                 const float* __restrict__ b3, const uint8_t* __restrict__ y, int n,
+                                                 float pos_weight, float* __restrict__ dz, double* __restrict__ loss) {
+    __shared__ float rows[kBceRows][kTHid + 1], w[kTHid];
+    const int r0 = blockIdx.x * kBceRows;
+    for (int t = threadIdx.x; t < kBceRows * kTHid / 4; t += 256) {
+        const int r = t / (kTHid / 4), c = 4 * (t % (kTHid / 4));
+        if (r0 + r >= n) break;
+        const float4 v = *reinterpret_cast<const float4*>(H2 + (size_t)(r0 + r) * kTHid + c);
+        rows[r][c] = v.x;
+        rows[r][c + 1] = v.y;
+        rows[r][c + 2] = v.z;
+        rows[r][c + 3] = v.w;
+    }
+    w[threadIdx.x] = __bfloat162float(w3[threadIdx.x]);
+    __syncthreads();
+    if (threadIdx.x >= kBceRows) return;
+    const int i = r0 + threadIdx.x;
     double l = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float zi = z[i];
+    if (i < n) {
+        float s = 0.f;
+#pragma unroll 16
+        for (int k = 0; k < kTHid; k++) s = fmaf(rows[threadIdx.x][k], w[k], s);
+        const float zi = s + b3[0];
         const float yi = y[i] ? 1.f : 0.f;
-        const float w = y[i] ? pos_weight : 1.f;
+        const float wt = y[i] ? pos_weight : 1.f;
         const float p = 1.f / (1.f + expf(-zi));
-        dz[i] = w * (p - yi) / (float)n;
+        dz[i] = wt * (p - yi) / (float)n;
         // log(1 + exp(-|z|)) + max(z, 0) - y z
         const float li = log1pf(expf(-fabsf(zi))) + fmaxf(zi, 0.f) - yi * zi;
-        l += (double)(w * li) / n;
+        l = (double)(wt * li) / n;
     }
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
-}
-
-// column sums: out[j] (=|+=) sum_i G[i][j]
-__global__ void k_colsum(const float* __restrict__ G, int rows, int cols, float* __restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= cols) return;
-    float s = 0.f;
-    for (int i = 0; i < rows; i++) s += G[(long)i * cols + j];
-    out[j] = s;
-}
-
-// dH2[i][j] = dz[i] * W3[j] * (H2[i][j] > 0)
-__global__ void k_outer_mask(const float* __restrict__ dz, int n, const __nv_bfloat16* __restrict__ w3,
-                             const float* __restrict__ H2, float* __restrict__ dH2) {
-    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < (long)n * kTHid; t += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / kTHid), j = (int)(t % kTHid);
-        dH2[t] = H2[t] > 0.f ? dz[i] * __bfloat162float(w3[j]) : 0.f;
-    }
+    if (threadIdx.x == 0) atomicAdd(loss, l);
 }
 
 // Adam (bias-corrected), fp32 masters, weights only (the normalisation
@@ -411,10 +657,6 @@ __global__ void k_gather_rows(const float* __restrict__ Xn, const uint8_t* __res
 }
 
 // ---- host side -------------------------------------------------------------------
-struct TriageDev {
-    DevBuf model, wb, X, Xn, y, H1, H2, z, dz, dH2, dH1, grad, m, v, loss;
-};
-
 int triage_upload_model(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* host_model);
 static int upload_model(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* host_model) {
     return triage_upload_model(h, model, wb, host_model);
@@ -435,58 +677,44 @@ int triage_upload_model(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* ho
     return SABER_OK;
 }
 
+// Row splits of the weight gradients: at least 128 rows each, at most 32 (the
+// partials stay under 10 MB and are added from L2).
+static int grad_splits(uint64_t n) { return (int)std::min<uint64_t>(std::max<uint64_t>(n / 128, 1), 32); }
+
 // forward + backward of one batch (inputs already normalised in Xn, labels
 // in y): gradients written to grad (model layout), loss added to *loss
-static int fwd_bwd(saber_gpu* h, TriageDev& d, int n, float pos_weight) {
+static int fwd_bwd(saber_gpu* h, TriageScratch& d, int n, float pos_weight) {
     cudaStream_t s = h->stream;
     const float* mdl = d.model.as<float>();
     const __nv_bfloat16* wb = d.wb.as<__nv_bfloat16>();
+    const float* Xn = d.Xn.as<float>();
     float* H1 = d.H1.as<float>();
     float* H2 = d.H2.as<float>();
-    float* z = d.z.as<float>();
-    float* g = d.grad.as<float>();
-    // forward
-    gemm<float, __nv_bfloat16, 1, false, false>(s, n, kTHid, kTIn, d.Xn.as<float>(), kTIn, 1, wb + kOffW1, kTHid, 1,
-                                                mdl + kOffB1, nullptr, H1, kTHid);
-    gemm<float, __nv_bfloat16, 1, false, false>(s, n, kTHid, kTHid, H1, kTHid, 1, wb + kOffW2, kTHid, 1, mdl + kOffB2,
-                                                nullptr, H2, kTHid);
-    gemm<float, __nv_bfloat16, 0, false, false>(s, n, 1, kTHid, H2, kTHid, 1, wb + kOffW3, 1, 1, mdl + kOffB3, nullptr,
-                                                z, 1);
-    // loss and dz
-    k_bce<<<nblocks(n, 256, 1024), 256, 0, s>>>(z, d.y.as<uint8_t>(), n, pos_weight, d.dz.as<float>(),
-                                                 d.loss.as<double>());
-    // output layer: dW3 = H2^T dz, db3 = sum dz
-    gemm<float, float, 0, false, false>(s, kTHid, 1, n, H2, 1, kTHid, d.dz.as<float>(), 1, 1, nullptr, nullptr,
-                                        g + kOffW3, 1);
-    k_colsum<<<1, 32, 0, s>>>(d.dz.as<float>(), n, 1, g + kOffB3);
-    // dH2 = dz W3^T * relu'(H2)
-    k_outer_mask<<<nblocks((uint64_t)n * kTHid, 256), 256, 0, s>>>(d.dz.as<float>(), n, wb + kOffW3, H2,
-                                                                      d.dH2.as<float>());
-    // dW2 = H1^T dH2, db2
-    gemm<float, float, 0, false, false>(s, kTHid, kTHid, n, H1, 1, kTHid, d.dH2.as<float>(), kTHid, 1, nullptr, nullptr,
-                                        g + kOffW2, kTHid);
-    k_colsum<<<(kTHid + 127) / 128, 128, 0, s>>>(d.dH2.as<float>(), n, kTHid, g + kOffB2);
-    // dH1 = dH2 W2^T * relu'(H1)
-    gemm<float, __nv_bfloat16, 0, false, true>(s, n, kTHid, kTHid, d.dH2.as<float>(), kTHid, 1, wb + kOffW2, 1, kTHid,
-                                               nullptr, H1, d.dH1.as<float>(), kTHid);
-    // dW1 = Xn^T dH1, db1
-    gemm<float, float, 0, false, false>(s, kTIn, kTHid, n, d.Xn.as<float>(), 1, kTIn, d.dH1.as<float>(), kTHid, 1,
-                                        nullptr, nullptr, g + kOffW1, kTHid);
-    k_colsum<<<(kTHid + 127) / 128, 128, 0, s>>>(d.dH1.as<float>(), n, kTHid, g + kOffB1);
-    CU(h, cudaMemsetAsync(g + kOffMu, 0, 2 * kTIn * 4, s));
+    float* dz = d.dz.as<float>();
+    const dim3 tiles(kTHid / kBT, (unsigned)((n + kBT - 1) / kBT));
+    k_layer<<<tiles, 256, 0, s>>>(Xn, n, kTIn, wb + kOffW1, mdl + kOffB1, H1);
+    k_layer<<<tiles, 256, 0, s>>>(H1, n, kTHid, wb + kOffW2, mdl + kOffB2, H2);
+    k_out_bce<<<(unsigned)((n + kBceRows - 1) / kBceRows), 256, 0, s>>>(
+        H2, wb + kOffW3, mdl + kOffB3, d.y.as<uint8_t>(), n, pos_weight, dz, d.loss.as<double>());
+    k_back_hidden<<<tiles, 256, 0, s>>>(H2, dz, wb + kOffW3, n, wb + kOffW2, H1, d.dH1.as<float>());
+    int splits = grad_splits((uint64_t)n);
+    const int per = (((n + splits - 1) / splits) + kBK - 1) / kBK * kBK;
+    splits = (n + per - 1) / per;
+    k_weight_grads<<<dim3(kTHid / kBT, 5, (unsigned)splits), 256, 0, s>>>(Xn, H1, H2, dz, wb + kOffW3,
+                                                                          d.dH1.as<float>(), n, per, d.part.as<float>());
+    k_sum_splits<<<nblocks(kModelFloats, 256), 256, 0, s>>>(d.part.as<float>(), splits, d.grad.as<float>());
     CU(h, cudaGetLastError());
     return SABER_OK;
 }
 
-static int reserve_batch(saber_gpu* h, TriageDev& d, uint64_t n) {
+static int reserve_batch(saber_gpu* h, TriageScratch& d, uint64_t n) {
     CUALLOC(h, d.Xn, n * kTIn * 4);
     CUALLOC(h, d.y, n + 16);
     CUALLOC(h, d.H1, n * kTHid * 4);
     CUALLOC(h, d.H2, n * kTHid * 4);
-    CUALLOC(h, d.z, n * 4 + 16);
     CUALLOC(h, d.dz, n * 4 + 16);
-    CUALLOC(h, d.dH2, n * kTHid * 4);
     CUALLOC(h, d.dH1, n * kTHid * 4);
+    CUALLOC(h, d.part, (uint64_t)grad_splits(n) * kOffMu * 4);
     CUALLOC(h, d.grad, kModelFloats * 4);
     CUALLOC(h, d.loss, 16);
     return SABER_OK;
@@ -494,13 +722,14 @@ static int reserve_batch(saber_gpu* h, TriageDev& d, uint64_t n) {
 
 int triage_grads(saber_gpu* h, const float* model, const float* X, const uint8_t* y, uint32_t n, float pos_weight,
                  float* grads, double* loss) {
-    TriageDev d;
+    if (n == 0) return fail(h, SABER_ERR_CUDA, "no rows: invalid launch configuration");
+    TriageScratch& d = h->tg;
     int rc = upload_model(h, d.model, d.wb, model);
     if (rc != SABER_OK) return rc;
-    rc = reserve_batch(h, d, std::max<uint32_t>(n, 1));
+    rc = reserve_batch(h, d, n);
     if (rc != SABER_OK) return rc;
     cudaStream_t s = h->stream;
-    CUALLOC(h, d.X, (uint64_t)std::max<uint32_t>(n, 1) * kTIn * 4);
+    CUALLOC(h, d.X, (uint64_t)n * kTIn * 4);
     CU(h, cudaMemcpyAsync(d.X.p, X, (uint64_t)n * kTIn * 4, cudaMemcpyHostToDevice, s));
     CU(h, cudaMemcpyAsync(d.y.p, y, n, cudaMemcpyHostToDevice, s));
     CU(h, cudaMemsetAsync(d.loss.p, 0, 8, s));
@@ -521,7 +750,7 @@ int triage_train(saber_gpu* h, float* model, const float* X, const uint8_t* y, u
     if (n == 0) return fail(h, SABER_ERR_ARG, "no training samples");
     cudaStream_t s = h->stream;
     const int B = (int)std::max<uint32_t>(32, cfg->batch);
-    TriageDev d;
+    TriageScratch& d = h->tg;
     int rc = upload_model(h, d.model, d.wb, model);
     if (rc != SABER_OK) return rc;
     rc = reserve_batch(h, d, (uint64_t)B);
@@ -595,15 +824,15 @@ int triage_predict(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* d_X, ui
 }
 
 int triage_predict_host(saber_gpu* h, const float* model, const float* X, uint64_t n, float* logits) {
-    DevBuf m, wb, dX, dz;
-    int rc = upload_model(h, m, wb, model);
+    TriageScratch& d = h->tg;
+    int rc = upload_model(h, d.model, d.wb, model);
     if (rc != SABER_OK) return rc;
-    CUALLOC(h, dX, std::max<uint64_t>(n, 1) * kTIn * 4);
-    CUALLOC(h, dz, std::max<uint64_t>(n, 1) * 4);
-    CU(h, cudaMemcpyAsync(dX.p, X, n * kTIn * 4, cudaMemcpyHostToDevice, h->stream));
-    rc = triage_predict(h, m, wb, dX.as<float>(), n, dz.as<float>());
+    CUALLOC(h, d.X, std::max<uint64_t>(n, 1) * kTIn * 4);
+    CUALLOC(h, d.z, std::max<uint64_t>(n, 1) * 4);
+    CU(h, cudaMemcpyAsync(d.X.p, X, n * kTIn * 4, cudaMemcpyHostToDevice, h->stream));
+    rc = triage_predict(h, d.model, d.wb, d.X.as<float>(), n, d.z.as<float>());
     if (rc != SABER_OK) return rc;
-    CU(h, cudaMemcpyAsync(logits, dz.p, n * 4, cudaMemcpyDeviceToHost, h->stream));
+    CU(h, cudaMemcpyAsync(logits, d.z.p, n * 4, cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
     return SABER_OK;
 }
