@@ -140,6 +140,13 @@ __device__ __forceinline__ bool code_rank(const uint2* __restrict__ grp, uint32_
     return (g.x & bit) != 0;
 }
 
+// A shape's care letters as nibbles of a 32-letter window (four words), hashed
+// to the top bits of one sum of products: the scan hashes a subject window
+// masked to the care nibbles, the seed tables hash a seed's letters one by one.
+__host__ __device__ constexpr uint32_t fil_mul(int w) {
+    return w == 0 ? 0x9E3779B1u : w == 1 ? 0x7FEB352Du : w == 2 ? 0x846CA68Bu : 0xB5297A4Du;
+}
+
 // The tables of all shapes, built together (blockIdx.y: the shape) so that a
 // batch costs nine launches whatever its shapes: a code space of 10^7 letters
 // words is touched as presence bits only (2.5 MB a shape), and everything per
@@ -153,6 +160,9 @@ __device__ __forceinline__ bool code_rank(const uint2* __restrict__ grp, uint32_
 //   pass 2: scatter of the batch positions
 constexpr int kMaxShapes = 32;
 struct SeedArgs {
+    uint32_t* fil;        // hash filter bits of all shapes, or null (ScanFilter)
+    uint32_t fil_words;   // 32-bit words per shape
+    int fil_shift;
     const uint8_t *qsb, *qrem;
     uint64_t QN;
     uint32_t asize;
@@ -183,6 +193,15 @@ __global__ void k_query_seeds(const __grid_constant__ SeedArgs a) {
         }
         if (PASS == 0) {
             atomicOr(&grp[c >> 5].x, 1u << (c & 31));
+            if (a.fil) {
+                uint32_t hsum = 0;
+                for (uint32_t t = 0; t < sh.w; t++) {
+                    const uint32_t o = sh.off[t];
+                    hsum += ((uint32_t)a.qsb[i + o] << (4 * (o & 7))) * fil_mul(o >> 3);
+                }
+                hsum >>= a.fil_shift;
+                atomicOr(&a.fil[(size_t)si * a.fil_words + (hsum >> 5)], 1u << (hsum & 31));
+            }
             kept++;
         } else {
             uint32_t k;
@@ -254,6 +273,13 @@ struct ScanArgs {
     unsigned long long* nsurv;  // counter (may exceed cap: overflow)
     uint64_t cap;
     unsigned long long* ctr;    // [2] hits, [3] filtered
+    // the hash filter's scan (k_scan_few): seed letters as nibbles, filter bits
+    const uint32_t* nib;
+    const uint32_t* fil;
+    uint32_t fil_words;
+    int fil_shift;
+    uint32_t care[kMaxShapes];      // bit o: offset o is a care position
+    uint32_t cmask[kMaxShapes][4];  // the care nibbles of the window words
     // per shape: care offsets, table / entry bases
     ShapeDev sh[kMaxShapes];
     uint64_t grp_off[kMaxShapes];
@@ -327,6 +353,7 @@ struct WarpScan {
     const uint32_t* resw;  // 32 staged words: residues of the same range
     uint32_t nsv;      // staged survivors (warp-uniform)
     uint32_t rd;       // this lane's position: rem | dst << 8
+    const uint16_t* rds;   // the same of every staged position (k_scan_few)
     uint64_t base;
 };
 
@@ -344,10 +371,12 @@ __device__ __forceinline__ void surv_drain(const ScanArgs& a, int lane, WarpScan
 // The queued segments' hits, 32 per round.  Each lane keeps kPer segments'
 // starts in registers; a round's owners come from the bits of the segments
 // that start inside it and the count of those that start before it.
-template <bool COMB>
+// kCap: segments the queue holds; RDS: rem | dst from shared memory (the warp
+// staged more positions than lanes).
+template <bool COMB, int kCap = kSegCap, bool RDS = false>
 __device__ __forceinline__ void scan_flush(const ScanArgs& a, int lane, int nseg, WarpScan& ws,
                                            unsigned long long& hits, unsigned long long& filtered) {
-    constexpr int kPer = kSegCap / 32;
+    constexpr int kPer = kCap / 32;
     uint32_t st[kPer];
     uint32_t sum = 0;
 #pragma unroll
@@ -389,7 +418,7 @@ __device__ __forceinline__ void scan_flush(const ScanArgs& a, int lane, int nseg
         const uint32_t own = live ? before + __popc(B & lanes_le) - 1u : 0u;
         const int rl = ws.seg_rl[own];
         // the subject position's rem | dst from the lane that scanned it
-        const uint32_t srd = __shfl_sync(0xffffffffu, ws.rd, rl);
+        const uint32_t srd = RDS ? ws.rds[rl] : __shfl_sync(0xffffffffu, ws.rd, rl);
         bool pass = false;
         uint32_t g = 0;
         if (live) {
@@ -482,7 +511,7 @@ __global__ void __launch_bounds__(256, SABER_SCAN_MIN_BLOCKS) k_scan(ScanArgs a)
     const uint64_t warp0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long hits = 0, filtered = 0;
-    WarpScan ws{s_n[w], s_eb[w], s_rl[w], s_sh[w], s_sv[w], s_sbw[w], s_resw[w], 0u, 0u, 0u};
+    WarpScan ws{s_n[w], s_eb[w], s_rl[w], s_sh[w], s_sv[w], s_sbw[w], s_resw[w], 0u, 0u, nullptr, 0u};
     const uint8_t* stb = reinterpret_cast<const uint8_t*>(s_sbw[w]) + 32 + lane;  // this lane's position
     for (uint64_t base = warp0 * 32; base < a.N; base += nwarps * 32) {
         const uint64_t r = base + lane;
@@ -541,6 +570,167 @@ __global__ void __launch_bounds__(256, SABER_SCAN_MIN_BLOCKS) k_scan(ScanArgs a)
     if (lane == 0) {
         atomicAdd(&a.ctr[2], hits);
         atomicAdd(&a.ctr[3], filtered);
+    }
+}
+
+// The scan of a small batch.  With few seeds nearly every table lookup finds
+// nothing, and the lookups (one random 8-byte read of a table larger than L2's
+// fast half per position and shape) bound k_scan: one query against 30 M
+// residues and 16 shapes took 2.5 ms, 6.2 TB/s of L2 sectors.  Here each
+// shape's seeds are also a hash bitmap in shared memory, read first; the
+// share that passes (at most a quarter, see few_filter_bits) is queued and
+// looked up in the exact tables 32 at a time.  A window's hash needs no seed
+// code: the subject's letters are kept as nibbles (0xF where no letter seeds),
+// a lane's 32-letter window is four words, and a shape costs a mask and a
+// multiply-add per word and one shared-memory read.
+//
+// Scan of 30 M residues, 16 shapes, on one GB300 (plain -> filtered): 1 query
+// 2.50 -> 0.72 ms, 64 queries 3.00 -> 1.57, 130 queries 3.16 -> 2.25; bound
+// now by the issue of the hash and queue instructions.
+//
+// A warp takes kFewPos positions per turn (four windows per lane), so that
+// the queue and the staged bytes are shared by more positions.  W: window
+// words in use (shapes' spans up to 8 W).
+constexpr int kFewWarps = 32, kFewPos = 128, kFewSeg = 96;
+struct FewWarp {
+    uint32_t seg_n[kFewSeg], seg_eb[kFewSeg];
+    uint2 sv[kSurvStage];
+    uint32_t sbw[kFewPos / 4 + 32], resw[kFewPos / 4 + 32];
+    uint16_t rds[kFewPos];
+    uint16_t q[64];
+    uint8_t seg_rl[kFewSeg], seg_sh[kFewSeg];
+};
+constexpr size_t kFewFilterBytes = 128u << 10;  // with the warps' buffers and the shapes below the 227 KB of a block
+
+template <bool COMB, int W>
+__global__ void __launch_bounds__(kFewWarps * 32, 1) k_scan_few(const __grid_constant__ ScanArgs a) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ ShapeDev s_shape[kMaxShapes];
+    const uint32_t fwords = (a.s1 - a.s0) * a.fil_words;
+    uint32_t* fil = smem;
+    FewWarp& fw = reinterpret_cast<FewWarp*>(smem + fwords)[threadIdx.x >> 5];
+    for (uint32_t i = threadIdx.x; i < a.s1; i += blockDim.x) s_shape[i] = a.sh[i];
+    for (uint32_t i = threadIdx.x; i < fwords; i += blockDim.x) fil[i] = a.fil[(size_t)a.s0 * a.fil_words + i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const uint64_t warp0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    unsigned long long hits = 0, filtered = 0;
+    WarpScan ws{fw.seg_n, fw.seg_eb, fw.seg_rl, fw.seg_sh, fw.sv, fw.sbw, fw.resw, 0u, 0u, fw.rds, 0u};
+    const uint8_t* stb = reinterpret_cast<const uint8_t*>(fw.sbw) + 32;
+    const uint32_t lanes_lt = (1u << lane) - 1u;
+    int nseg = 0;
+    uint32_t nq = 0;
+    // the first n <= 32 queued (position, shape) pairs through the exact tables
+    auto lookup = [&](uint32_t n) {
+        __syncwarp();
+        const uint32_t it = (uint32_t)lane < n ? fw.q[lane] : 0u;
+        const uint32_t rl = it & 0xFFu, si = it >> 8;
+        uint2 r = make_uint2(0u, 0u);
+        if ((uint32_t)lane < n) {
+            const int64_t c = seed_code(stb + rl, s_shape[si], a.asize);
+            uint32_t k;
+            if (c >= 0 && code_rank(a.grp + a.grp_off[si], (uint32_t)c, k)) r = a.rng[k];
+        }
+        const uint32_t bal = __ballot_sync(0xffffffffu, r.y > 0);
+        if (r.y > 0) {
+            const int slot = nseg + __popc(bal & lanes_lt);
+            fw.seg_n[slot] = r.y;
+            fw.seg_eb[slot] = r.x;
+            fw.seg_rl[slot] = (uint8_t)rl;
+            fw.seg_sh[slot] = (uint8_t)si;
+        }
+        nseg += __popc(bal);
+        const uint32_t rest = nq - n;  // at most 31
+        const uint16_t mv = (uint32_t)lane < rest ? fw.q[n + lane] : (uint16_t)0;
+        __syncwarp();
+        if ((uint32_t)lane < rest) fw.q[lane] = mv;
+        nq = rest;
+        __syncwarp();
+        if (nseg > kFewSeg - 32) {
+            scan_flush<COMB, kFewSeg, true>(a, lane, nseg, ws, hits, filtered);
+            nseg = 0;
+        }
+    };
+    for (uint64_t base = warp0 * kFewPos; base < a.N; base += nwarps * kFewPos) {
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            const int64_t wb = (int64_t)base - 32 + 4 * (lane + 32 * t);
+            fw.sbw[lane + 32 * t] = stage_word(a.sb, wb, a.N, kNonSeed);
+            fw.resw[lane + 32 * t] = COMB ? stage_word(a.cb, wb, a.N, 0xEEu) : stage_word(a.res, wb, a.N, 0xFFu);
+        }
+#pragma unroll
+        for (int t = 0; t < kFewPos / 32; t++) {
+            const uint64_t r = base + 32 * t + lane;
+            fw.rds[32 * t + lane] = r < a.N ? (uint16_t)(a.rem[r] | (a.dst[r] << 8)) : (uint16_t)0;
+        }
+        ws.base = base;
+        __syncwarp();
+        // letters that seed nothing, by position: a lane's window mask is a
+        // funnel shift of two neighbouring words
+        uint32_t bad = __ballot_sync(0xffffffffu, stb[lane] >= a.asize);
+#pragma unroll 1
+        for (int t = 0; t < kFewPos / 32; t++) {
+            const uint32_t bad1 = __ballot_sync(0xffffffffu, stb[32 * (t + 1) + lane] >= a.asize);
+            const uint32_t inv = __funnelshift_r(bad, bad1, lane);
+            bad = bad1;
+            const uint32_t rem = fw.rds[32 * t + lane] & 0xFFu;
+            const uint32_t* np = a.nib + ((base + 32 * t + lane) >> 3);
+            uint32_t x[W + 1], win[W];
+#pragma unroll
+            for (int k = 0; k <= W; k++) x[k] = __ldg(np + k);
+#pragma unroll
+            for (int k = 0; k < W; k++) win[k] = __funnelshift_r(x[k], x[k + 1], 4 * (lane & 7));
+            uint32_t mine = 0;  // bit: this position passes shape s0 + bit
+            const uint32_t* fs = fil;
+            for (uint32_t si = a.s0; si < a.s1; si++, fs += a.fil_words) {
+                uint32_t hsum = 0;
+#pragma unroll
+                for (int k = 0; k < W; k++) hsum += (win[k] & a.cmask[si][k]) * fil_mul(k);
+                hsum >>= a.fil_shift;
+                const bool ok = ((fs[hsum >> 5] >> (hsum & 31)) & 1u) && (inv & a.care[si]) == 0 && rem >= a.sh[si].span;
+                mine |= (ok ? 1u : 0u) << (si - a.s0);
+            }
+            uint32_t any;
+            while ((any = __ballot_sync(0xffffffffu, mine != 0)) != 0) {
+                if (mine) {
+                    const uint32_t si = a.s0 + (uint32_t)__ffs(mine) - 1u;
+                    mine &= mine - 1u;
+                    fw.q[nq + __popc(any & lanes_lt)] = (uint16_t)((32 * t + lane) | (si << 8));
+                }
+                nq += __popc(any);
+                if (nq >= 32) lookup(32);
+            }
+        }
+        if (nq) lookup(nq);
+        if (nseg) {
+            __syncwarp();
+            scan_flush<COMB, kFewSeg, true>(a, lane, nseg, ws, hits, filtered);
+            nseg = 0;
+        }
+    }
+    if (ws.nsv) surv_drain(a, lane, ws);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) filtered += __shfl_xor_sync(0xffffffffu, filtered, o);
+    if (lane == 0) {
+        atomicAdd(&a.ctr[2], hits);
+        atomicAdd(&a.ctr[3], filtered);
+    }
+}
+
+// Seed letters as nibbles, eight to a word (0xF: no seeding letter); `words`
+// covers the positions and the windows that run past them.
+__global__ void k_nibbles(const uint8_t* __restrict__ sb, uint64_t N, uint32_t asize, uint64_t words,
+                          uint32_t* __restrict__ nib) {
+    for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t v = 0;
+        for (int b = 0; b < 8; b++) {
+            const uint64_t r = 8 * w + b;
+            const uint32_t c = r < N ? sb[r] : kNonSeed;
+            v |= (c < asize ? c : 0xFu) << (4 * b);
+        }
+        nib[w] = v;
     }
 }
 
@@ -1164,6 +1354,44 @@ __global__ void k_comb_bytes(const uint8_t* __restrict__ res, uint64_t N, CombTa
         cb[r] = tab.t[res[r]];
 }
 
+// ---- the small-batch scan's filter -------------------------------------------
+// Letters fit a nibble below 0xF and a window 32 letters.
+static bool few_shapes_fit(const saber_scan_params* p) {
+    if (p->alpha_size > 15) return false;
+    for (uint32_t si = 0; si < p->nshapes; si++) {
+        if (p->shape_span[si] > 32) return false;
+        for (uint32_t k = 0; k < p->shape_weight[si]; k++)
+            if (p->shape_off[si][k] >= p->shape_span[si]) return false;
+    }
+    return true;
+}
+// the words of the positions, of the last turn's positions past the end and
+// of the windows that start there
+static uint64_t few_nibble_words(uint64_t N) { return (N + kFewPos) / 8 + 8; }
+
+// Shapes per pass over the database and filter bits per shape of a batch of QN
+// positions; 0 shapes: too many seeds, the plain scan.  A shape's bitmap is at
+// most a quarter full (each position that passes costs a lookup in the exact
+// tables, which is what the filter is there to save), and a pass takes at
+// least four shapes: fewer would not pay for reading the database again.
+// At the rule's edge (62 k positions, four shapes a pass) the filtered scan
+// still wins, 2.61 against 3.78 ms over 30 M residues; past it the hits
+// themselves are most of the scan.
+static uint32_t few_filter_bits(const saber_scan_params* p, uint64_t QN, uint32_t& log2_bits) {
+    for (uint32_t spp = p->nshapes; spp >= std::min(p->nshapes, 4u); spp = (spp + 1) / 2) {
+        uint32_t lb = 10;
+        while (lb < 20 && ((uint64_t)spp << (lb + 1)) / 8 <= kFewFilterBytes) lb++;
+        // no larger than 64 bits a seed
+        while (lb > 10 && (1ull << (lb - 1)) >= 64 * QN) lb--;
+        if (4 * QN <= (1ull << lb)) {
+            log2_bits = lb;
+            return spp;
+        }
+        if (spp <= 4) break;
+    }
+    return 0;
+}
+
 int scan_build_db(saber_gpu* h, const saber_scan_params* p) {
     const Dataset& ds = h->main;
     cudaStream_t s = h->stream;
@@ -1197,6 +1425,13 @@ int scan_build_db(saber_gpu* h, const saber_scan_params* p) {
         k_dists<<<nblocks(N, 256, h->sm_count * 32), 256, 0, s>>>(ds.soff.as<uint64_t>(), ds.nsub, N,
                                                                    h->sc_rem.as<uint8_t>(), h->sc_dst.as<uint8_t>());
         CU(h, cudaGetLastError());
+        if (few_shapes_fit(p)) {
+            const uint64_t words = few_nibble_words(N);
+            CUALLOC(h, h->sc_nib, words * 4);
+            k_nibbles<<<nblocks(words, 256, h->sm_count * 32), 256, 0, s>>>(h->sc_sb.as<uint8_t>(), N, p->alpha_size,
+                                                                            words, h->sc_nib.as<uint32_t>());
+            CU(h, cudaGetLastError());
+        }
     }
     // frequent codes per shape
     h->sc_caps.assign(p->nshapes, 0);
@@ -1516,6 +1751,9 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     const uint32_t nsh = p->nshapes;
     std::vector<uint64_t> gbase(nsh + 1, 0);
     for (uint32_t si = 0; si < nsh; si++) gbase[si + 1] = gbase[si] + (ncodes_of(p, si) + 31) / 32;
+    // a small batch's scan reads hash bitmaps of the seeds first
+    uint32_t few_bits = 0;
+    const uint32_t few = QN && N && few_shapes_fit(p) ? few_filter_bits(p, QN, few_bits) : 0;
     const uint64_t ngroups = gbase[nsh], nranks = (uint64_t)nsh * QN;
     CUALLOC(h, h->sc_qpres, ngroups * 8 + 8);
     CUALLOC(h, h->sc_qslot, nranks * 4 + 4);
@@ -1535,6 +1773,17 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
         sa.slot = h->sc_qslot.as<uint32_t>();
         sa.ent = h->sc_qent.as<uint32_t>();
         sa.ctr = ctr;
+        sa.fil = nullptr;
+        sa.fil_words = 0;
+        sa.fil_shift = 0;
+        if (few) {
+            const uint64_t bytes = ((uint64_t)nsh << few_bits) / 8;
+            CUALLOC(h, h->sc_fil, bytes);
+            CU(h, cudaMemsetAsync(h->sc_fil.p, 0, bytes, s));
+            sa.fil = h->sc_fil.as<uint32_t>();
+            sa.fil_words = (1u << few_bits) / 32;
+            sa.fil_shift = 32 - (int)few_bits;
+        }
         for (uint32_t si = 0; si < nsh; si++) {
             sa.sh[si] = shape_dev(p, si);
             sa.grp_off[si] = gbase[si];
@@ -1588,10 +1837,24 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     a.asize = p->alpha_size;
     a.nsurv = ctr + 10;
     a.ctr = ctr;
+    uint32_t span_max = 0;
     for (uint32_t si = 0; si < nsh; si++) {
         a.sh[si] = shape_dev(p, si);
         a.grp_off[si] = gbase[si];
+        span_max = std::max(span_max, p->shape_span[si]);
+        a.care[si] = 0;
+        memset(a.cmask[si], 0, sizeof(a.cmask[si]));
+        if (!few) continue;
+        for (uint32_t k = 0; k < p->shape_weight[si]; k++) {
+            const uint32_t o = p->shape_off[si][k];
+            a.care[si] |= 1u << o;
+            a.cmask[si][o >> 3] |= 0xFu << (4 * (o & 7));
+        }
     }
+    a.nib = h->sc_nib.as<uint32_t>();
+    a.fil = h->sc_fil.as<uint32_t>();
+    a.fil_words = few ? (1u << few_bits) / 32 : 0;
+    a.fil_shift = few ? 32 - (int)few_bits : 0;
     // passes over groups of shapes whose tables stay within the L2 budget:
     // as many shapes per pass as the largest shape's tables allow, rounded
     // down to whole unroll groups, and at least one unroll group: with fewer
@@ -1602,7 +1865,8 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     for (uint32_t si = 0; si < nsh; si++)
         shape_bytes = std::max(shape_bytes, (gbase[si + 1] - gbase[si]) * 8 + QN * 8 + QN * 4);
     uint64_t per_pass = std::max<uint64_t>(1, h->scan_table_bytes / std::max<uint64_t>(shape_bytes, 1));
-    if (per_pass >= (uint64_t)kShapeUnroll) per_pass -= per_pass % kShapeUnroll;
+    if (few) per_pass = few;
+    else if (per_pass >= (uint64_t)kShapeUnroll) per_pass -= per_pass % kShapeUnroll;
     else per_pass = kShapeUnroll;
     std::vector<std::pair<uint32_t, uint32_t>> passes;
     for (uint32_t si = 0; si < nsh; si += (uint32_t)std::min<uint64_t>(per_pass, nsh))
@@ -1611,6 +1875,11 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     CU(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scan_bps, comb ? k_scan<true> : k_scan<false>,
                                                         kScanWarps * 32, 0));
     const unsigned scan_grid = (unsigned)std::max(1, scan_bps) * (unsigned)h->sm_count;
+    const size_t few_smem = few * (((size_t)1 << few_bits) / 8) + kFewWarps * sizeof(FewWarp);
+    auto scan_few = span_max <= 16 ? (comb ? k_scan_few<true, 2> : k_scan_few<false, 2>)
+                    : span_max <= 24 ? (comb ? k_scan_few<true, 3> : k_scan_few<false, 3>)
+                                     : (comb ? k_scan_few<true, 4> : k_scan_few<false, 4>);
+    if (few) CU(h, cudaFuncSetAttribute(scan_few, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem));
     for (int attempt = 0; attempt < 8; attempt++) {
         CUALLOC(h, h->sc_surv, scap * 8);
         CU(h, cudaMemsetAsync(ctr + 2, 0, 9 * 8, s));  // hits, filtered, ..., survivors
@@ -1620,7 +1889,8 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
             for (const auto& ps : passes) {
                 a.s0 = ps.first;
                 a.s1 = ps.second;
-                if (comb) k_scan<true><<<scan_grid, kScanWarps * 32, 0, s>>>(a);
+                if (few) scan_few<<<(unsigned)h->sm_count, kFewWarps * 32, few_smem, s>>>(a);
+                else if (comb) k_scan<true><<<scan_grid, kScanWarps * 32, 0, s>>>(a);
                 else k_scan<false><<<scan_grid, kScanWarps * 32, 0, s>>>(a);
             }
             CU(h, cudaGetLastError());
