@@ -35,29 +35,11 @@
 // the optimum and feed no cell of the window; cells past the band (k >= w in
 // the last lanes) are held at H = 0 by a mask, so that neither E nor F carries
 // a score across the band's edge.
-#include "band_common.cuh"
-
-#include <cuda_runtime.h>
+#include "band_wave.cuh"
 
 namespace saber {
 
-constexpr int kWaveRow = kWaveRowBytes;   // bytes per row of the score table (26 entries)
-constexpr int kWaveSent = 24;             // row / column of the sentinel score
 constexpr unsigned kWaveThreads = 128;
-constexpr int kWaveAhead = 4;             // pairs of steps between a letter's load and its use
-
-__device__ __forceinline__ uint32_t wv_prmt(uint32_t x, uint32_t y, uint32_t sel) { return __byte_perm(x, y, sel); }
-__device__ __forceinline__ uint32_t wv_pk2(int v) { return (uint32_t)(uint16_t)(int16_t)v * 0x10001u; }
-
-// Row word of query position i: byte offset of its table row | bias << 16;
-// the sentinel row outside [0, m).
-__device__ __forceinline__ uint32_t wv_row(const uint32_t* __restrict__ qrow, int i, int m) {
-    return (unsigned)i < (unsigned)m ? __ldg(qrow + i) : (uint32_t)(kWaveSent * kWaveRow);
-}
-// Residue code of window column c, the sentinel code outside [0, n).
-__device__ __forceinline__ uint32_t wv_col(const uint8_t* __restrict__ win, int c, int n) {
-    return (unsigned)c < (unsigned)n ? (uint32_t)__ldg(win + c) : (uint32_t)kWaveSent;
-}
 
 // Jobs [task * 32 / L, ...) of one (L, J) class of the sorted list, one per
 // group of L lanes.
@@ -84,15 +66,7 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
         lo = (int)l64;
         qrow += q0;
         win += jj.win_begin;
-        // anti-diagonals of the cells inside the window
-        const int first = h64 < 0 ? (int)-h64 : 0;
-        int last = n - 1 - lo;
-        if (last > m - 1) last = m - 1;
-        const int s_min = 2 * first + (-lo - first > 0 ? -lo - first : 0);
-        const int k_end = n - 1 - lo - last;
-        const int s_max = 2 * last + (k_end < w - 1 ? k_end : w - 1);
-        s0 = s_min & ~1;
-        nit = (s_max - s0) / 2 + 1;
+        wv_span(m, n, lo, w, s0, nit);
     }
     const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)nit);
     const int go = a.go;
@@ -125,11 +99,6 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
     i0 += kWaveAhead;
     c0 += 2 * J + kWaveAhead;
     uint32_t best = 0;
-    auto sub = [&](uint32_t ra, uint32_t ca, uint32_t rb, uint32_t cb, uint32_t bias) {
-        const uint32_t x = *reinterpret_cast<const uint16_t*>(tab + ra + ca);
-        const uint32_t y = *reinterpret_cast<const uint16_t*>(tab + rb + cb);
-        return __vadd2(wv_prmt(x, y, 0x5410), bias);
-    };
     for (int it = 0; it < nmax; it += kWaveAhead) {
 #pragma unroll
         for (int t = 0; t < kWaveAhead; t++) {
@@ -142,7 +111,7 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
                 const uint32_t Ein = wv_prmt(left, own, 0x5432);
                 left = own;
                 const uint32_t Fin = F[j];
-                const uint32_t ds = __vadd2(Ge[j], sub(R[2 * j], C[2 * j], R[2 * j + 1], C[2 * j + 1], B[j]));
+                const uint32_t ds = __vadd2(Ge[j], wv_sub(tab, R[2 * j], C[2 * j], R[2 * j + 1], C[2 * j + 1], B[j]));
                 const uint32_t H = __vimax3_s16x2_relu(Ein, Fin, ds) & keep_e[j];
                 const uint32_t Gv = __vadd2(H, ngo2);
                 Ge[j] = Gv;
@@ -157,7 +126,7 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
             for (int j = 0; j < J; j++) {
                 const uint32_t Ein = E[j];
                 const uint32_t Fin = wv_prmt(F[j], j + 1 < J ? F[j + 1 < J ? j + 1 : j] : down, 0x5432);
-                const uint32_t ds = __vadd2(Go[j], sub(R[2 * j], C[2 * j + 1], R[2 * j + 1], C[2 * j + 2], B[j]));
+                const uint32_t ds = __vadd2(Go[j], wv_sub(tab, R[2 * j], C[2 * j + 1], R[2 * j + 1], C[2 * j + 2], B[j]));
                 const uint32_t H = __vimax3_s16x2_relu(Ein, Fin, ds) & keep_o[j];
                 const uint32_t Gv = __vadd2(H, ngo2);
                 Go[j] = Gv;
@@ -199,10 +168,7 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
 // a class the list is largest first.
 __global__ void __launch_bounds__(kWaveThreads, 4) k_band_wave(WaveArgs a) {
     __shared__ __align__(4) int16_t tab[25 * kWaveRow / 2];
-    for (int t = threadIdx.x; t < 25 * (kWaveRow / 2); t += blockDim.x) {
-        const int r = t / (kWaveRow / 2), c = t - r * (kWaveRow / 2);
-        tab[t] = r < 24 && c < 24 ? (int16_t)(a.matrix[r * 24 + c] + a.go) : (int16_t)kSent16;
-    }
+    wv_table(tab, a.matrix, a.go);
     __syncthreads();
     const uint8_t* tb = reinterpret_cast<const uint8_t*>(tab);
     const int lane = threadIdx.x & 31;

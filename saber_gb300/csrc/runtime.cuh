@@ -188,7 +188,7 @@ struct saber_gpu {
     std::vector<int32_t> tt_lambda_matrix;  // the matrix whose implied lambda is cached
     double tt_lambda = 0.0;
     // traceback scratch
-    saber::DevBuf al_reqs, al_outs, al_dir, al_opbytes, al_runs, al_slabs, al_packed, al_pack_off;
+    saber::DevBuf al_reqs, al_outs, al_dir, al_opbytes, al_runs, al_slabs, al_packed, al_pack_off, al_next;
 };
 
 namespace saber {

@@ -16,7 +16,7 @@
 #include <thread>
 #include <vector>
 
-#include "band_common.cuh"
+#include "band_wave.cuh"
 #include "saber_gpu.h"
 
 #include "runtime.cuh"
@@ -919,16 +919,20 @@ struct AlignReq {
     int32_t mpad;
     int32_t stop_at;
     int32_t want_dir;
-    int32_t pad_;
+    int32_t zero;
+    const uint32_t* qrow;
 };
 struct AlignOut {
     int32_t status;
     int32_t score;
     uint32_t q_start, q_end, s_start, s_end;
     uint32_t n_ops;
-    uint32_t pad_;
+    uint32_t run_first;
     uint64_t cells;
 };
+constexpr int kAlignRedo = 3;  // a status of launch_align_wave: run the job through launch_band_align
+cudaError_t launch_align_wave(unsigned sm_count, cudaStream_t s, const AlignReq* reqs, uint32_t nreq, uint8_t* dir_pool,
+                              uint32_t* runs, const int32_t* matrix, int go, int ge, uint32_t* next, AlignOut* outs);
 cudaError_t launch_band_align(unsigned grid, cudaStream_t s, const AlignReq* reqs, uint32_t nreq, uint8_t* dir_pool,
                               uint8_t* opbytes, uint32_t* runs, int32_t* slabs, uint32_t slab_stride, int go, int ge,
                               AlignOut* outs);
@@ -966,6 +970,8 @@ using RunPools = std::vector<std::vector<uint32_t>>;
 // 6.6 GB of direction bytes) fits one launch.
 constexpr uint64_t kDirPoolBudget = 8ull << 30;
 constexpr uint64_t kAlignSlabBudget = 512ull << 20;
+// Widest band of the anti-diagonal kernel: 32 lanes x 16 band indices.
+constexpr int64_t kAlignWaveWidth = 512;
 
 static int align_batch(saber_gpu* h, const Scheme& sch, const Dataset& ds, const std::vector<AlignHostReq>& in,
                        uint64_t max_dir_bytes, std::vector<AlignResult>& out, RunPools& pools) {
@@ -1015,20 +1021,38 @@ static int align_batch(saber_gpu* h, const Scheme& sch, const Dataset& ds, const
         for (size_t k = 0; k < todo.size(); k++) sorted[start[cls[k]]++] = todo[k];
         todo.swap(sorted);
     }
+    // the anti-diagonal kernel takes the bands it is built for, the row kernel
+    // the rest and what the first one hands back (stable partition: both keep
+    // the size order)
+    auto by_wave = [&](size_t t) {
+        const AlignHostReq& r = in[t];
+        int64_t lo = r.lo, hi = r.hi;
+        const int64_t m = (int64_t)(qs.offs[r.query + 1] - qs.offs[r.query]);
+        const int64_t w = clip_band(m, r.win_len, lo, hi);
+        return r.want_dir && r.stop_at >= 1 && w <= kAlignWaveWidth && m < (1 << 28) && r.win_len < (1u << 28);
+    };
+    const size_t n_wave = (size_t)(std::stable_partition(todo.begin(), todo.end(), by_wave) - todo.begin());
     cudaStream_t s = h->stream;
     size_t pos = 0;
     while (pos < todo.size()) {
         // one launch: as many jobs as fit the pool budget
+        const bool wave = pos < n_wave;
+        const size_t pos_end = wave ? n_wave : todo.size();
         std::vector<AlignReq> reqs;
         std::vector<size_t> idx;
         uint64_t dir_tot = 0, ops_tot = 0;
         int64_t wmax = 1;
-        while (pos < todo.size()) {
+        while (pos < pos_end) {
             const AlignHostReq& r = in[todo[pos]];
             int64_t m = (int64_t)(qs.offs[r.query + 1] - qs.offs[r.query]);
             int64_t lo = r.lo, hi = r.hi;
             int64_t w = clip_band(m, r.win_len, lo, hi);
             uint64_t dbytes = r.want_dir ? (uint64_t)m * (uint64_t)w : 0;
+            if (wave) {  // one word per pair of steps and four band indices
+                int s0, nit;
+                wv_span((int)m, (int)r.win_len, (int)lo, (int)w, s0, nit);
+                dbytes = (uint64_t)nit * (uint64_t)((w + 3) / 4) * 4;
+            }
             if (!reqs.empty() && dir_tot + dbytes > kDirPoolBudget) break;
             AlignReq q;
             q.win = ds.res.as<uint8_t>() + r.win_begin;
@@ -1042,7 +1066,8 @@ static int align_batch(saber_gpu* h, const Scheme& sch, const Dataset& ds, const
             q.mpad = (int32_t)qs.pmpad[r.query];
             q.stop_at = r.stop_at;
             q.want_dir = r.want_dir ? 1 : 0;
-            q.pad_ = 0;
+            q.zero = 0;
+            q.qrow = qs.qrow.as<uint32_t>() + qs.offs[r.query];
             dir_tot += (dbytes + 15) / 16 * 16;
             if (r.want_dir) ops_tot += (uint64_t)m + r.win_len + 2;
             wmax = std::max(wmax, w);
@@ -1062,13 +1087,21 @@ static int align_batch(saber_gpu* h, const Scheme& sch, const Dataset& ds, const
         CUALLOC(h, h->al_reqs, nreq * sizeof(AlignReq));
         CUALLOC(h, h->al_outs, nreq * sizeof(AlignOut));
         CUALLOC(h, h->al_dir, dir_tot + 16);
-        CUALLOC(h, h->al_opbytes, ops_tot + 16);
         CUALLOC(h, h->al_runs, (ops_tot + 16) * 4);
-        CUALLOC(h, h->al_slabs, (thr / 32) * stride * 16);
         CU(h, cudaMemcpyAsync(h->al_reqs.p, reqs.data(), nreq * sizeof(AlignReq), cudaMemcpyHostToDevice, s));
-        CU(h, launch_band_align(grid, s, h->al_reqs.as<AlignReq>(), nreq, h->al_dir.as<uint8_t>(),
-                                h->al_opbytes.as<uint8_t>(), h->al_runs.as<uint32_t>(), h->al_slabs.as<int32_t>(),
-                                stride, sch.go, sch.ge, h->al_outs.as<AlignOut>()));
+        if (wave) {
+            CUALLOC(h, h->al_next, 4);
+            CU(h, cudaMemsetAsync(h->al_next.p, 0, 4, s));
+            CU(h, launch_align_wave((unsigned)h->sm_count, s, h->al_reqs.as<AlignReq>(), nreq, h->al_dir.as<uint8_t>(),
+                                    h->al_runs.as<uint32_t>(), sch.d_matrix.as<int32_t>(), sch.go, sch.ge,
+                                    h->al_next.as<uint32_t>(), h->al_outs.as<AlignOut>()));
+        } else {
+            CUALLOC(h, h->al_opbytes, ops_tot + 16);
+            CUALLOC(h, h->al_slabs, (thr / 32) * stride * 16);
+            CU(h, launch_band_align(grid, s, h->al_reqs.as<AlignReq>(), nreq, h->al_dir.as<uint8_t>(),
+                                    h->al_opbytes.as<uint8_t>(), h->al_runs.as<uint32_t>(), h->al_slabs.as<int32_t>(),
+                                    stride, sch.go, sch.ge, h->al_outs.as<AlignOut>()));
+        }
         std::vector<AlignOut> outs(nreq);
         CU(h, cudaMemcpyAsync(outs.data(), h->al_outs.p, nreq * sizeof(AlignOut), cudaMemcpyDeviceToHost, s));
         CU(h, cudaStreamSynchronize(s));
@@ -1077,7 +1110,7 @@ static int align_batch(saber_gpu* h, const Scheme& sch, const Dataset& ds, const
         std::vector<uint32_t> cnt(nreq);
         uint64_t packed = 0;
         for (uint32_t t = 0; t < nreq; t++) {
-            src[t] = reqs[t].ops_off;
+            src[t] = reqs[t].ops_off + outs[t].run_first;
             dst[t] = packed;
             cnt[t] = outs[t].n_ops;
             packed += outs[t].n_ops;
@@ -1103,6 +1136,10 @@ static int align_batch(saber_gpu* h, const Scheme& sch, const Dataset& ds, const
         for (uint32_t t = 0; t < nreq; t++) {
             AlignResult& r = out[idx[t]];
             const AlignOut& o = outs[t];
+            if (wave && o.status == kAlignRedo) {
+                todo.push_back(idx[t]);
+                continue;
+            }
             r.status = o.status;
             r.score = o.score;
             r.q_start = o.q_start;
