@@ -364,16 +364,28 @@ __global__ void __launch_bounds__(kTtWarps * 32, 4) k_tantan(const __grid_consta
 // and IEEE addition commutes), and the remaining states W mod 8 sit in
 // register W/8 of lanes 0.. and are added by broadcast, in order.
 //
-// Partner codes come from a per-group ring of 128 codes in shared memory,
-// stored twice (slots q & 127 and 128 + (q & 127)) so that the code of
-// position p-1-k-8j is at the fixed offset ((p-1-k) & 127) + 128 - 8j; ring
-// slots of positions before the sequence hold 24 (no partner, ratio 0).
-// The scratch row of a position keeps lane k's eight states contiguous
-// (index 8k + j: two 16-byte stores per lane).
+// Partner codes x[p-1-i] of a lane's states are bytes of two registers (j =
+// 0..3 and 4..6).  A position's move shifts every state's code to the next
+// state: one shuffle of each register to the neighbouring lane, the group's
+// end lane moving them by a byte and taking the code that enters (24, no
+// partner, ratio 0, before the sequence).
+//
+// The emission ratios stand in shared memory once per lane (word 32 (25 a +
+// c) + lane), so that the seven random reads of a position are free of bank
+// conflicts.
+//
+// A position's scratch row is two quads of states (j = 0..3, 4..7), each
+// contiguous over the group's lanes: every 16-byte access of a group fills a
+// 128-byte line.  The backward pass keeps D rows in flight in registers.
+//
+// One GB300 (before: codes from a ring in shared memory, one table of ratios
+// for a block, rows one position ahead): 600 k residues with posteriors 1.52
+// -> 0.86 ms a call, bound by the serial chain of its longest sequences; 30 M
+// residues 7.3 -> 4.0 ms, bound by the rows (7.7 GB written and read) and
+// issue.
 constexpr int kTg = 8;          // lanes per sequence
 constexpr int kTgSeqs = 4;      // sequences per warp
-constexpr int kRingPitch = 264; // bytes per group ring (256 + 8: the two words a group reads never share a
-                                // bank with the neighbouring groups')
+constexpr size_t kTgTabBytes = 24 * 25 * 32 * sizeof(float);
 
 template <int W>
 __device__ __forceinline__ float tg_sum(const float (&v)[8]) {
@@ -392,28 +404,22 @@ __device__ __forceinline__ float tg_sum(const float (&v)[8]) {
     return acc;
 }
 
-// Ring chunk c (positions 32c .. 32c+31) of one group: lane k loads the
-// codes of positions 32c + 4k .. 32c + 4k + 3 (24 before the sequence) as
-// one word and stores it into both copies of the ring.
-__device__ __forceinline__ uint32_t tg_load(const uint8_t* __restrict__ x, int64_t n, int64_t c, int k) {
-    const int64_t q0 = 32 * c + 4 * k;
-    uint32_t word = 0;
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-        const int64_t q = q0 + t;
-        const uint32_t code = q < 0 ? 24u : (q < n ? (uint32_t)min((int)x[q], 23) : 0u);
-        word |= code << (8 * t);
-    }
-    return word;
-}
-__device__ __forceinline__ void tg_store(uint8_t* ring, int64_t c, int k, uint32_t word) {
-    const int slot = (int)((32 * c + 4 * k) & 127);
-    *reinterpret_cast<uint32_t*>(ring + slot) = word;
-    *reinterpret_cast<uint32_t*>(ring + 128 + slot) = word;
+// Code of position q of a sequence: 24 before it, 0 past its end.
+__device__ __forceinline__ uint32_t tg_code(const uint8_t* __restrict__ x, int q, int n) {
+    return q < 0 ? 24u : (q < n ? (uint32_t)min((int)x[q], 23) : 0u);
 }
 
-template <int W>
-__global__ void __launch_bounds__(kTtWarps * 32, 4) k_tantan8(const __grid_constant__ TantanModel M,
+// Emission ratios of a lane's states for residue row `row` (the lane's column
+// of the table).
+template <int J>
+__device__ __forceinline__ void tg_emit(const float* row, uint32_t ca, uint32_t cb, float (&e)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        e[j] = j < J ? row[32 * __byte_perm(j < 4 ? ca : cb, 0u, 0x4440u | (uint32_t)(j & 3))] : 0.f;
+}
+
+template <int W, int D, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) k_tantan8(const __grid_constant__ TantanModel M,
                                                               const uint8_t* __restrict__ codes,
                                                               const uint64_t* __restrict__ offs,
                                                               const uint32_t* __restrict__ ord,
@@ -422,186 +428,180 @@ __global__ void __launch_bounds__(kTtWarps * 32, 4) k_tantan8(const __grid_const
                                                               float2* __restrict__ fwdBS, uint8_t* __restrict__ mask,
                                                               float* __restrict__ probs,
                                                               unsigned long long* __restrict__ n_masked) {
-    static_assert(W >= 1 && W <= kTtMaxW, "repeat states");
+    static_assert(W >= 1 && W <= 56, "repeat states in seven registers");
+    static_assert(8 % D == 0, "rows in flight divide the unrolled positions");
     constexpr int J = (W + 7) / 8;  // registers holding states
-    __shared__ float lr[24 * 33];
-    __shared__ __align__(16) uint8_t rings[kTtWarps * kTgSeqs * kRingPitch];
-    for (int i = threadIdx.x; i < 24 * 33; i += blockDim.x) {
-        const int r = i / 33, c = i % 33;
-        lr[i] = c < 32 ? M.lr[r * 32 + c] : 0.f;
+    extern __shared__ __align__(16) float lr[];
+    for (int i = threadIdx.x; i < 24 * 25 * 32; i += blockDim.x) {
+        const int r = i / (25 * 32), c = (i / 32) % 25;
+        lr[i] = c < 24 ? M.lr[r * 32 + c] : 0.f;
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, g = lane >> 3, k = lane & 7;
     const int wib = threadIdx.x >> 5;
-    uint8_t* ring = rings + (wib * kTgSeqs + g) * kRingPitch;
     const uint64_t kk = k0 + ((uint64_t)blockIdx.x * (blockDim.x >> 5) + wib) * kTgSeqs + g;
-    int64_t n = 0;
+    int n = 0;  // (host: sequences are shorter than 2^31)
     uint64_t st = 0;
     float* F = fwdF;
     float2* BS = fwdBS;
     if (kk < k1) {
         const uint32_t sid = ord[kk];
         st = offs[sid];
-        n = (int64_t)(offs[sid + 1] - st);
-        F = fwdF + base[kk] * (uint64_t)kTtMaxW + 8 * k;
+        n = (int)(offs[sid + 1] - st);
+        F = fwdF + base[kk] * (uint64_t)kTtMaxW + 4 * k;
         BS = fwdBS + base[kk];
     }
-    const int64_t nmax = (int64_t)__reduce_max_sync(kFull, (unsigned)n);
+    const int nmax = (int)__reduce_max_sync(kFull, (unsigned)n);
     if (nmax == 0) return;
+    const int pend = (nmax - 1) & ~7;  // first position of the last block of eight
     const uint8_t* x = codes + st;
+    const float* tab = lr + lane;
     float b2f[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) b2f[j] = j < J ? M.b2f[k + 8 * j] : 0.f;
     const float b2b = M.b2b, f2f = M.f2f, f2b = M.f2b;
-    // ring: 24 everywhere (positions before the sequence), then chunks 0 and 1
-#pragma unroll
-    for (int t = 0; t < 8; t++) *reinterpret_cast<uint32_t*>(ring + 32 * t + 4 * k) = 0x18181818u;
-    __syncwarp();
 
     // ---- forward (masking.rs:476-497) ----
     float pb = 1.f, pf[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) pf[j] = 0.f;
-    float mb = 0.f, ms = 0.f;
-    uint32_t wnext = tg_load(x, n, 0, k);  // codes one chunk ahead
-    for (int64_t p = 0; p < nmax; p++) {
-        if ((p & 31) == 0) {
-            __syncwarp();
-            tg_store(ring, p >> 5, k, wnext);
-            __syncwarp();
-            wnext = tg_load(x, n, (p >> 5) + 1, k);
-        }
-        const int xrow = 33 * (int)ring[p & 127];
-        const uint8_t* rp = ring + ((p - 1 - k) & 127) + 128;
-        float e[8];
+    uint32_t ca = 0x18181818u, cb = 0x18181818u;
+    uint32_t cx = tg_code(x, k, n), cxn = tg_code(x, 8 + k, n);  // codes of this block of eight and the next
+    for (int64_t p0 = 0; p0 <= pend; p0 += 8) {
+        float mb = 0.f, ms = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; j++) e[j] = j < J ? lr[xrow + rp[-8 * j]] : 0.f;
-        const float sum_f = tg_sum<W>(pf);
-        float c[8];
+        for (int t = 0; t < 8; t++) {
+            const int64_t p = p0 + t;
+            const uint32_t xp = __shfl_sync(kFull, cx, t, kTg);
+            float e[8];
+            tg_emit<J>(tab + 800 * xp, ca, cb, e);
+            const float sum_f = tg_sum<W>(pf);
+            float c[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++) c[j] = __fmul_rn(__fadd_rn(__fmul_rn(pb, b2f[j]), __fmul_rn(pf[j], f2f)), e[j]);
-        const float cb = __fadd_rn(__fmul_rn(pb, b2b), __fmul_rn(sum_f, f2b));
-        const float tot = __fadd_rn(cb, tg_sum<W>(c));
-        const float s = tot > 0.f ? __fdiv_rn(1.f, tot) : 1.f;
-        pb = __fmul_rn(cb, s);
+            for (int j = 0; j < 8; j++)
+                c[j] = __fmul_rn(__fadd_rn(__fmul_rn(pb, b2f[j]), __fmul_rn(pf[j], f2f)), e[j]);
+            const float cbk = __fadd_rn(__fmul_rn(pb, b2b), __fmul_rn(sum_f, f2b));
+            const float tot = __fadd_rn(cbk, tg_sum<W>(c));
+            const float s = tot > 0.f ? __frcp_rn(tot) : 1.f;  // = 1 / tot, correctly rounded
+            pb = __fmul_rn(cbk, s);
 #pragma unroll
-        for (int j = 0; j < 8; j++) pf[j] = __fmul_rn(c[j], s);
-        if (p < n) {
-            float4* row = reinterpret_cast<float4*>(F + p * kTtMaxW);
-            row[0] = make_float4(pf[0], pf[1], pf[2], pf[3]);
-            row[1] = make_float4(pf[4], pf[5], pf[6], pf[7]);
+            for (int j = 0; j < 8; j++) pf[j] = __fmul_rn(c[j], s);
+            if (p < n) {
+                float* row = F + p * kTtMaxW;
+                *reinterpret_cast<float4*>(row) = make_float4(pf[0], pf[1], pf[2], pf[3]);
+                *reinterpret_cast<float4*>(row + 32) = make_float4(pf[4], pf[5], pf[6], pf[7]);
+            }
+            if (k == t) {
+                mb = pb;
+                ms = s;
+            }
+            // states' partners at p + 1: x[p] enters at state 0
+            const uint32_t na = __shfl_sync(kFull, ca, k - 1, kTg), nb = __shfl_sync(kFull, cb, k - 1, kTg);
+            ca = k ? na : ((na << 8) | xp);
+            cb = k ? nb : __funnelshift_l(na, nb, 8);
         }
-        const int j8 = (int)(p & 7);
-        if (k == j8) {
-            mb = pb;
-            ms = s;
-        }
-        if (j8 == 7 || p == nmax - 1) {
-            const int64_t q = (p & ~(int64_t)7) + k;
-            if (q < n && q <= p) BS[q] = make_float2(mb, ms);
-        }
+        const int64_t q = p0 + k;
+        if (q < n) BS[q] = make_float2(mb, ms);
+        cx = cxn;
+        cxn = p0 + 16 + k < n ? tg_code(x, (int)p0 + 16 + k, n) : 0u;
     }
 
     // ---- backward with the same scales (masking.rs:499-528) ----
     float nb = 1.f, nf[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) nf[j] = f2b;
-    // B values and scales one block of eight positions ahead, codes one
-    // chunk ahead, the F row one position ahead
-    auto bs_load = [&](int64_t blk) {
-        const int64_t q = 8 * blk + k;
-        return blk >= 0 && q < n ? BS[q] : make_float2(0.f, 0.f);
+    // B values, scales, codes and the codes that enter one block of eight
+    // positions ahead, the F rows D positions ahead
+    auto bs_load = [&](int p0) { return p0 >= 0 && p0 + k < n ? BS[p0 + k] : make_float2(0.f, 0.f); };
+    auto row_load = [&](int64_t p, float4& a, float4& b) {
+        a = b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p >= 0 && p < n) {
+            const float* row = F + p * kTtMaxW;
+            a = *reinterpret_cast<const float4*>(row);
+            b = *reinterpret_cast<const float4*>(row + 32);
+        }
     };
-    float2 bs = bs_load((nmax - 1) >> 3), bsn = bs_load(((nmax - 1) >> 3) - 1);
-    float keep = 0.f;
-    unsigned masked = 0;
-    float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb4 = ra;
+    float2 bs = bs_load(pend), bsn = bs_load(pend - 8);
+    cx = tg_code(x, pend + k, n);
+    cxn = tg_code(x, pend - 8 + k, n);
+    // state 55's partner at position p - 1 is x[p - 57]
+    uint32_t in = tg_code(x, pend - 57 + k, n), inn = tg_code(x, pend - 65 + k, n);
     {
-        const int64_t p = nmax - 1;
-        if (p < n) {
-            const float4* row = reinterpret_cast<const float4*>(F + p * kTtMaxW);
-            ra = row[0];
-            rb4 = row[1];
-        }
-        const uint32_t w0 = tg_load(x, n, p >> 5, k), w1 = tg_load(x, n, (p >> 5) - 1, k),
-                       w2 = tg_load(x, n, (p >> 5) - 2, k);
-        __syncwarp();
-        tg_store(ring, p >> 5, k, w0);
-        tg_store(ring, (p >> 5) - 1, k, w1);
-        tg_store(ring, (p >> 5) - 2, k, w2);
-        __syncwarp();
-        wnext = tg_load(x, n, (p >> 5) - 3, k);
-    }
-    for (int64_t p = nmax - 1; p >= 0; p--) {
-        if ((p & 31) == 31 && p != nmax - 1) {
-            __syncwarp();
-            tg_store(ring, (p >> 5) - 2, k, wnext);
-            __syncwarp();
-            wnext = tg_load(x, n, (p >> 5) - 3, k);
-        }
-        const int j8 = (int)(p & 7);
-        if (j8 == 7 && p != nmax - 1) {
-            bs = bsn;
-            bsn = bs_load((p >> 3) - 1);
-        }
-        float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb4 = na;
-        if (p > 0 && p - 1 < n) {
-            const float4* row = reinterpret_cast<const float4*>(F + (p - 1) * kTtMaxW);
-            na = row[0];
-            nb4 = row[1];
-        }
-        const float rbv = __shfl_sync(kFull, bs.x, j8, kTg), s = __shfl_sync(kFull, bs.y, j8, kTg);
-        const float r[8] = {ra.x, ra.y, ra.z, ra.w, rb4.x, rb4.y, rb4.z, rb4.w};
-        const bool active = p < n;
-        const float onb = nb;
-        float onf[8];
+        const int p = pend + 7;
+        ca = cb = 0;
 #pragma unroll
-        for (int j = 0; j < 8; j++) onf[j] = nf[j];
-        {
-            const int xrow = 33 * (int)ring[p & 127];
-            const uint8_t* rp = ring + ((p - 1 - k) & 127) + 128;
-            float be[8], t[8];
+        for (int j = 0; j < 4; j++) {
+            ca |= tg_code(x, p - 1 - k - 8 * j, n) << (8 * j);
+            cb |= tg_code(x, p - 33 - k - 8 * j, n) << (8 * j);
+        }
+    }
+    float4 ra[D], rb[D];
+#pragma unroll
+    for (int d = 0; d < D; d++) row_load((int64_t)pend + 7 - d, ra[d], rb[d]);
+    unsigned masked = 0;
+    for (int64_t p0 = pend; p0 >= 0; p0 -= 8) {
+        float kp = 0.f, kz = 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int t = 7 - u;
+            const int64_t p = p0 + t;
+            const float r[8] = {ra[u % D].x, ra[u % D].y, ra[u % D].z, ra[u % D].w,
+                                rb[u % D].x, rb[u % D].y, rb[u % D].z, rb[u % D].w};
+            row_load(p - D, ra[u % D], rb[u % D]);
+            const float rbv = __shfl_sync(kFull, bs.x, t, kTg), s = __shfl_sync(kFull, bs.y, t, kTg);
+            const uint32_t xp = __shfl_sync(kFull, cx, t, kTg), xin = __shfl_sync(kFull, in, t, kTg);
+            float pr[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) pr[j] = __fmul_rn(r[j], nf[j]);
+            const float pbv = __fmul_rn(rbv, nb);
+            float be[8], tt[8];
+            tg_emit<J>(tab + 800 * xp, ca, cb, be);
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                be[j] = j < J ? __fmul_rn(lr[xrow + rp[-8 * j]], onf[j]) : 0.f;
-                t[j] = __fmul_rn(b2f[j], be[j]);
+                be[j] = j < J ? __fmul_rn(be[j], nf[j]) : 0.f;
+                tt[j] = __fmul_rn(b2f[j], be[j]);
             }
-            const float to_fg = tg_sum<W>(t);
-            if (active && p > 0) {
-                const float fb = __fmul_rn(f2b, onb);
+            const float to_fg = tg_sum<W>(tt);
+            if (p < n && p > 0) {
+                const float fb = __fmul_rn(f2b, nb);
 #pragma unroll
                 for (int j = 0; j < 8; j++) nf[j] = __fmul_rn(__fadd_rn(__fmul_rn(f2f, be[j]), fb), s);
-                nb = __fmul_rn(__fadd_rn(__fmul_rn(b2b, onb), to_fg), s);
+                nb = __fmul_rn(__fadd_rn(__fmul_rn(b2b, nb), to_fg), s);
             }
-        }
-        float pr[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) pr[j] = __fmul_rn(r[j], onf[j]);
-        const float pbv = __fmul_rn(rbv, onb);
-        const float pfv = tg_sum<W>(pr);
-        const float z = __fadd_rn(pbv, pfv);
-        const float post = z > 0.f ? __fdiv_rn(pfv, z) : 0.f;
-        if (k == j8) keep = post;
-        if (j8 == 0) {
-            const int64_t q = p + k;
-            const bool ok = q < n;
-            const bool m = ok && (double)keep >= M.min_prob;
-            if (ok) {
-                mask[st + q] = m ? 1 : 0;
-                if (probs) probs[st + q] = keep;
+            const float pfv = tg_sum<W>(pr);
+            if (k == t) {
+                kp = pfv;
+                kz = __fadd_rn(pbv, pfv);
             }
-            masked += __popc(__ballot_sync(kFull, m));
+            // states' partners at p - 1: x[p - 57] enters at state 55
+            const uint32_t da = __shfl_sync(kFull, ca, k + 1, kTg), db = __shfl_sync(kFull, cb, k + 1, kTg);
+            ca = k < 7 ? da : __funnelshift_r(da, db, 8);
+            cb = k < 7 ? db : __byte_perm(db, xin, 0x3421);  // bytes 1, 2, x[p - 57], unused
         }
-        ra = na;
-        rb4 = nb4;
+        const float post = kz > 0.f ? __fdiv_rn(kp, kz) : 0.f;
+        const int64_t q = p0 + k;
+        const bool ok = q < n;
+        const bool m = ok && (double)post >= M.min_prob;
+        if (ok) {
+            mask[st + q] = m ? 1 : 0;
+            if (probs) probs[st + q] = post;
+        }
+        masked += __popc(__ballot_sync(kFull, m));
+        bs = bsn;
+        bsn = bs_load((int)p0 - 16);
+        cx = cxn;
+        cxn = tg_code(x, (int)p0 - 16 + k, n);
+        in = inn;
+        inn = tg_code(x, (int)p0 - 73 + k, n);
     }
     if (lane == 0 && masked) atomicAdd(n_masked, (unsigned long long)masked);
 }
 
 // ---- host driver ------------------------------------------------------------------
 
-// Scratch rows (positions) per launch: 64 F floats + one float2 each.
-constexpr uint64_t kTtRowsPerLaunch = 8ull << 20;
+// Scratch rows (positions) per launch: 64 F floats + one float2 each (8.9 GB;
+// 30 M residues are one launch, which ends once instead of four times).
+constexpr uint64_t kTtRowsPerLaunch = 32ull << 20;
 
 // Masks the sequences [offs[i], offs[i+1]) of the device residues d_codes
 // (offsets on the host: h_offs; on the device: d_offs) into d_mask (one byte
@@ -659,15 +659,27 @@ int tantan_run(saber_gpu* h, const TantanModel& M, const uint8_t* d_codes, const
     for (size_t c = 0; c + 1 < cuts.size(); c++) {
         const uint64_t k0 = cuts[c], k1 = cuts[c + 1];
         if (M.w == 50) {  // tantan's protein default: eight lanes per sequence
-            // a batch too small to fill every SM with full blocks (a query
-            // batch) runs two warps per block: more SMs, less contention
-            // on each sequence's serial chain
-            const unsigned warps = (k1 - k0) < (uint64_t)h->sm_count * kTtWarps * kTgSeqs ? 2u : kTtWarps;
-            const uint64_t per_block = (uint64_t)warps * kTgSeqs;
-            const unsigned blocks = (unsigned)((k1 - k0 + per_block - 1) / per_block);
-            k_tantan8<50><<<blocks, warps * 32, 0, h->stream>>>(
-                M, d_codes, d_offs, (const uint32_t*)h->tt_ord.p, (const uint64_t*)h->tt_base.p, k0, k1,
-                (float*)h->tt_F.p, (float2*)h->tt_BS.p, d_mask, d_probs, (unsigned long long*)h->tt_count.p);
+            // Shape by sequences per SM: two warps per block and eight rows in
+            // flight while latency rules (one sequence's serial chain is the
+            // launch), more warps and fewer rows in flight as the memory
+            // traffic takes over.  Calls of 2,400 / 20,000 / 40,000 / 100,000
+            // sequences on one GB300: two warps 0.86 / 1.42 / 2.75 / 6.8 ms,
+            // eight warps 1.06 / 1.49 / 1.84 / 4.2, twelve 1.31 / 1.82 / 2.18
+            // / 4.0.
+            auto go = [&](auto kern, unsigned warps) -> int {
+                const uint64_t per_block = (uint64_t)warps * kTgSeqs;
+                const unsigned blocks = (unsigned)((k1 - k0 + per_block - 1) / per_block);
+                CU(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTgTabBytes));
+                kern<<<blocks, warps * 32, kTgTabBytes, h->stream>>>(
+                    M, d_codes, d_offs, (const uint32_t*)h->tt_ord.p, (const uint64_t*)h->tt_base.p, k0, k1,
+                    (float*)h->tt_F.p, (float2*)h->tt_BS.p, d_mask, d_probs, (unsigned long long*)h->tt_count.p);
+                return SABER_OK;
+            };
+            const uint64_t per_sm = (k1 - k0) / (uint64_t)h->sm_count;
+            const int rc = per_sm < 128   ? go(k_tantan8<50, 8, 64, 2>, 2)
+                           : per_sm < 400 ? go(k_tantan8<50, 4, 256, 2>, 8)
+                                          : go(k_tantan8<50, 1, 384, 2>, 12);
+            if (rc) return rc;
             CU(h, cudaGetLastError());
             continue;
         }
