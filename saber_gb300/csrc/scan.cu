@@ -263,9 +263,9 @@ struct ScanArgs {
     const uint2* grp;                // rank-compressed presence tables of all shapes
     const uint2* rng;                // rank -> (first entry, entries) of all shapes
     const uint32_t* qent;            // batch positions of all shapes
-    const uint4* qwin;               // per batch position: seed-letter window record (32 bytes)
-    const uint4* qwinx;              // per batch position: full-code window record (32 bytes)
-    const uint8_t* cb;               // combined filter codes of the database (combined mode)
+    const uint4* qwin;               // per batch position: window record (32 bytes; planes or seed letters)
+    const uint4* qwinx;              // per batch position: full-code window record (32 bytes; not in plane mode)
+    const uint4* pl;                 // bit planes of the database, a block of 32 positions in front (plane mode)
     int cfil;
     uint32_t min_ids, kx;
     uint32_t s0, s1, asize;          // this pass's shapes [s0, s1)
@@ -310,6 +310,32 @@ __device__ __forceinline__ void ld256(uint32_t (&v)[8], const void* p) {
         : "l"(p));
 }
 
+// The window filter on bit planes.  A window of 32 letters is eight words, bit
+// t of word p being bit p of letter t's code: words 0..3 the reduced letter,
+// 4..6 the residue's index within its letter's group, 7 whether the letter
+// counts.  Two windows compare in seven three-input logic operations (a byte
+// per letter took about ten instructions per four letters, and an unaligned
+// read of nine words for the subject).
+//
+// The subject window of position r: two neighbouring blocks of the
+// database's planes, funnel-shifted; the letters outside the subject (rd =
+// its rem | dst << 8) do not count.
+__device__ __forceinline__ void subject_planes(const ScanArgs& a, uint64_t r, uint32_t rd, uint32_t (&S)[8]) {
+    const int64_t o = (int64_t)r + a.cfil - 16 + 32;
+    const uint4* b = a.pl + 2 * (o >> 5);
+    const uint32_t sh = (uint32_t)o & 31u;
+    const uint4 x0 = __ldg(b), x1 = __ldg(b + 1), y0 = __ldg(b + 2), y1 = __ldg(b + 3);
+    S[0] = __funnelshift_r(x0.x, y0.x, sh);
+    S[1] = __funnelshift_r(x0.y, y0.y, sh);
+    S[2] = __funnelshift_r(x0.z, y0.z, sh);
+    S[3] = __funnelshift_r(x0.w, y0.w, sh);
+    S[4] = __funnelshift_r(x1.x, y1.x, sh);
+    S[5] = __funnelshift_r(x1.y, y1.y, sh);
+    S[6] = __funnelshift_r(x1.z, y1.z, sh);
+    const int sdst = (int)(rd >> 8), srem = (int)(rd & 0xFFu);
+    S[7] = __funnelshift_r(x1.w, y1.w, sh) & lane_range(max(0, 16 - a.cfil - sdst), min(32, srem + 16 - a.cfil));
+}
+
 // 8 words of a staged byte buffer from byte `idx` on (9 aligned word reads
 // and a funnel shift).
 __device__ __forceinline__ void staged_words(const uint32_t* buf, int idx, uint32_t (&S)[8]) {
@@ -350,7 +376,8 @@ struct WarpScan {
     uint8_t* seg_sh;   // kSegCap: shape
     uint2* sv;         // kSurvStage survivor records
     const uint32_t* sbw;   // 32 staged words: seed letters of [base - 32, base + 96)
-    const uint32_t* resw;  // 32 staged words: residues of the same range
+    const uint32_t* resw;  // 32 staged words: residues of the same range (not in plane mode)
+    const uint4* win;      // plane windows of the 32 positions (plane mode, k_scan)
     uint32_t nsv;      // staged survivors (warp-uniform)
     uint32_t rd;       // this lane's position: rem | dst << 8
     const uint16_t* rds;   // the same of every staged position (k_scan_few)
@@ -426,26 +453,28 @@ __device__ __forceinline__ void scan_flush(const ScanArgs& a, int lane, int nseg
             if (a.min_ids == 0) {
                 pass = true;
             } else if (COMB) {
-                // one compare of combined codes: equal low nibbles are
-                // reduced-letter identities, equal bytes exact ones; the
-                // reference's decision (ids >= min_ids, else ids + kx * exact
-                // >= min_ids) is ids + kx * exact >= min_ids since exact <= ids
+                // the reference's decision (ids >= min_ids, else ids + kx *
+                // exact >= min_ids) is ids + kx * exact >= min_ids since
+                // exact <= ids
                 uint32_t Q[8], S[8];
                 ld256(Q, a.qwin + 2 * (uint64_t)g);
-                const int idx = rl + a.cfil + 16;  // staged byte of r + cfil - 16
-                staged_words(ws.resw, idx, S);
-                const int sdst = (int)(srd >> 8), srem = (int)(srd & 0xFFu);
-                const uint32_t L = lane_range(max(0, 16 - a.cfil - sdst), min(32, srem + 16 - a.cfil));
-                uint32_t Er = 0, Ee = 0;
-#pragma unroll
-                for (int w = 0; w < 8; w++) {
-                    const uint32_t x = Q[w] ^ S[w];
-                    const uint32_t zr = ~((x & 0x0F0F0F0Fu) + 0x0F0F0F0Fu) & 0x10101010u;
-                    const uint32_t ze = ~(((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;
-                    Er |= (((zr >> 4) * 0x10204080u) >> 28) << (4 * w);
-                    Ee |= (((ze >> 7) * 0x10204080u) >> 28) << (4 * w);
+                if (RDS) {
+                    subject_planes(a, ws.base + rl, srd, S);
+                } else {
+                    const uint4 x0 = ws.win[2 * rl], x1 = ws.win[2 * rl + 1];
+                    S[0] = x0.x;
+                    S[1] = x0.y;
+                    S[2] = x0.z;
+                    S[3] = x0.w;
+                    S[4] = x1.x;
+                    S[5] = x1.y;
+                    S[6] = x1.z;
+                    S[7] = x1.w;
                 }
-                pass = __popc(Er & L) + a.kx * __popc(Ee & L) >= a.min_ids;
+                const uint32_t dr = (Q[0] ^ S[0]) | (Q[1] ^ S[1]) | (Q[2] ^ S[2]) | (Q[3] ^ S[3]);
+                const uint32_t Er = Q[7] & S[7] & ~dr;
+                const uint32_t Ee = Er & ~((Q[4] ^ S[4]) | (Q[5] ^ S[5]) | (Q[6] ^ S[6]));
+                pass = __popc(Er) + a.kx * __popc(Ee) >= a.min_ids;
             } else {
                 uint32_t Q[8], S[8];
                 ld256(Q, a.qwin + 2 * (uint64_t)g);
@@ -503,7 +532,8 @@ __global__ void __launch_bounds__(256, SABER_SCAN_MIN_BLOCKS) k_scan(ScanArgs a)
     __shared__ uint32_t s_n[kScanWarps][kSegCap], s_eb[kScanWarps][kSegCap];
     __shared__ uint8_t s_rl[kScanWarps][kSegCap], s_sh[kScanWarps][kSegCap];
     __shared__ uint2 s_sv[kScanWarps][kSurvStage];
-    __shared__ uint32_t s_sbw[kScanWarps][32], s_resw[kScanWarps][32];
+    __shared__ uint32_t s_sbw[kScanWarps][32], s_resw[COMB ? 1 : kScanWarps][32];
+    __shared__ uint4 s_win[COMB ? kScanWarps : 1][64];
     __shared__ ShapeDev s_shape[kMaxShapes];
     for (uint32_t i = threadIdx.x; i < a.s1; i += blockDim.x) s_shape[i] = a.sh[i];
     __syncthreads();
@@ -511,16 +541,23 @@ __global__ void __launch_bounds__(256, SABER_SCAN_MIN_BLOCKS) k_scan(ScanArgs a)
     const uint64_t warp0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long hits = 0, filtered = 0;
-    WarpScan ws{s_n[w], s_eb[w], s_rl[w], s_sh[w], s_sv[w], s_sbw[w], s_resw[w], 0u, 0u, nullptr, 0u};
+    WarpScan ws{s_n[w], s_eb[w], s_rl[w], s_sh[w], s_sv[w], s_sbw[w], s_resw[COMB ? 0 : w], s_win[COMB ? w : 0],
+                0u, 0u, nullptr, 0u};
     const uint8_t* stb = reinterpret_cast<const uint8_t*>(s_sbw[w]) + 32 + lane;  // this lane's position
     for (uint64_t base = warp0 * 32; base < a.N; base += nwarps * 32) {
         const uint64_t r = base + lane;
         const int64_t wb = (int64_t)base - 32 + 4 * lane;
         __syncwarp();
         s_sbw[w][lane] = stage_word(a.sb, wb, a.N, kNonSeed);
-        s_resw[w][lane] = COMB ? stage_word(a.cb, wb, a.N, 0xEEu) : stage_word(a.res, wb, a.N, 0xFFu);
+        if (!COMB) s_resw[w][lane] = stage_word(a.res, wb, a.N, 0xFFu);
         const int rem = r < a.N ? a.rem[r] : 0;
         ws.rd = r < a.N ? ((uint32_t)rem | ((uint32_t)a.dst[r] << 8)) : 0u;
+        if (COMB && a.min_ids) {
+            uint32_t S[8];
+            subject_planes(a, r, ws.rd, S);
+            s_win[w][2 * lane] = make_uint4(S[0], S[1], S[2], S[3]);
+            s_win[w][2 * lane + 1] = make_uint4(S[4], S[5], S[6], S[7]);
+        }
         ws.base = base;
         __syncwarp();
         int nseg = 0;
@@ -595,7 +632,7 @@ constexpr int kFewWarps = 32, kFewPos = 128, kFewSeg = 96;
 struct FewWarp {
     uint32_t seg_n[kFewSeg], seg_eb[kFewSeg];
     uint2 sv[kSurvStage];
-    uint32_t sbw[kFewPos / 4 + 32], resw[kFewPos / 4 + 32];
+    uint32_t sbw[kFewPos / 4 + 32], resw[kFewPos / 4 + 32];  // (resw: not in plane mode)
     uint16_t rds[kFewPos];
     uint16_t q[64];
     uint8_t seg_rl[kFewSeg], seg_sh[kFewSeg];
@@ -616,7 +653,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) k_scan_few(const __grid_con
     const uint64_t warp0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     unsigned long long hits = 0, filtered = 0;
-    WarpScan ws{fw.seg_n, fw.seg_eb, fw.seg_rl, fw.seg_sh, fw.sv, fw.sbw, fw.resw, 0u, 0u, fw.rds, 0u};
+    WarpScan ws{fw.seg_n, fw.seg_eb, fw.seg_rl, fw.seg_sh, fw.sv, fw.sbw, fw.resw, nullptr, 0u, 0u, fw.rds, 0u};
     const uint8_t* stb = reinterpret_cast<const uint8_t*>(fw.sbw) + 32;
     const uint32_t lanes_lt = (1u << lane) - 1u;
     int nseg = 0;
@@ -658,7 +695,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) k_scan_few(const __grid_con
         for (int t = 0; t < 2; t++) {
             const int64_t wb = (int64_t)base - 32 + 4 * (lane + 32 * t);
             fw.sbw[lane + 32 * t] = stage_word(a.sb, wb, a.N, kNonSeed);
-            fw.resw[lane + 32 * t] = COMB ? stage_word(a.cb, wb, a.N, 0xEEu) : stage_word(a.res, wb, a.N, 0xFFu);
+            if (!COMB) fw.resw[lane + 32 * t] = stage_word(a.res, wb, a.N, 0xFFu);
         }
 #pragma unroll
         for (int t = 0; t < kFewPos / 32; t++) {
@@ -737,13 +774,9 @@ __global__ void k_nibbles(const uint8_t* __restrict__ sb, uint64_t N, uint32_t a
 // Window records of the batch positions: record g holds the 32 letters at
 // g + cfil - 16 + t (t < 32), QSENT where that position lies outside g's
 // query (the filter's query-side lane bounds).
-// With `comb` (a combined code table) a single record of combined codes is
-// written to `win`: (group index << 4 | letter) where the letter counts, 0xFF
-// elsewhere; `winx` is then unused.
 __global__ void k_query_windows(const uint8_t* __restrict__ qsb, const uint8_t* __restrict__ qfull,
                                 const uint8_t* __restrict__ qrem, const uint8_t* __restrict__ qdst, uint64_t QN,
-                                int cfil, const CombTab* __restrict__ comb, uint8_t* __restrict__ win,
-                                uint8_t* __restrict__ winx) {
+                                int cfil, uint8_t* __restrict__ win, uint8_t* __restrict__ winx) {
     const uint64_t total = QN * 32;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t g = i >> 5;
@@ -755,14 +788,59 @@ __global__ void k_query_windows(const uint8_t* __restrict__ qsb, const uint8_t* 
             v = qsb[q];
             vx = qfull[q];
         }
-        if (comb) {
-            // letter from the seed byte, group index from the full code
-            win[i] = v == kQSent ? (uint8_t)0xFF
-                                 : (uint8_t)((vx < 24 ? (comb->t[vx] & 0xF0u) : 0xF0u) | (v & 0x0Fu));
-        } else {
-            win[i] = v;
-            winx[i] = vx;
+        win[i] = v;
+        winx[i] = vx;
+    }
+}
+
+// The eight plane words of 32 letters, one code byte (index << 4 | letter,
+// bit 7 set: does not count) per lane; lane p < 8 returns word p.
+__device__ __forceinline__ uint32_t plane_word(uint32_t code, bool counts, int lane) {
+    uint32_t mine = 0;
+#pragma unroll
+    for (int p = 0; p < 7; p++) {
+        const uint32_t w = __ballot_sync(0xffffffffu, (code >> p) & 1u);
+        if (lane == p) mine = w;
+    }
+    const uint32_t v = __ballot_sync(0xffffffffu, counts);
+    return lane == 7 ? v : mine;
+}
+
+// Plane records of the batch positions' windows, one warp per position; codes
+// >= 24 take index 7, which no residue has.
+__global__ void k_query_planes(const uint8_t* __restrict__ qsb, const uint8_t* __restrict__ qfull,
+                               const uint8_t* __restrict__ qrem, const uint8_t* __restrict__ qdst, uint64_t QN,
+                               int cfil, const CombTab* __restrict__ comb, uint32_t* __restrict__ win) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t g = w0; g < QN; g += nw) {
+        const int lo = 16 - cfil - (int)qdst[g], hi = (int)qrem[g] + 16 - cfil;
+        uint32_t code = 0;
+        bool counts = false;
+        if (lane >= lo && lane < hi) {
+            const uint64_t q = g + (uint64_t)(int64_t)(cfil - 16 + lane);
+            const uint32_t v = qsb[q], vx = qfull[q];
+            counts = v != kQSent;
+            code = (vx < 24 ? (comb->t[vx] & 0x70u) : 0x70u) | (v & 0x0Fu);
         }
+        const uint32_t word = plane_word(code, counts, lane);
+        if (lane < 8) win[8 * g + lane] = word;
+    }
+}
+
+// Bit planes of the database, block b + 1 holding positions 32 b .. 32 b + 31
+// (block 0 and those past the end: nothing counts).
+__global__ void k_db_planes(const uint8_t* __restrict__ res, uint64_t N, CombTab tab, uint64_t blocks,
+                            uint32_t* __restrict__ pl) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t b = w0; b < blocks; b += nw) {
+        const int64_t r = 32 * ((int64_t)b - 1) + lane;
+        const uint32_t c = r >= 0 && (uint64_t)r < N ? tab.t[res[r]] : 0xEEu;
+        const uint32_t word = plane_word(c, c != 0xEEu, lane);
+        if (lane < 8) pl[8 * b + lane] = word;
     }
 }
 
@@ -1328,30 +1406,23 @@ static uint64_t fingerprint(const saber_gpu* h, const saber_scan_params* p) {
     return f;
 }
 
-// Combined filter codes for alphabets of at most 14 letters whose groups
-// hold at most 15 codes: byte = (index of the code within its letter's group)
-// << 4 | letter, so that equal low nibbles are a reduced-letter identity and
-// equal bytes an exact one.  Subject residues without a letter are 0xEE;
-// query positions that never count are 0xFF; query codes >= 24 take group
-// index 15, which no residue has.  Returns false when the alphabet does not
-// fit (the filter then compares separate letter and residue records).
+// Plane codes (the window filter's bit planes) for alphabets of at most 16
+// letters whose groups hold at most 7 codes: byte = (index of the code within
+// its letter's group) << 4 | letter.  Residues without a letter are 0xEE and
+// never count; index 7 is no residue's.  Returns false when the alphabet does
+// not fit (the filter then compares letter and residue bytes).
 static bool comb_table(const saber_scan_params* p, uint8_t* tab /* 256 */) {
-    if (p->alpha_size > 14) return false;
+    if (p->alpha_size > 16) return false;
     int cnt[256] = {0};
     for (int c = 0; c < 256; c++) tab[c] = 0xEE;
     for (int c = 0; c < 24; c++) {
         const uint8_t L = p->alpha_map[c];
         if (L == 255) continue;
         if (L >= p->alpha_size) return false;
-        if (cnt[L] >= 15) return false;
+        if (cnt[L] >= 7) return false;
         tab[c] = (uint8_t)((cnt[L]++ << 4) | L);
     }
     return true;
-}
-
-__global__ void k_comb_bytes(const uint8_t* __restrict__ res, uint64_t N, CombTab tab, uint8_t* __restrict__ cb) {
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < N; r += (uint64_t)gridDim.x * blockDim.x)
-        cb[r] = tab.t[res[r]];
 }
 
 // ---- the small-batch scan's filter -------------------------------------------
@@ -1402,10 +1473,12 @@ int scan_build_db(saber_gpu* h, const saber_scan_params* p) {
         CombTab ct;
         h->sc_comb = comb_table(p, ct.t);
         if (h->sc_comb) {
-            CUALLOC(h, h->sc_cb, N + 128);
-            CU(h, cudaMemsetAsync(h->sc_cb.p, 0xEE, N + 128, s));
-            if (N) k_comb_bytes<<<nblocks(N, 256, h->sm_count * 32), 256, 0, s>>>(ds.res.as<uint8_t>(), N, ct,
-                                                                                 h->sc_cb.as<uint8_t>());
+            // a block in front, and those that the windows of the last
+            // positions and of the scan's idle lanes reach
+            const uint64_t blocks = N / 32 + 8;
+            CUALLOC(h, h->sc_pl, blocks * 32);
+            k_db_planes<<<nblocks(blocks * 32, 256, h->sm_count * 32), 256, 0, s>>>(ds.res.as<uint8_t>(), N, ct, blocks,
+                                                                                    h->sc_pl.as<uint32_t>());
             CU(h, cudaGetLastError());
         }
     }
@@ -1818,17 +1891,20 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     a.rng = h->sc_qrng.as<uint2>();
     a.qent = h->sc_qent.as<uint32_t>();
     CUALLOC(h, h->sc_qwin, QN * 32 + 32);
-    CUALLOC(h, h->sc_qwinx, QN * 32 + 32);
     CombTab ctab;
     const bool comb = h->sc_comb && comb_table(p, ctab.t);
     CUALLOC(h, h->sc_combtab, sizeof(CombTab));
     if (comb) CU(h, cudaMemcpyAsync(h->sc_combtab.p, &ctab, sizeof(CombTab), cudaMemcpyHostToDevice, s));
-    if (QN)
+    if (!comb) CUALLOC(h, h->sc_qwinx, QN * 32 + 32);
+    if (QN && comb)
+        k_query_planes<<<nblocks(QN * 32, 256), 256, 0, s>>>(
+            h->sc_qsb.as<uint8_t>(), h->sc_qfull.as<uint8_t>(), h->sc_qrem.as<uint8_t>(), h->sc_qdst.as<uint8_t>(),
+            QN, cfil, h->sc_combtab.as<CombTab>(), h->sc_qwin.as<uint32_t>());
+    else if (QN)
         k_query_windows<<<nblocks(QN * 32, 256), 256, 0, s>>>(
             h->sc_qsb.as<uint8_t>(), h->sc_qfull.as<uint8_t>(), h->sc_qrem.as<uint8_t>(), h->sc_qdst.as<uint8_t>(),
-            QN, cfil, comb ? h->sc_combtab.as<CombTab>() : nullptr, h->sc_qwin.as<uint8_t>(),
-            h->sc_qwinx.as<uint8_t>());
-    a.cb = comb ? h->sc_cb.as<uint8_t>() : nullptr;
+            QN, cfil, h->sc_qwin.as<uint8_t>(), h->sc_qwinx.as<uint8_t>());
+    a.pl = comb ? h->sc_pl.as<uint4>() : nullptr;
     a.qwin = h->sc_qwin.as<uint4>();
     a.qwinx = h->sc_qwinx.as<uint4>();
     a.cfil = cfil;
