@@ -160,7 +160,7 @@ struct saber_gpu {
         sc_qslot, sc_qent, sc_qpres, sc_surv, sc_key1, sc_key2, sc_val, sc_key1o, sc_key2o, sc_valo,
         sc_chains, sc_hsp, sc_hkey, sc_hkeyo, sc_hval, sc_hvalo, sc_pairs, sc_regions, sc_rthr, sc_ctr, sc_tmp,
         sc_rk64a, sc_rk64b, sc_rk64c, sc_rk32a, sc_rk32b, sc_ridxa, sc_ridxb, sc_regions2, sc_rstat, sc_rstat2,
-        sc_flags, sc_nib, sc_fil, sc_qwin, sc_qwinx, sc_surv2, sc_qrng, sc_pl, sc_combtab;
+        sc_flags, sc_nib, sc_fil, sc_qwin, sc_qwinx, sc_surv2, sc_qrng, sc_ewin, sc_pl, sc_combtab;
     bool sc_comb = false;  // the database's bit planes (sc_pl) are built
     uint64_t scan_table_bytes = 48ull << 20;  // tuning: seed-table bytes per scan pass (L2 budget)
     bool has_db_mask = false;

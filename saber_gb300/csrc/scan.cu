@@ -157,20 +157,25 @@ __host__ __device__ constexpr uint32_t fil_mul(int w) {
 //           shapes (grp.y), in shape order
 //   pass 1: entries per rank (rng.y), each seed keeping its arrival number;
 //           then one scan places the ranks' entries (rng.x)
-//   pass 2: scatter of the batch positions
+//   pass 2: scatter of the batch positions and, for a batch whose window
+//           records do not fit L2 (kEntryWindowBytes), of those records: a hit
+//           then reads its window beside those of the other entries of its
+//           code, not 32 bytes anywhere behind a read of the entry
 constexpr int kMaxShapes = 32;
 struct SeedArgs {
     uint32_t* fil;        // hash filter bits of all shapes, or null (ScanFilter)
     uint32_t fil_words;   // 32-bit words per shape
     int fil_shift;
     const uint8_t *qsb, *qrem;
-    uint64_t QN;
+    uint64_t i0, QN;      // first batch position and positions of the block
     uint32_t asize;
     const unsigned long long* freq;
     uint2* grp;
     uint2* rng;
-    uint32_t* slot;  // per shape and batch position
+    uint32_t* slot;  // per shape and position of the block
     uint32_t* ent;
+    const uint4* qwin;    // plane windows of the batch positions, and where the
+    uint4* ewin;          // entries' copies go (plane mode), or null
     unsigned long long* ctr;
     ShapeDev sh[kMaxShapes];
     uint64_t grp_off[kMaxShapes], freq_off[kMaxShapes];
@@ -183,7 +188,8 @@ __global__ void k_query_seeds(const __grid_constant__ SeedArgs a) {
     const unsigned long long* freq = a.freq + a.freq_off[si];
     uint2* grp = a.grp + a.grp_off[si];
     unsigned long long kept = 0, skipped = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.QN; i += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.QN; t += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = a.i0 + t;
         if (a.qrem[i] < sh.span) continue;
         const int64_t c = seed_code(a.qsb + i, sh, a.asize);
         if (c < 0) continue;
@@ -195,8 +201,8 @@ __global__ void k_query_seeds(const __grid_constant__ SeedArgs a) {
             atomicOr(&grp[c >> 5].x, 1u << (c & 31));
             if (a.fil) {
                 uint32_t hsum = 0;
-                for (uint32_t t = 0; t < sh.w; t++) {
-                    const uint32_t o = sh.off[t];
+                for (uint32_t k = 0; k < sh.w; k++) {
+                    const uint32_t o = sh.off[k];
                     hsum += ((uint32_t)a.qsb[i + o] << (4 * (o & 7))) * fil_mul(o >> 3);
                 }
                 hsum >>= a.fil_shift;
@@ -206,9 +212,17 @@ __global__ void k_query_seeds(const __grid_constant__ SeedArgs a) {
         } else {
             uint32_t k;
             code_rank(grp, (uint32_t)c, k);
-            uint32_t* slot = a.slot + (uint64_t)si * a.QN + i;
-            if (PASS == 1) *slot = atomicAdd(&a.rng[k].y, 1u);
-            else a.ent[a.rng[k].x + *slot] = (uint32_t)i;
+            uint32_t* slot = a.slot + (uint64_t)si * a.QN + t;
+            if (PASS == 1) {
+                *slot = atomicAdd(&a.rng[k].y, 1u);
+            } else {
+                const uint32_t e = a.rng[k].x + *slot;
+                a.ent[e] = (uint32_t)i;
+                if (a.ewin) {
+                    a.ewin[2 * (uint64_t)e] = a.qwin[2 * i];
+                    a.ewin[2 * (uint64_t)e + 1] = a.qwin[2 * i + 1];
+                }
+            }
         }
     }
     if (PASS == 0) {
@@ -263,6 +277,7 @@ struct ScanArgs {
     const uint2* grp;                // rank-compressed presence tables of all shapes
     const uint2* rng;                // rank -> (first entry, entries) of all shapes
     const uint32_t* qent;            // batch positions of all shapes
+    const uint4* ewin;               // per entry: its position's plane window (32 bytes), or null
     const uint4* qwin;               // per batch position: window record (32 bytes; planes or seed letters)
     const uint4* qwinx;              // per batch position: full-code window record (32 bytes; not in plane mode)
     const uint4* pl;                 // bit planes of the database, a block of 32 positions in front (plane mode)
@@ -449,7 +464,8 @@ __device__ __forceinline__ void scan_flush(const ScanArgs& a, int lane, int nseg
         bool pass = false;
         uint32_t g = 0;
         if (live) {
-            g = a.qent[ws.seg_eb[own] + k];
+            const uint64_t en = ws.seg_eb[own] + k;
+            if (!COMB || !a.ewin) g = a.qent[en];
             if (a.min_ids == 0) {
                 pass = true;
             } else if (COMB) {
@@ -457,7 +473,7 @@ __device__ __forceinline__ void scan_flush(const ScanArgs& a, int lane, int nseg
                 // exact >= min_ids) is ids + kx * exact >= min_ids since
                 // exact <= ids
                 uint32_t Q[8], S[8];
-                ld256(Q, a.qwin + 2 * (uint64_t)g);
+                ld256(Q, a.ewin ? a.ewin + 2 * en : a.qwin + 2 * (uint64_t)g);
                 if (RDS) {
                     subject_planes(a, ws.base + rl, srd, S);
                 } else {
@@ -475,6 +491,7 @@ __device__ __forceinline__ void scan_flush(const ScanArgs& a, int lane, int nseg
                 const uint32_t Er = Q[7] & S[7] & ~dr;
                 const uint32_t Ee = Er & ~((Q[4] ^ S[4]) | (Q[5] ^ S[5]) | (Q[6] ^ S[6]));
                 pass = __popc(Er) + a.kx * __popc(Ee) >= a.min_ids;
+                if (pass && a.ewin) g = a.qent[en];
             } else {
                 uint32_t Q[8], S[8];
                 ld256(Q, a.qwin + 2 * (uint64_t)g);
@@ -1425,6 +1442,24 @@ static bool comb_table(const saber_scan_params* p, uint8_t* tab /* 256 */) {
     return true;
 }
 
+// Window records of a batch above this size are copied to the seed entries (one
+// copy per shape).  Scan stage without / with the copies on one GB300: 105 MB
+// of records (11,000 queries x 150 M residues) 112.0 / 90.2 ms; 49 MB (5,000 x
+// 100 M) 35.5 / 34.7 and the tables 2.1 / 2.7; 14 MB (1,500 x 60 M) 10.5 / 10.8,
+// with the shorter seeds of the sensitive preset 12.9 / 15.2.
+constexpr uint64_t kEntryWindowBytes = 64ull << 20;
+
+// Positions per block of a batch's scan.  Blocks bound the tables' memory (48
+// bytes a position and shape; 16 GB in a block) and nothing else: every block
+// reads the database again, 18 ms for 150 M residues and 16 shapes, and
+// smaller blocks that would keep the windows in L2 lost more to that (11,000
+// queries in 1 / 2 / 3 / 6 blocks: 113 / 117 / 126 / 166 ms).
+static uint64_t scan_block_len(uint64_t QN, uint32_t nshapes) {
+    const uint64_t most = (16ull << 30) / 48 / nshapes;
+    const uint64_t blocks = std::max<uint64_t>(1, (QN + most - 1) / most);
+    return std::max<uint64_t>(1, (QN + blocks - 1) / blocks);
+}
+
 // ---- the small-batch scan's filter -------------------------------------------
 // Letters fit a nibble below 0xF and a window 32 letters.
 static bool few_shapes_fit(const saber_scan_params* p) {
@@ -1827,69 +1862,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     // a small batch's scan reads hash bitmaps of the seeds first
     uint32_t few_bits = 0;
     const uint32_t few = QN && N && few_shapes_fit(p) ? few_filter_bits(p, QN, few_bits) : 0;
-    const uint64_t ngroups = gbase[nsh], nranks = (uint64_t)nsh * QN;
-    CUALLOC(h, h->sc_qpres, ngroups * 8 + 8);
-    CUALLOC(h, h->sc_qslot, nranks * 4 + 4);
-    CUALLOC(h, h->sc_qent, nranks * 4 + 4);
-    CUALLOC(h, h->sc_qrng, nranks * 8 + 8);
-    CU(h, cudaMemsetAsync(h->sc_qpres.p, 0, ngroups * 8, s));
-    if (QN) {
-        CU(h, cudaMemsetAsync(h->sc_qrng.p, 0, nranks * 8, s));
-        SeedArgs sa;
-        sa.qsb = h->sc_qsb.as<uint8_t>();
-        sa.qrem = h->sc_qrem.as<uint8_t>();
-        sa.QN = QN;
-        sa.asize = p->alpha_size;
-        sa.freq = h->sc_freq.as<unsigned long long>();
-        sa.grp = h->sc_qpres.as<uint2>();
-        sa.rng = h->sc_qrng.as<uint2>();
-        sa.slot = h->sc_qslot.as<uint32_t>();
-        sa.ent = h->sc_qent.as<uint32_t>();
-        sa.ctr = ctr;
-        sa.fil = nullptr;
-        sa.fil_words = 0;
-        sa.fil_shift = 0;
-        if (few) {
-            const uint64_t bytes = ((uint64_t)nsh << few_bits) / 8;
-            CUALLOC(h, h->sc_fil, bytes);
-            CU(h, cudaMemsetAsync(h->sc_fil.p, 0, bytes, s));
-            sa.fil = h->sc_fil.as<uint32_t>();
-            sa.fil_words = (1u << few_bits) / 32;
-            sa.fil_shift = 32 - (int)few_bits;
-        }
-        for (uint32_t si = 0; si < nsh; si++) {
-            sa.sh[si] = shape_dev(p, si);
-            sa.grp_off[si] = gbase[si];
-            sa.freq_off[si] = h->sc_freq_off[si];
-        }
-        const PairWordIn<true> bits{h->sc_qpres.as<uint32_t>()};
-        const PairWordOut rank{h->sc_qpres.as<uint32_t>() + 1};
-        const PairWordIn<false> count{h->sc_qrng.as<uint32_t>() + 1};
-        const PairWordOut first{h->sc_qrng.as<uint32_t>()};
-        size_t t1 = 0, t2 = 0;
-        CU(h, cub::DeviceScan::ExclusiveSum(nullptr, t1, bits, rank, (int64_t)ngroups, s));
-        CU(h, cub::DeviceScan::ExclusiveSum(nullptr, t2, count, first, (int64_t)nranks, s));
-        CUALLOC(h, h->cub_tmp, std::max(t1, t2));
-        const dim3 grid(nblocks(QN, 256), nsh);
-        k_query_seeds<0><<<grid, 256, 0, s>>>(sa);
-        size_t tb = h->cub_tmp.cap;
-        CU(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, tb, bits, rank, (int64_t)ngroups, s));
-        k_query_seeds<1><<<grid, 256, 0, s>>>(sa);
-        tb = h->cub_tmp.cap;
-        CU(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, tb, count, first, (int64_t)nranks, s));
-        k_query_seeds<2><<<grid, 256, 0, s>>>(sa);
-        CU(h, cudaGetLastError());
-    }
-    CU(h, cudaEventRecord(ev[1], s));
-    ScanArgs a;
-    a.sb = h->sc_sb.as<uint8_t>();
-    a.res = ds.res.as<uint8_t>();
-    a.rem = h->sc_rem.as<uint8_t>();
-    a.dst = h->sc_dst.as<uint8_t>();
-    a.N = N;
-    a.grp = h->sc_qpres.as<uint2>();
-    a.rng = h->sc_qrng.as<uint2>();
-    a.qent = h->sc_qent.as<uint32_t>();
+    // window records of the batch positions
     CUALLOC(h, h->sc_qwin, QN * 32 + 32);
     CombTab ctab;
     const bool comb = h->sc_comb && comb_table(p, ctab.t);
@@ -1904,7 +1877,79 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
         k_query_windows<<<nblocks(QN * 32, 256), 256, 0, s>>>(
             h->sc_qsb.as<uint8_t>(), h->sc_qfull.as<uint8_t>(), h->sc_qrem.as<uint8_t>(), h->sc_qdst.as<uint8_t>(),
             QN, cfil, h->sc_qwin.as<uint8_t>(), h->sc_qwinx.as<uint8_t>());
+    const bool windows = comb && p->hit_filter_min_ids > 0 && QN * 32 > kEntryWindowBytes;  // copied to the entries
+    // a large batch goes in blocks of positions (scan_block_len), each with its
+    // own tables and its own passes over the database
+    const uint64_t block_len = scan_block_len(QN, nsh);
+    const uint64_t ngroups = gbase[nsh], nranks = (uint64_t)nsh * block_len;
+    CUALLOC(h, h->sc_qpres, ngroups * 8 + 8);
+    CUALLOC(h, h->sc_qslot, nranks * 4 + 4);
+    CUALLOC(h, h->sc_qent, nranks * 4 + 4);
+    CUALLOC(h, h->sc_qrng, nranks * 8 + 8);
+    if (windows) CUALLOC(h, h->sc_ewin, nranks * 32 + 32);
+    if (few) CUALLOC(h, h->sc_fil, ((uint64_t)nsh << few_bits) / 8);
+    SeedArgs sa;
+    sa.qsb = h->sc_qsb.as<uint8_t>();
+    sa.qrem = h->sc_qrem.as<uint8_t>();
+    sa.asize = p->alpha_size;
+    sa.freq = h->sc_freq.as<unsigned long long>();
+    sa.grp = h->sc_qpres.as<uint2>();
+    sa.rng = h->sc_qrng.as<uint2>();
+    sa.slot = h->sc_qslot.as<uint32_t>();
+    sa.ent = h->sc_qent.as<uint32_t>();
+    sa.qwin = h->sc_qwin.as<uint4>();
+    sa.ewin = windows ? h->sc_ewin.as<uint4>() : nullptr;
+    sa.ctr = ctr;
+    sa.fil = few ? h->sc_fil.as<uint32_t>() : nullptr;
+    sa.fil_words = few ? (1u << few_bits) / 32 : 0;
+    sa.fil_shift = few ? 32 - (int)few_bits : 0;
+    for (uint32_t si = 0; si < nsh; si++) {
+        sa.sh[si] = shape_dev(p, si);
+        sa.grp_off[si] = gbase[si];
+        sa.freq_off[si] = h->sc_freq_off[si];
+    }
+    auto build_tables = [&](uint64_t i0) -> int {
+        const uint64_t len = std::min<uint64_t>(block_len, QN - i0), n = (uint64_t)nsh * len;
+        CU(h, cudaMemsetAsync(h->sc_qpres.p, 0, ngroups * 8, s));
+        CU(h, cudaMemsetAsync(h->sc_qrng.p, 0, n * 8, s));
+        if (few) CU(h, cudaMemsetAsync(h->sc_fil.p, 0, ((uint64_t)nsh << few_bits) / 8, s));
+        sa.i0 = i0;
+        sa.QN = len;
+        const PairWordIn<true> bits{h->sc_qpres.as<uint32_t>()};
+        const PairWordOut rank{h->sc_qpres.as<uint32_t>() + 1};
+        const PairWordIn<false> count{h->sc_qrng.as<uint32_t>() + 1};
+        const PairWordOut first{h->sc_qrng.as<uint32_t>()};
+        size_t t1 = 0, t2 = 0;
+        CU(h, cub::DeviceScan::ExclusiveSum(nullptr, t1, bits, rank, (int64_t)ngroups, s));
+        CU(h, cub::DeviceScan::ExclusiveSum(nullptr, t2, count, first, (int64_t)n, s));
+        CUALLOC(h, h->cub_tmp, std::max(t1, t2));
+        const dim3 grid(nblocks(len, 256), nsh);
+        k_query_seeds<0><<<grid, 256, 0, s>>>(sa);
+        size_t tb = h->cub_tmp.cap;
+        CU(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, tb, bits, rank, (int64_t)ngroups, s));
+        k_query_seeds<1><<<grid, 256, 0, s>>>(sa);
+        tb = h->cub_tmp.cap;
+        CU(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, tb, count, first, (int64_t)n, s));
+        k_query_seeds<2><<<grid, 256, 0, s>>>(sa);
+        CU(h, cudaGetLastError());
+        return SABER_OK;
+    };
+    if (QN) {
+        const int rc = build_tables(0);
+        if (rc != SABER_OK) return rc;
+    }
+    CU(h, cudaEventRecord(ev[1], s));
+    ScanArgs a;
+    a.sb = h->sc_sb.as<uint8_t>();
+    a.res = ds.res.as<uint8_t>();
+    a.rem = h->sc_rem.as<uint8_t>();
+    a.dst = h->sc_dst.as<uint8_t>();
+    a.N = N;
+    a.grp = h->sc_qpres.as<uint2>();
+    a.rng = h->sc_qrng.as<uint2>();
+    a.qent = h->sc_qent.as<uint32_t>();
     a.pl = comb ? h->sc_pl.as<uint4>() : nullptr;
+    a.ewin = windows ? h->sc_ewin.as<uint4>() : nullptr;
     a.qwin = h->sc_qwin.as<uint4>();
     a.qwinx = h->sc_qwinx.as<uint4>();
     a.cfil = cfil;
@@ -1939,7 +1984,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     // 4 shapes 298 ms; 2,000 queries: 4 shapes 65.8 ms, 8 or more 68 ms)
     uint64_t shape_bytes = 0;
     for (uint32_t si = 0; si < nsh; si++)
-        shape_bytes = std::max(shape_bytes, (gbase[si + 1] - gbase[si]) * 8 + QN * 8 + QN * 4);
+        shape_bytes = std::max(shape_bytes, (gbase[si + 1] - gbase[si]) * 8 + block_len * 12);
     uint64_t per_pass = std::max<uint64_t>(1, h->scan_table_bytes / std::max<uint64_t>(shape_bytes, 1));
     if (few) per_pass = few;
     else if (per_pass >= (uint64_t)kShapeUnroll) per_pass -= per_pass % kShapeUnroll;
@@ -1962,14 +2007,22 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
         if (QN && N) {
             a.surv = h->sc_surv.as<uint2>();
             a.cap = scap;
-            for (const auto& ps : passes) {
-                a.s0 = ps.first;
-                a.s1 = ps.second;
-                if (few) scan_few<<<(unsigned)h->sm_count, kFewWarps * 32, few_smem, s>>>(a);
-                else if (comb) k_scan<true><<<scan_grid, kScanWarps * 32, 0, s>>>(a);
-                else k_scan<false><<<scan_grid, kScanWarps * 32, 0, s>>>(a);
+            // (the first block's tables stand, unless a rerun finds the last one's)
+            if (attempt && block_len < QN) CU(h, cudaMemsetAsync(ctr, 0, 2 * 8, s));
+            for (uint64_t i0 = 0; i0 < QN; i0 += block_len) {
+                if (i0 || (attempt && block_len < QN)) {
+                    const int rc = build_tables(i0);
+                    if (rc != SABER_OK) return rc;
+                }
+                for (const auto& ps : passes) {
+                    a.s0 = ps.first;
+                    a.s1 = ps.second;
+                    if (few) scan_few<<<(unsigned)h->sm_count, kFewWarps * 32, few_smem, s>>>(a);
+                    else if (comb) k_scan<true><<<scan_grid, kScanWarps * 32, 0, s>>>(a);
+                    else k_scan<false><<<scan_grid, kScanWarps * 32, 0, s>>>(a);
+                }
+                CU(h, cudaGetLastError());
             }
-            CU(h, cudaGetLastError());
         }
         unsigned long long hc[16];
         CU(h, cudaMemcpyAsync(hc, ctr, 16 * 8, cudaMemcpyDeviceToHost, s));

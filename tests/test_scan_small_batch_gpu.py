@@ -42,8 +42,8 @@ def _sets(seed, qn, n_db=40000):
     return ProteinSet(q, qoff), ProteinSet(db, soff), rng
 
 
-def _compare(dev, seed, qn, shapes, alpha, **kw):
-    qs, ss, rng = _sets(seed, qn)
+def _compare(dev, seed, qn, shapes, alpha, n_db=40000, **kw):
+    qs, ss, rng = _sets(seed, qn, n_db)
     amap, asz = alpha
     db_mask = (rng.random(ss.codes.size) < 0.03).astype(np.uint8)
     q_mask = (rng.random(qn) < 0.05).astype(np.uint8)
@@ -76,3 +76,9 @@ def test_alphabet_sizes(dev, letters):
     amap = [c % letters if c < 20 else 255 for c in range(24)]
     shapes = ["111011011", "1111110111"] if letters == 2 else ["11011", "1000111"]
     _compare(dev, letters, 700, shapes, (amap, letters), min_ids=22, exact_weight=1)
+
+
+@pytest.mark.parametrize("qn", [(64 << 20) // 32, (64 << 20) // 32 + 1])
+def test_batches_at_the_entry_window_edge(dev, qn):
+    """The plain scan with window records read by position (up to 64 MB of them) and copied to the entries (above)."""
+    _compare(dev, 11, qn, presets.DS16[:6], presets.alphabet_map(), n_db=3000, min_ids=27, exact_weight=2)
