@@ -32,10 +32,7 @@ void* pinned_scratch(saber_gpu* h, int slot, size_t bytes);
 
 namespace {
 
-constexpr double kRegionFloorEvalue = 10.0;     // engine.rs:518
-constexpr int64_t kBandScoreMinCells = 1 << 20;  // engine.rs:401
-constexpr int64_t kBandCostRatio = 12;           // engine.rs:402
-constexpr int64_t kBandBridge = 1024;            // engine.rs:404
+constexpr double kRegionFloorEvalue = 10.0;  // engine.rs:518
 constexpr int64_t kI32Max = 2147483647;
 constexpr int64_t kI64Max = std::numeric_limits<int64_t>::max();
 const double kLn2 = std::log(2.0);
@@ -359,107 +356,6 @@ struct Engine {
         }
     }
 
-    // engine.rs:1247-1324
-    std::vector<Plan> plan_windows(const std::vector<Region>& regs, int64_t qlen) const {
-        const size_t n = regs.size();
-        // per-thread work buffers (a query's regions are planned on one thread)
-        thread_local std::vector<int64_t> span_lo, span_hi;
-        thread_local std::vector<uint32_t> by, tmp;
-        thread_local std::vector<size_t> idx;
-        span_lo.resize(n);
-        span_hi.resize(n);
-        for (size_t i = 0; i < n; i++) {
-            span_lo[i] = regs[i].dmin;
-            span_hi[i] = regs[i].dmax;
-        }
-        // group by subject, stable (the index breaks ties): 12-bit counting
-        // passes over the subject ids, least significant digit first
-        by.resize(n);
-        tmp.resize(n);
-        uint32_t smax = 0;
-        for (size_t i = 0; i < n; i++) {
-            by[i] = (uint32_t)i;
-            smax = std::max(smax, regs[i].subject);
-        }
-        for (int sh = 0; sh == 0 || (sh < 32 && (smax >> sh) != 0); sh += 12) {
-            uint32_t cnt[4097] = {0};
-            for (size_t i = 0; i < n; i++) cnt[((regs[by[i]].subject >> sh) & 4095u) + 1]++;
-            for (int b = 0; b < 4096; b++) cnt[b + 1] += cnt[b];
-            for (size_t i = 0; i < n; i++) tmp[cnt[(regs[by[i]].subject >> sh) & 4095u]++] = by[i];
-            std::swap(by, tmp);
-        }
-        for (size_t a = 0; a < n;) {
-            size_t b = a;
-            while (b < n && regs[by[b]].subject == regs[by[a]].subject) b++;
-            int64_t top = std::numeric_limits<int64_t>::min();
-            for (size_t t = a; t < b; t++) top = std::max(top, regs[by[t]].best);
-            const int64_t strong = std::max<int64_t>(2 * (int64_t)P.hsp_threshold, top / 4);
-            idx.clear();
-            for (size_t t = a; t < b; t++)
-                if (regs[by[t]].best >= strong) idx.push_back(by[t]);
-            std::sort(idx.begin(), idx.end(), [&](size_t x, size_t y) {
-                if (regs[x].dmin != regs[y].dmin) return regs[x].dmin < regs[y].dmin;
-                if (regs[x].dmax != regs[y].dmax) return regs[x].dmax < regs[y].dmax;
-                return x < y;
-            });
-            size_t start = 0;
-            while (start < idx.size()) {
-                int64_t lo = regs[idx[start]].dmin, hi = regs[idx[start]].dmax;
-                size_t end = start + 1;
-                while (end < idx.size() && regs[idx[end]].dmin - hi <= kBandBridge) {
-                    hi = std::max(hi, regs[idx[end]].dmax);
-                    end++;
-                }
-                for (size_t t = start; t < end; t++) {
-                    span_lo[idx[t]] = lo;
-                    span_hi[idx[t]] = hi;
-                }
-                start = end;
-            }
-            a = b;
-        }
-        std::vector<Plan> plans(n);
-        for (size_t ri = 0; ri < n; ri++) {
-            const Region& r = regs[ri];
-            int64_t lo, hi;
-            window(r.dmin, r.dmax, r.sl, qlen, lo, hi);
-            Plan own{lo, hi, false, 0, 0};
-            if (P.exhaustive || r.best == 0 || (int64_t)P.window_slack >= kI64Max / 8) {
-                plans[ri] = own;
-                continue;
-            }
-            if (P.score_band > 0) {
-                const int64_t w = P.score_band, dmin = span_lo[ri], dmax = span_hi[ri], sl = r.sl;
-                const int64_t lo2 = std::min(std::max<int64_t>(dmin - w, 0), sl);
-                const int64_t hi2 = std::max(std::min(qlen + dmax + w, sl), lo2);
-                const int64_t nn = hi2 - lo2;
-                int64_t blo = dmin - w - lo2, bhi = dmax + w - lo2;
-                band_clip(blo, bhi, qlen, nn);
-                if (nn == 0 || band_covers(blo, bhi, qlen, nn)) plans[ri] = Plan{lo2, hi2, false, 0, 0};
-                else plans[ri] = Plan{lo2, hi2, true, blo, bhi};
-                continue;
-            }
-            if (qlen * (hi - lo) < kBandScoreMinCells) {
-                plans[ri] = own;
-                continue;
-            }
-            int64_t ulo, uhi;
-            window(span_lo[ri], span_hi[ri], r.sl, qlen, ulo, uhi);
-            const int64_t nn = uhi - ulo;
-            int64_t blo = span_lo[ri] - ulo - P.window_slack, bhi = span_hi[ri] - ulo + P.window_slack;
-            band_clip(blo, bhi, qlen, nn);
-            if (band_covers(blo, bhi, qlen, nn)) {
-                plans[ri] = own;
-                continue;
-            }
-            const int64_t rows = std::min(qlen, nn + band_width(blo, bhi));
-            const int64_t rect = qlen * nn;
-            if (band_width(blo, bhi) * rows * kBandCostRatio < rect) plans[ri] = Plan{ulo, uhi, true, blo, bhi};
-            else plans[ri] = own;
-        }
-        return plans;
-    }
-
     saber_band_job job(uint32_t qi, const Region& r, int64_t lo, int64_t hi, int64_t blo, int64_t bhi) const {
         saber_band_job j{};
         j.query = qi;
@@ -484,119 +380,70 @@ struct Engine {
         int rc = saber_gpu_score_band_jobs(h, jobs, n, sc, &ss);
         if (rc != SABER_OK) return rc;
         st.t_score_calls_ms += now_ms() - t0;
+        add_score_stats(ss);
+        return SABER_OK;
+    }
+
+    // The exhaustive mode: every subject's whole window (engine.rs:1223-1234,
+    // 1247-1260), one full-window job each.  (The scan's regions are planned and
+    // scored on the device, plan.cu.)
+    int score_exhaustive(const std::vector<std::vector<Region>>& per_q, const std::vector<int64_t>& qlens,
+                         std::vector<std::vector<Plan>>& plans, std::vector<std::vector<int64_t>>& scores) {
+        const size_t nq = per_q.size();
+        std::vector<size_t> base(nq + 1, 0);
+        for (size_t qi = 0; qi < nq; qi++) base[qi + 1] = base[qi] + per_q[qi].size();
+        const size_t n = base[nq];
+        scores.resize(nq);
+        saber_band_job* jobs = static_cast<saber_band_job*>(saber::pinned_scratch(h, 0, n * sizeof(saber_band_job)));
+        if (n && !jobs) return SABER_ERR_NOMEM;
+        parallel_for(nq, [&](size_t q) {
+            const int64_t m = qlens[q];
+            plans[q].resize(per_q[q].size());
+            for (size_t ri = 0; ri < per_q[q].size(); ri++) {
+                const Region& r = per_q[q][ri];
+                int64_t lo, hi;
+                window(r.dmin, r.dmax, r.sl, m, lo, hi);
+                plans[q][ri] = Plan{lo, hi, false, 0, 0};
+                jobs[base[q] + ri] = job((uint32_t)q, r, lo, hi, -m, hi - lo);
+            }
+        });
+        const int32_t* sc = nullptr;
+        int rc = score(jobs, n, 2, &sc);
+        if (rc != SABER_OK) return rc;
+        for (size_t q = 0; q < nq; q++) scores[q].assign(sc + base[q], sc + base[q + 1]);
+        return SABER_OK;
+    }
+
+    saber::PlanParams plan_params(const std::vector<Prep>& preps) const {
+        saber::PlanParams p{};
+        p.window_slack = P.window_slack;
+        p.score_band = P.score_band;
+        p.prefilter_band = P.score_prefilter_band;
+        p.hsp_threshold = P.hsp_threshold;
+        p.database_model = P.evalue_model == 1;
+        p.even = kp.even;
+        p.has_bits = has_bits;
+        p.prefilter_frac = P.score_prefilter_frac;
+        p.region_evalue = region_evalue();
+        p.evalue_cut = (P.evalue > 0.0 && std::isfinite(P.evalue)) ? P.evalue : kInf;
+        p.min_bitscore = has_bits ? P.min_bitscore : 0.0;
+        p.lambda = kp.lambda;
+        p.k = kp.k;
+        p.log_k = kp.log_k;
+        p.adl = kp.adl;
+        p.beta = kp.beta;
+        p.num_seqs = preps.empty() ? 1.0 : preps[0].qs.num_seqs;
+        return p;
+    }
+
+    void add_score_stats(const saber_score_stats& ss) {
+        if (!ss.jobs) return;
         st.t_score_device_ms += ss.t_prep_ms + ss.t_fast_ms + ss.t_generic_ms;
         st.t_score_prep_ms += ss.t_prep_ms;
         st.t_score_fast_ms += ss.t_fast_ms;
         st.t_score_generic_ms += ss.t_generic_ms;
         st.banded_cells += ss.banded_cells;
         st.score_launches += 1;
-        return SABER_OK;
-    }
-
-    // engine.rs:1021-1099, batched over the queries.  The jobs are built in
-    // the handle's pinned staging buffers (no zero-fill, fast copies), every
-    // per-region loop runs over the queries in parallel.
-    int score_windows(const std::vector<Prep>& preps, const std::vector<std::vector<Region>>& per_q,
-                      const std::vector<std::vector<Plan>>& plans, const std::vector<int64_t>& qlens,
-                      std::vector<std::vector<int64_t>>& scores) {
-        const int64_t wn = P.score_prefilter_band, full_band = P.score_band;
-        struct Ref {
-            uint32_t qi, ri;
-            int kind;  // 0 full, 1 narrow, 2 band
-        };
-        const size_t nq = per_q.size();
-        const double tb0 = now_ms();
-        scores.resize(nq);
-        std::vector<size_t> base(nq + 1, 0);
-        for (size_t qi = 0; qi < nq; qi++) base[qi + 1] = base[qi] + per_q[qi].size();
-        const size_t n1 = base[nq];
-        saber_band_job* s1 = static_cast<saber_band_job*>(saber::pinned_scratch(h, 0, n1 * sizeof(saber_band_job)));
-        if (n1 && !s1) return SABER_ERR_NOMEM;
-        std::unique_ptr<Ref[]> r1(new Ref[n1 ? n1 : 1]);
-        std::vector<uint64_t> banded(nq, 0);
-        parallel_for(nq, [&](size_t q) {
-            const uint32_t qi = (uint32_t)q;
-            scores[qi].assign(per_q[qi].size(), 0);
-            const int64_t m = qlens[qi];
-            for (uint32_t ri = 0; ri < per_q[qi].size(); ri++) {
-                const Region& r = per_q[qi][ri];
-                const Plan& pl = plans[qi][ri];
-                const int64_t n = pl.hi - pl.lo;
-                const size_t k = base[qi] + ri;
-                if (!pl.band) {
-                    s1[k] = job(qi, r, pl.lo, pl.hi, -m, n);
-                    r1[k] = {qi, ri, 0};
-                } else if (0 < wn && wn < full_band) {
-                    int64_t blo = r.dmin - wn - pl.lo, bhi = r.dmax + wn - pl.lo;
-                    band_clip(blo, bhi, m, n);
-                    s1[k] = job(qi, r, pl.lo, pl.hi, blo, bhi);
-                    r1[k] = {qi, ri, 1};
-                    banded[qi]++;
-                } else {
-                    s1[k] = job(qi, r, pl.lo, pl.hi, pl.blo, pl.bhi);
-                    r1[k] = {qi, ri, 2};
-                    banded[qi]++;
-                }
-            }
-        });
-        for (uint64_t v : banded) st.band_scored_regions += v;
-        st.t_score_build_ms += now_ms() - tb0;
-        const int32_t* sc1 = nullptr;
-        int rc = score(s1, n1, 2, &sc1);
-        if (rc != SABER_OK) return rc;
-        const double ts0 = now_ms();
-        // stage-2 decision per region (f64 threshold of the region's subject length)
-        const double re = region_evalue();
-        std::vector<uint8_t> again(n1, 0);
-        std::vector<size_t> n2q(nq + 1, 0);
-        parallel_for(nq, [&](size_t q) {
-            size_t c = 0;
-            LenMemo memo;  // the threshold depends on the query and the subject length only
-            for (size_t k = base[q]; k < base[q + 1]; k++) {
-                const Ref& x = r1[k];
-                if (x.kind != 1) {
-                    scores[x.qi][x.ri] = sc1[k];
-                    continue;
-                }
-                const Region& r = per_q[x.qi][x.ri];
-                const Prep& pr = preps[x.qi];
-                const int64_t sl = r.sl;
-                const double thr = memo.get(sl, [&]() {
-                    return P.score_prefilter_frac * pr.qs.floor_lower_bound(re, false, 0.0, sl, pr.region_floor);
-                });
-                if ((double)sc1[k] >= thr) {
-                    again[k] = 1;
-                    c++;
-                } else {
-                    scores[x.qi][x.ri] = sc1[k];
-                }
-            }
-            n2q[q + 1] = c;
-        });
-        for (size_t q = 0; q < nq; q++) n2q[q + 1] += n2q[q];
-        const size_t n2 = n2q[nq];
-        saber_band_job* s2 = static_cast<saber_band_job*>(saber::pinned_scratch(h, 1, n2 * sizeof(saber_band_job)));
-        if (n2 && !s2) return SABER_ERR_NOMEM;
-        std::unique_ptr<Ref[]> r2(new Ref[n2 ? n2 : 1]);
-        parallel_for(nq, [&](size_t q) {
-            size_t w = n2q[q];
-            for (size_t k = base[q]; k < base[q + 1]; k++) {
-                if (!again[k]) continue;
-                const Ref& x = r1[k];
-                const Region& r = per_q[x.qi][x.ri];
-                const Plan& pl = plans[x.qi][x.ri];
-                s2[w] = job(x.qi, r, pl.lo, pl.hi, pl.blo, pl.bhi);
-                r2[w] = x;
-                w++;
-            }
-        });
-        st.t_score_stage2_ms += now_ms() - ts0;
-        const int32_t* sc2 = nullptr;
-        rc = score(s2, n2, 3, &sc2);
-        if (rc != SABER_OK) return rc;
-        for (size_t k = 0; k < n2; k++) scores[r2[k].qi][r2[k].ri] = sc2[k];
-        st.band_rescored += n2;
-        return SABER_OK;
     }
 
     // engine.rs:1447-1530
@@ -894,8 +741,9 @@ extern "C" int saber_gpu_search(saber_gpu* h, const saber_search_params* params,
 
 namespace saber {
 int scheme_matrix(saber_gpu* h, int32_t* out576);  // saber_gpu.cu
-int scan_search_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask, const int32_t* region_thr,
-                        RegionSink& sink, saber_scan_stats* st);  // saber_gpu.cu
+int scan_plan_score(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask, const int32_t* region_thr,
+                    RegionSink& sink, saber_scan_stats* st, const PlanParams& pp, const int64_t* floors,
+                    const int64_t* region_floors, const PlanTie& tie, PlanResult& out, double* scan_ms);  // saber_gpu.cu
 void triage_set_labels(saber_gpu* h, const std::vector<uint64_t>& hit_regions);
 }
 
@@ -927,57 +775,59 @@ extern "C" int saber_gpu_search(saber_gpu* h, const saber_search_params* params,
     if (rc != SABER_OK) return rc;
     const double t1 = now_ms();
 
-    // candidate regions
+    // candidate regions, their plans and scores
     std::vector<std::vector<Region>> per_q(nq);
-    double t_scan_end = 0;
+    std::vector<std::vector<Plan>> plans(nq);
+    std::vector<std::vector<int64_t>> scores(nq);
+    double t2 = t1;
     bool collecting = false;
     if (P.exhaustive) {
-        for (uint32_t qi = 0; qi < nq; qi++)
+        for (uint32_t qi = 0; qi < nq; qi++) {
             if (qlens[qi] > 0)
                 for (uint32_t s = 0; s < nsub; s++)
                     per_q[qi].push_back({s, -qlens[qi], E.slen(s), 0, 0, db_offsets[s], E.slen(s)});
+            E.st.regions += per_q[qi].size();
+        }
+        t2 = now_ms();
+        rc = E.score_exhaustive(per_q, qlens, plans, scores);
+        if (rc != SABER_OK) return rc;
     } else if (nq && nsub) {
         std::vector<int32_t> thr(nq);
-        for (uint32_t qi = 0; qi < nq; qi++) thr[qi] = (int32_t)preps[qi].region_thr;
-        // candidate regions, capped per query and triaged (a no-op without a
-        // model or collection) on the device; the kept ones arrive grouped by
-        // query in region order, each with its position in the capped list
+        std::vector<int64_t> floors(nq), rfloors(nq);
+        for (uint32_t qi = 0; qi < nq; qi++) {
+            thr[qi] = (int32_t)preps[qi].region_thr;
+            floors[qi] = preps[qi].floor;
+            rfloors[qi] = preps[qi].region_floor;
+        }
         saber::RegionSink sink;
         sink.lambda = (float)P.lambda;
         sink.logk = (float)std::log(P.k);
-        rc = saber::scan_search_regions(h, &P.scan, q_mask, thr.data(), sink, &E.st.scan);
+        const double re = E.region_evalue();
+        const saber::PlanTie tie = [&](uint32_t q, int64_t sl, int32_t score) {
+            return (double)score >= P.score_prefilter_frac *
+                                        preps[q].qs.floor_lower_bound(re, false, 0.0, sl, preps[q].region_floor);
+        };
+        saber::PlanResult kept;
+        double scan_ms = 0;
+        rc = saber::scan_plan_score(h, &P.scan, q_mask, thr.data(), sink, &E.st.scan, E.plan_params(preps),
+                                    floors.data(), rfloors.data(), tie, kept, &scan_ms);
         if (rc != SABER_OK) return rc;
-        t_scan_end = now_ms();
+        t2 = t1 + scan_ms;
         collecting = sink.collecting;
         if (sink.triaged) E.st.triage_dropped += sink.ncap - sink.n;
-        const saber_region* R = sink.regs;
-        const uint32_t* src = sink.src;
-        const uint64_t* sbase = sink.sbase;
-        const uint32_t* slen = sink.slen;
-        const uint64_t nr = sink.n;
-        parallel_for(nq, [&](size_t qi) {
-            auto by_query = [](const saber_region& r, uint64_t q) { return r.query < q; };
-            const uint64_t b = (uint64_t)(std::lower_bound(R, R + nr, (uint64_t)qi, by_query) - R);
-            const uint64_t e = (uint64_t)(std::lower_bound(R + b, R + nr, (uint64_t)qi + 1, by_query) - R);
-            auto& v = per_q[qi];
-            v.reserve(e - b);
-            for (uint64_t t = b; t < e; t++)
-                v.push_back({R[t].subject, R[t].d_min, R[t].d_max, R[t].best, src[t], sbase[t], (int64_t)slen[t]});
-        });
+        E.st.regions += sink.n;
+        E.st.band_scored_regions += kept.banded;
+        E.st.band_rescored += kept.n2;
+        E.add_score_stats(kept.stage1);
+        E.add_score_stats(kept.stage2);
+        E.st.t_score_calls_ms += now_ms() - t2;
+        for (uint64_t t = 0; t < kept.n; t++) {
+            const saber::KeptRegion& r = kept.kept[t];
+            per_q[r.query].push_back({r.subject, r.d_min, r.d_max, r.best, r.src, r.sbase, (int64_t)r.slen});
+            plans[r.query].push_back({r.lo, r.hi, r.band != 0, r.blo, r.bhi});
+            scores[r.query].push_back(r.score);
+        }
     }
-    for (uint32_t qi = 0; qi < nq; qi++) {
-        if (qlens[qi] == 0) per_q[qi].clear();
-        E.st.regions += per_q[qi].size();
-    }
-    const double t2 = now_ms();
-    if (t_scan_end == 0) t_scan_end = t2;
-
-    std::vector<std::vector<Plan>> plans(nq);
-    parallel_for(nq, [&](size_t qi) { plans[qi] = E.plan_windows(per_q[qi], qlens[qi]); });
-    const double t3 = now_ms();
-    std::vector<std::vector<int64_t>> scores;
-    rc = E.score_windows(preps, per_q, plans, qlens, scores);
-    if (rc != SABER_OK) return rc;
     const double t4 = now_ms();
     std::vector<std::vector<HitRec>> result;
     std::vector<uint64_t> hit_src;
@@ -995,10 +845,8 @@ extern "C" int saber_gpu_search(saber_gpu* h, const saber_search_params* params,
     *n_hits = nh;
     *n_ops = no;
     E.st.t_prep_ms = t1 - t0;
-    E.st.t_scan_ms = t_scan_end - t1;
-    E.st.t_triage_ms = t2 - t_scan_end;
-    E.st.t_plan_ms = t3 - t2;
-    E.st.t_score_ms = t4 - t3;
+    E.st.t_scan_ms = t2 - t1;
+    E.st.t_score_ms = t4 - t2;
     E.st.t_finish_ms = t5 - t4;
     E.st.t_total_ms = t5 - t0;
     if (stats) *stats = E.st;

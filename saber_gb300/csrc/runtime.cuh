@@ -176,9 +176,12 @@ struct saber_gpu {
     uint64_t sc_key = 0;            // fingerprint of the database state built
     std::vector<uint64_t> sc_caps;  // per shape
     std::vector<uint64_t> sc_freq_off;
-    // device-side region cap / triage / compaction, pinned host staging
-    saber::DevBuf rg_qcnt, rg_qstart, rg_rank, rg_flag, rg_idx, rg_idx2, rg_out, rg_sbase, rg_slen;
-    saber::HostBuf pin_reg, pin_src, pin_sbase, pin_slen;
+    // device-side region cap / triage / compaction
+    saber::DevBuf rg_qcnt, rg_qstart, rg_rank, rg_flag, rg_idx, rg_idx2, rg_out;
+    // window plans and scoring of the regions (plan.cu)
+    saber::DevBuf pl_key, pl_keyo, pl_idx, pl_by, pl_flag, pl_list, pl_span, pl_plan, pl_score, pl_floor, pl_ctr, pl_tmp,
+        pl_kept;
+    saber::HostBuf pin_kept;
     saber::HostBuf pin_scratch[4];  // the batch engine's staging (pinned_scratch)
     saber::DevBuf mask_runs;  // database mask runs being expanded
     // six-frame translation scratch
@@ -222,6 +225,13 @@ static int fail(saber_gpu* h, int code, const char* fmt, ...) {
 int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask, const int32_t* region_thr,
                  saber_region* out, uint64_t out_cap, uint64_t* n_out, saber_scan_stats* st,
                  RegionSink* sink = nullptr);
+
+// Scoring of jobs that stand in the handle's jobs_dev (scores in scores_dev):
+// room for n of them, and the scoring itself.
+int reserve_resident_jobs(saber_gpu* h, uint64_t njobs);
+int score_resident_jobs(saber_gpu* h, uint64_t njobs, saber_score_stats* st);
+int plan_and_score(saber_gpu* h, const RegionSink& sk, const PlanParams& P, const int64_t* floors,
+                   const int64_t* region_floors, const PlanTie& tie, PlanResult& out);
 
 static inline unsigned nblocks(uint64_t n, unsigned t, unsigned cap = 65535u * 16u) {
     uint64_t b = (n + t - 1) / t;

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -730,6 +731,34 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     return SABER_OK;
 }
 
+int reserve_resident_jobs(saber_gpu* h, uint64_t njobs) {
+    const uint64_t n = h->use_graphs ? pow2_at_least(njobs, 1 << 12) : njobs;
+    CUALLOC(h, h->jobs_dev, n * sizeof(saber_band_job));
+    CUALLOC(h, h->scores_dev, n * 4);
+    return SABER_OK;
+}
+
+int score_resident_jobs(saber_gpu* h, uint64_t njobs, saber_score_stats* st) {
+    if (!h->use_graphs)
+        return score_pipeline(h, h->scheme, h->main, h->jobs_dev.as<saber_band_job>(), njobs,
+                              h->scores_dev.as<int32_t>(), st);
+    // the widest clipped band sizes the graph's scratch and the cell total sets
+    // the automatic long-job threshold: one reduction on the device, 16 bytes
+    // read back
+    const QuerySet& qs = h->main.qs;
+    CUALLOC(h, h->g_wmax, 16);
+    CU(h, cudaMemsetAsync(h->g_wmax.p, 0, 16, h->stream));
+    if (qs.has)
+        k_job_wmax<<<nblocks(njobs, 256, h->sm_count * 8), 256, 0, h->stream>>>(
+            h->jobs_dev.as<saber_band_job>(), njobs, qs.offsets.as<uint64_t>(), qs.nq,
+            h->g_wmax.as<unsigned long long>());
+    CU(h, cudaGetLastError());
+    unsigned long long r[2] = {0, 0};
+    CU(h, cudaMemcpyAsync(r, h->g_wmax.p, 16, cudaMemcpyDeviceToHost, h->stream));
+    CU(h, cudaStreamSynchronize(h->stream));
+    return score_pipeline_graph(h, h->scheme, h->main, njobs, r[0], r[1], st);
+}
+
 static int build_profiles(saber_gpu* h, const Scheme& sch, QuerySet& q) {
     q.p8 = false;
     if (!q.has || !sch.has || q.nq == 0) return SABER_OK;
@@ -1390,13 +1419,19 @@ void* pinned_scratch(saber_gpu* h, int slot, size_t bytes) {
     return h->pin_scratch[slot].reserve(std::max<size_t>(bytes, 64)) == cudaSuccess ? h->pin_scratch[slot].p : nullptr;
 }
 
-// The batch's candidate regions for the host engine (engine.cpp): capped per
-// query and triaged on the device, kept ones in pinned memory (sink).
-int scan_search_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask, const int32_t* region_thr,
-                        RegionSink& sink, saber_scan_stats* st) {
+// The batch's candidate regions for the host engine (engine.cpp): scanned,
+// capped per query, triaged, planned and scored on the device; those that may
+// be reported come back in pinned memory.  *scan_ms: the scan's share.
+int scan_plan_score(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask, const int32_t* region_thr,
+                    RegionSink& sink, saber_scan_stats* st, const PlanParams& pp, const int64_t* floors,
+                    const int64_t* region_floors, const PlanTie& tie, PlanResult& out, double* scan_ms) {
     ENTER(h);
     uint64_t n = 0;
-    return scan_regions(h, p, q_mask, region_thr, nullptr, 0, &n, st, &sink);
+    const auto t0 = std::chrono::steady_clock::now();
+    int rc = scan_regions(h, p, q_mask, region_thr, nullptr, 0, &n, st, &sink);
+    *scan_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (rc != SABER_OK) return rc;
+    return plan_and_score(h, sink, pp, floors, region_floors, tie, out);
 }
 
 int triage_grads(saber_gpu* h, const float* model, const float* X, const uint8_t* y, uint32_t n, float pos_weight,
@@ -1495,35 +1530,10 @@ int saber_gpu_score_band_jobs(saber_gpu* h, const saber_band_job* jobs, uint64_t
         if (stats) *stats = saber_score_stats{};
         return SABER_OK;
     }
-    int rc;
-    if (h->use_graphs) {
-        // the widest clipped band sizes the graph's scratch and the cell total
-        // sets the automatic long-job threshold: one reduction on the device
-        // after the copy, 16 bytes read back
-        const QuerySet& qs = h->main.qs;
-        const uint64_t npad = pow2_at_least(njobs, 1 << 12);
-        CUALLOC(h, h->jobs_dev, npad * sizeof(saber_band_job));
-        CUALLOC(h, h->scores_dev, npad * 4);
-        CUALLOC(h, h->g_wmax, 16);
-        CU(h, cudaMemcpyAsync(h->jobs_dev.p, jobs, njobs * sizeof(saber_band_job), cudaMemcpyHostToDevice, h->stream));
-        CU(h, cudaMemsetAsync(h->g_wmax.p, 0, 16, h->stream));
-        if (qs.has)
-            k_job_wmax<<<nblocks(njobs, 256, h->sm_count * 8), 256, 0, h->stream>>>(
-                h->jobs_dev.as<saber_band_job>(), njobs, qs.offsets.as<uint64_t>(), qs.nq,
-                h->g_wmax.as<unsigned long long>());
-        CU(h, cudaGetLastError());
-        unsigned long long r[2] = {0, 0};
-        CU(h, cudaMemcpyAsync(r, h->g_wmax.p, 16, cudaMemcpyDeviceToHost, h->stream));
-        CU(h, cudaStreamSynchronize(h->stream));
-        rc = score_pipeline_graph(h, h->scheme, h->main, njobs, r[0], r[1], stats);
-    } else {
-        CUALLOC(h, h->jobs_dev, njobs * sizeof(saber_band_job));
-        CUALLOC(h, h->scores_dev, njobs * 4);
-        CU(h, cudaMemcpyAsync(h->jobs_dev.p, jobs, njobs * sizeof(saber_band_job), cudaMemcpyHostToDevice,
-                              h->stream));
-        rc = score_pipeline(h, h->scheme, h->main, h->jobs_dev.as<saber_band_job>(), njobs,
-                            h->scores_dev.as<int32_t>(), stats);
-    }
+    int rc = reserve_resident_jobs(h, njobs);
+    if (rc != SABER_OK) return rc;
+    CU(h, cudaMemcpyAsync(h->jobs_dev.p, jobs, njobs * sizeof(saber_band_job), cudaMemcpyHostToDevice, h->stream));
+    rc = score_resident_jobs(h, njobs, stats);
     if (rc != SABER_OK) return rc;
     CU(h, cudaMemcpyAsync(scores, h->scores_dev.p, njobs * 4, cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
