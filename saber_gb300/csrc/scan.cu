@@ -113,14 +113,19 @@ __global__ void k_freq_bits(const uint32_t* __restrict__ counts, uint64_t ncodes
 }
 
 // ---- query tables ------------------------------------------------------------
+constexpr int kXPad = 16;  // entries in front of and behind a batch's code words (k_chains)
+
 __global__ void k_query_bytes(const uint8_t* __restrict__ qcodes, const uint8_t* __restrict__ qmask, uint64_t QN,
-                              AlphaMap am, uint8_t* __restrict__ qsb, uint8_t* __restrict__ qfull) {
+                              AlphaMap am, uint8_t* __restrict__ qsb, uint8_t* __restrict__ qfull,
+                              const int8_t* __restrict__ qbias, uint16_t* __restrict__ qcb) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < QN; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint8_t c = qcodes[i];
         const uint8_t r = am.m[c < 24 ? c : 23];
         const bool ok = !(qmask && qmask[i]) && r != 255;
         qsb[i] = ok ? r : kQSent;
         qfull[i] = ok ? c : kQSent;
+        // code as the scores read it | bias << 8, for the extensions
+        qcb[kXPad + i] = (uint16_t)((c < 24 ? c : 22u) | ((uint32_t)(uint8_t)(qbias ? qbias[i] : 0) << 8));
     }
 }
 
@@ -869,7 +874,8 @@ __global__ void k_region_keys(const saber_region* __restrict__ regs, uint32_t n,
                               uint32_t* __restrict__ idx) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const saber_region r = regs[i];
-        k_lo[i] = ((unsigned long long)((uint32_t)r.d_min ^ 0x80000000u) << 32) | ((uint32_t)r.d_max ^ 0x80000000u);
+        // diagonals lie in (-2^19, 2^19)
+        k_lo[i] = ((unsigned long long)(uint32_t)(r.d_min + kDBias) << 20) | (uint32_t)(r.d_max + kDBias);
         k_sub[i] = r.subject;
         k_hi[i] = ((unsigned long long)r.query << 32) | (0xFFFFFFFFu - ((uint32_t)r.best ^ 0x80000000u));
         idx[i] = i;
@@ -974,6 +980,7 @@ struct ChainArgs {
     const uint64_t *soffs, *qoffs;
     const uint8_t* res;               // canonical residues
     uint64_t n_res;                   // residues (the buffer holds 64 more)
+    const uint32_t* qcb;              // query batch codes and biases, two positions a word (kXPad in front)
     const uint8_t* qcodes;            // query batch codes (16 bytes of padding)
     const int8_t* qbias;              // per batch position score bias, or null
     uint64_t qn;                      // batch positions
@@ -986,6 +993,8 @@ struct ChainArgs {
     uint64_t hcap;
     unsigned long long* ctr;          // [4] extensions, [5] avoided, [6] steps
     uint32_t* next;                   // chain work counter (zero at launch)
+    uint32_t zero;                    // 0, as an argument: with an immediate 0 the packed maximum of nvcc 13.0
+                                      // returns wrong predicates
 };
 
 // Chains, one per lane (one subject, query and diagonal; hits in (query
@@ -1004,7 +1013,8 @@ struct ChainArgs {
 // chains' lengths, and lanes that finish a chain take the next one from a
 // shared counter (chains are in query-major order, so a warp's lanes mostly
 // read one query's profile).
-constexpr int kXBlock = 8;
+
+constexpr int kXBlock = 8;  // positions per block of an extension
 
 // 8 consecutive bytes of buf from byte index x on (bytes outside [0, limit)
 // read as 0): two words, from three aligned loads when all are in range.
@@ -1087,10 +1097,149 @@ __device__ __forceinline__ void xdrop_eval(XDir& d, const XBlock& L, bool right,
     }
 }
 
+// The packed block of k_chains<true>: 8 positions of both directions at once,
+// rightwards in the low halves and leftwards in the high ones.  The sums are
+// kept relative to the best so far, so that they fit int16 whatever the
+// score; a direction that drops is held far below, and the positions past a
+// direction's end score kXSent.  The steps at which a half improved or dropped
+// are bits of a mask, read after the block.
+// One GB300, the whole visit stage (keys, sort, chains), int32 blocks -> these:
+// 11,000 queries x 60 M residues 45.3 -> 39.8 ms, 400 x 150 M bases 14.0 -> 12.0.
+constexpr int kXMaxDrop = 8000;     // largest x-drop of the packed block
+constexpr int kXSent = -12000;      // below any x-drop, above int16's end after a drop
+constexpr int kXDead = -16384;
+constexpr int kXRow = 52;           // bytes per row of the int16 score table (25 rows, 26 columns)
+
+// The 8 positions of a block in one direction, ascending: query codes and
+// biases two to a word, subject codes four to a word.
+struct XWords {
+    uint32_t q[4];
+    uint2 s;
+};
+
+// Positions from query index gq and residue gs on (gq >= -8, gs >= -8: what
+// lies before the first sequence is masked by x_limit).  All offsets fit 32
+// bits: batches are below 2^27 positions, databases below 2^32 residues.
+__device__ __forceinline__ void x_load(XWords& w, const ChainArgs& a, int gq, int64_t gs) {
+    const uint32_t qi = (uint32_t)(gq + kXPad);
+    const uint32_t* qp = a.qcb + (qi >> 1);
+    const uint32_t qs = (qi & 1u) * 16u;
+    uint32_t v = __ldg(qp);
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        const uint32_t nx = __ldg(qp + p + 1);
+        w.q[p] = __funnelshift_r(v, nx, qs);
+        v = nx;
+    }
+    const int wi = (int)(gs >> 2);
+    const uint32_t* sp = reinterpret_cast<const uint32_t*>(a.res);
+    const uint32_t ss = (uint32_t)(gs & 3) * 8u;
+    const uint32_t w0 = __ldg(sp + (uint32_t)max(wi, 0)), w1 = __ldg(sp + (uint32_t)max(wi + 1, 0)),
+                   w2 = __ldg(sp + (uint32_t)(wi + 2));
+    w.s = make_uint2(__funnelshift_r(w0, w1, ss), __funnelshift_r(w1, w2, ss));
+}
+
+// Positions past a direction's end score the sentinel row 24: entries lim ..
+// rightwards, entries .. 7 - lim leftwards (its position u is entry 7 - u).
+__device__ __forceinline__ void x_limit(XWords& w, int lim, bool right) {
+    if (lim >= kXBlock) return;
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        const int m = right ? lim - 2 * p : lim - 6 + 2 * p;  // valid entries of the word
+        if (m <= 0) w.q[p] = 0x00180018u;
+        else if (m == 1) w.q[p] = right ? (w.q[p] & 0xFFFFu) | 0x00180000u : (w.q[p] & 0xFFFF0000u) | 0x18u;
+    }
+}
+
+// Table offsets of the entries 2 p, 2 p + 1, packed.
+__device__ __forceinline__ uint32_t x_offs(const XWords& w, int p) {
+    const uint32_t sel = p & 1 ? 0x4342u : 0x4140u;
+    const uint32_t s2 = __byte_perm(p < 2 ? w.s.x : w.s.y, 0u, sel);
+    return (w.q[p] & 0x00FF00FFu) * (uint32_t)kXRow + 2u * s2;
+}
+
+struct XPair {
+    uint32_t cur;      // both directions' running sums, relative to their bests
+    int best_r, best_l;
+};
+
+// Evaluates a block; the directions' state as xdrop_eval leaves it.
+__device__ __forceinline__ void xdrop_pair(XDir& R, XDir& L, XPair& P, XWords& BR, XWords& BL, bool has_bias,
+                                           const uint8_t* tab, uint32_t negx2, uint32_t zero2) {
+    const int lim_r = R.run ? R.n - R.t : 0, lim_l = L.run ? L.n - L.t : 0;
+    x_limit(BR, lim_r, true);
+    x_limit(BL, lim_l, false);
+    uint32_t cur = P.cur, best = zero2, up_r = 0, up_l = 0, dn_r = 0, dn_l = 0;
+    const uint32_t dead = (uint32_t)(uint16_t)(int16_t)kXDead * 0x10001u;
+#pragma unroll
+    for (int u = 0; u < kXBlock; u += 2) {
+        const uint32_t ir = x_offs(BR, u / 2);      // positions u, u + 1
+        const uint32_t il = x_offs(BL, 3 - u / 2);  // positions u + 1, u
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+            const uint32_t a = *reinterpret_cast<const uint16_t*>(tab + (v ? ir >> 16 : ir & 0xFFFFu));
+            const uint32_t b = *reinterpret_cast<const uint16_t*>(tab + (v ? il & 0xFFFFu : il >> 16));
+            uint32_t sub = __byte_perm(a, b, 0x5410);
+            if (has_bias) {
+                // bytes 1 and 3 of a word are its entries' biases
+                const uint32_t kr = v ? 3u : 1u, kl = v ? 5u : 7u;
+                uint32_t bias;
+                asm("prmt.b32 %0, %1, %2, %3;"
+                    : "=r"(bias)
+                    : "r"(BR.q[u / 2]), "r"(BL.q[3 - u / 2]),
+                      "r"(kr | ((8u | kr) << 4) | (kl << 8) | ((8u | kl) << 12)));
+                sub = __vadd2(sub, bias);
+            }
+            bool ph, pl;
+            cur = __vadd2(cur, sub);
+            best = __vibmax_s16x2(best, cur, &ph, &pl);
+            if (!pl) up_r |= 1u << (u + v);
+            if (!ph) up_l |= 1u << (u + v);
+            (void)__vibmax_s16x2(cur, __vadd2(best, negx2), &ph, &pl);
+            if (!pl) {
+                dn_r |= 1u << (u + v);
+                cur = __byte_perm(cur, dead, 0x3254);
+            }
+            if (!ph) {
+                dn_l |= 1u << (u + v);
+                cur = __byte_perm(cur, dead, 0x7610);
+            }
+        }
+    }
+    auto finish = [&](XDir& d, int& total, uint32_t up, uint32_t dn, int lim, int b16) {
+        if (!d.run) return;
+        total += b16;
+        if (up) d.xe = d.t + 32 - __clz(up);
+        const int f = dn ? __ffs(dn) - 1 : kXBlock;
+        d.t += kXBlock;
+        if (f < lim && f < kXBlock) {
+            d.run = false;
+            d.done = d.t - kXBlock + f + 1;
+        } else if (lim <= kXBlock) {
+            d.run = false;
+            d.done = d.n;
+        }
+    };
+    finish(R, P.best_r, up_r, dn_r, lim_r, (int)(int16_t)(best & 0xFFFFu));
+    finish(L, P.best_l, up_l, dn_l, lim_l, (int)(int16_t)(best >> 16));
+    P.cur = __vsub2(cur, best);
+}
+
+// PACKED: x-drops of 0 .. kXMaxDrop (xdrop_pair); else int32 blocks.
+template <bool PACKED>
 __global__ void __launch_bounds__(256, SABER_CHAINS_MIN_BLOCKS) k_chains(ChainArgs a) {
-    __shared__ int32_t smat[576];
-    for (int t = threadIdx.x; t < 576; t += blockDim.x) smat[t] = a.matrix[t];
+    __shared__ int32_t smat[PACKED ? 1 : 576];
+    __shared__ __align__(4) int16_t xtab[PACKED ? 25 * kXRow / 2 : 2];
+    if (PACKED) {
+        for (int t = threadIdx.x; t < 25 * (kXRow / 2); t += blockDim.x) {
+            const int r = t / (kXRow / 2), c = t - r * (kXRow / 2);
+            xtab[t] = r < 24 && c < 24 ? (int16_t)a.matrix[r * 24 + c] : (int16_t)kXSent;
+        }
+    } else {
+        for (int t = threadIdx.x; t < 576; t += blockDim.x) smat[t] = a.matrix[t];
+    }
     __syncthreads();
+    const uint32_t negx2 = (uint32_t)(uint16_t)(int16_t)(-a.x) * 0x10001u;
     const int lane = threadIdx.x & 31;
     const uint32_t nch = *a.nchains;
     unsigned long long ext = 0, avoided = 0, steps = 0;
@@ -1105,6 +1254,7 @@ __global__ void __launch_bounds__(256, SABER_CHAINS_MIN_BLOCKS) k_chains(ChainAr
     const uint8_t* subj = nullptr;
     int qp = 0, sp = 0;
     XDir R{0, 0, 0, 0, 0, 0, false}, Lf{0, 0, 0, 0, 0, 0, false};
+    XPair X{0u, 0, 0};
     uint2 vnext = make_uint2(0, 0);
     bool have_next = false;  // vnext holds survivor i + 1 of this lane's chain
     const uint32_t m27 = (1u << 27) - 1u;
@@ -1152,16 +1302,26 @@ __global__ void __launch_bounds__(256, SABER_CHAINS_MIN_BLOCKS) k_chains(ChainAr
                 R = XDir{0, qlen - qp < sl - sp ? qlen - qp : sl - sp, 0, 0, 0, 0, true};
                 Lf = XDir{0, qp < sp ? qp : sp, 0, 0, 0, 0, false};
                 Lf.run = Lf.n > 0;
+                X = XPair{0u, 0, 0};
                 extending = true;
             }
             // both directions advance a block per iteration: their loads are
             // issued together, then both are evaluated
             const int64_t gq0 = (int64_t)q0 + qp, gs0 = (int64_t)(subj - a.res) + sp;
-            XBlock BR, BL;
-            if (R.run) xdrop_load(BR, R, true, gq0, gs0, a);
-            if (Lf.run) xdrop_load(BL, Lf, false, gq0, gs0, a);
-            if (R.run) xdrop_eval(R, BR, true, smat, a.x);
-            if (Lf.run) xdrop_eval(Lf, BL, false, smat, a.x);
+            if (PACKED) {
+                XWords BR{}, BL{};
+                if (R.run) x_load(BR, a, (int)gq0 + R.t, gs0 + R.t);
+                if (Lf.run) x_load(BL, a, (int)gq0 - Lf.t - kXBlock, gs0 - Lf.t - kXBlock);
+                xdrop_pair(R, Lf, X, BR, BL, a.qbias != nullptr, reinterpret_cast<const uint8_t*>(xtab), negx2, a.zero);
+                R.best = X.best_r;
+                Lf.best = X.best_l;
+            } else {
+                XBlock BR, BL;
+                if (R.run) xdrop_load(BR, R, true, gq0, gs0, a);
+                if (Lf.run) xdrop_load(BL, Lf, false, gq0, gs0, a);
+                if (R.run) xdrop_eval(R, BR, true, smat, a.x);
+                if (Lf.run) xdrop_eval(Lf, BL, false, smat, a.x);
+            }
             if (!R.run && !Lf.run) {
                 steps += (uint64_t)(R.done + Lf.done);
                 ext++;
@@ -1798,6 +1958,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     // query bytes and distances
     CUALLOC(h, h->sc_qsb, QN + 128);
     CUALLOC(h, h->sc_qfull, QN + 64);
+    CUALLOC(h, h->sc_qcb, (QN + 2 * kXPad + 16) * 2);
     CUALLOC(h, h->sc_qrem, QN + 64);
     CUALLOC(h, h->sc_qdst, QN + 64);
     CUALLOC(h, h->sc_tmp, QN + 64);
@@ -1805,7 +1966,9 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     CU(h, cudaMemsetAsync(h->sc_qsb.p, kQSent, QN + 128, s));
     if (QN) {
         k_query_bytes<<<nblocks(QN, 256), 256, 0, s>>>(qs.codes.as<uint8_t>(), q_mask ? h->sc_tmp.as<uint8_t>() : nullptr,
-                                                       QN, am, h->sc_qsb.as<uint8_t>(), h->sc_qfull.as<uint8_t>());
+                                                       QN, am, h->sc_qsb.as<uint8_t>(), h->sc_qfull.as<uint8_t>(),
+                                                       qs.has_bias ? qs.bias.as<int8_t>() : nullptr,
+                                                       h->sc_qcb.as<uint16_t>());
         k_dists<<<nblocks(QN, 256), 256, 0, s>>>(qs.offsets.as<uint64_t>(), qs.nq, QN, h->sc_qrem.as<uint8_t>(),
                                                  h->sc_qdst.as<uint8_t>());
         CU(h, cudaGetLastError());
@@ -2108,6 +2271,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
         c.res = ds.res.as<uint8_t>();
         c.n_res = ds.n_res;
         c.qcodes = qs.codes.as<uint8_t>();
+        c.qcb = h->sc_qcb.as<uint32_t>();
         c.qbias = qs.has_bias ? qs.bias.as<int8_t>() : nullptr;
         c.qn = qs.offs[qs.nq];
         c.matrix = h->scheme.d_matrix.as<int32_t>();
@@ -2116,8 +2280,10 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
         c.nhsp = ctr + 11;
         c.ctr = ctr;
         c.next = reinterpret_cast<uint32_t*>(ctr + 14);
+        c.zero = 0;
         int chain_bps = 0;
-        CU(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&chain_bps, k_chains, 256, 0));
+        auto chains = p->x_drop >= 0 && p->x_drop <= kXMaxDrop ? k_chains<true> : k_chains<false>;
+        CU(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&chain_bps, chains, 256, 0));
         unsigned long long nh = 0;
         for (int attempt = 0;; attempt++) {
             CUALLOC(h, h->sc_hsp, hcap * 16);
@@ -2133,7 +2299,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
             CU(h, cudaMemsetAsync(ctr + 4, 0, 3 * 8, s));
             CU(h, cudaMemsetAsync(ctr + 11, 0, 8, s));
             CU(h, cudaMemsetAsync(c.next, 0, 4, s));
-            k_chains<<<(unsigned)std::max(1, chain_bps) * (unsigned)h->sm_count, 256, 0, s>>>(c);
+            chains<<<(unsigned)std::max(1, chain_bps) * (unsigned)h->sm_count, 256, 0, s>>>(c);
             CU(h, cudaGetLastError());
             CU(h, cudaMemcpyAsync(&nh, ctr + 11, 8, cudaMemcpyDeviceToHost, s));
             CU(h, cudaStreamSynchronize(s));
@@ -2145,15 +2311,17 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
         CU(h, cudaEventRecord(ev[3], s));
         const uint32_t nhsp = (uint32_t)nh;
         if (nhsp) {
+            // (query, diagonal) below the subject, which leads
+            const int hsp_bits = 40 + bits_for(ds.nsub ? ds.nsub - 1 : 0);
             size_t t4 = 0;
             CU(h, cub::DeviceRadixSort::SortPairs(nullptr, t4, h->sc_hkey.as<unsigned long long>(),
                                                   h->sc_hkeyo.as<unsigned long long>(), h->sc_hval.as<uint32_t>(),
-                                                  h->sc_hvalo.as<uint32_t>(), (int)nhsp, 0, 64, s));
+                                                  h->sc_hvalo.as<uint32_t>(), (int)nhsp, 0, hsp_bits, s));
             CUALLOC(h, h->cub_tmp, t4);
             tb = h->cub_tmp.cap;
             CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, tb, h->sc_hkey.as<unsigned long long>(),
                                                   h->sc_hkeyo.as<unsigned long long>(), h->sc_hval.as<uint32_t>(),
-                                                  h->sc_hvalo.as<uint32_t>(), (int)nhsp, 0, 64, s));
+                                                  h->sc_hvalo.as<uint32_t>(), (int)nhsp, 0, hsp_bits, s));
             CUALLOC(h, h->sc_pairs, (uint64_t)nhsp * 4 + 8);
             k_run_flags<<<nblocks(nhsp, 256), 256, 0, s>>>(h->sc_hkeyo.as<unsigned long long>(), nhsp, 20,
                                                            h->sc_flags.as<uint8_t>());
@@ -2214,13 +2382,15 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
                 CUALLOC(h, h->cub_tmp, std::max(r1, r2));
                 size_t rb = h->cub_tmp.cap;
                 // pass 1: (d_min, d_max); ib = order
-                CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, rb, klo, k64o, ia, ib, (int)nrg, 0, 64, s));
+                CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, rb, klo, k64o, ia, ib, (int)nrg, 0, 40, s));
                 // pass 2: subject, stable
                 k_gather_u32_by<<<nblocks(nrg, 256), 256, 0, s>>>(ksub, ib, nrg, k32o);
-                CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, rb, k32o, ksub, ib, ia, (int)nrg, 0, 32, s));
+                CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, rb, k32o, ksub, ib, ia, (int)nrg, 0,
+                                                      bits_for(ds.nsub ? ds.nsub - 1 : 0), s));
                 // pass 3: (query, best desc), stable
                 k_gather_u64_by<<<nblocks(nrg, 256), 256, 0, s>>>(khi, ia, nrg, k64o);
-                CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, rb, k64o, klo, ia, ib, (int)nrg, 0, 64, s));
+                CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, rb, k64o, klo, ia, ib, (int)nrg, 0,
+                                                      32 + bits_for(qs.nq ? qs.nq - 1 : 0), s));
                 k_gather_regions<<<nblocks(nrg, 256), 256, 0, s>>>(h->sc_regions.as<saber_region>(), ib, nrg,
                                                                    h->sc_regions2.as<saber_region>());
                 if (sink) {
