@@ -42,14 +42,16 @@ namespace saber {
 constexpr unsigned kWaveThreads = 128;
 
 // Jobs [task * 32 / L, ...) of one (L, J) class of the sorted list, one per
-// group of L lanes.
+// group of L lanes.  L = 128: one job on the block's four warps, whose edge
+// lanes pass E and F through shared memory (xch), a barrier per step.
 template <int L, int J>
 __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __restrict__ list, uint32_t njobs,
-                                          uint32_t task, int lane, const uint8_t* tab) {
-    constexpr int G = 32 / L;
-    const int gl = lane % L;
-    const uint32_t pos = task * G + (uint32_t)(lane / L);
-    const bool has = pos < njobs && lane < G * L;
+                                          uint32_t task, int lane, const uint8_t* tab, uint32_t* xch) {
+    constexpr bool kBlock = L > 32;
+    constexpr int G = kBlock ? 1 : 32 / L;
+    const int gl = kBlock ? (int)threadIdx.x : lane % L, wib = (int)threadIdx.x >> 5;
+    const uint32_t pos = kBlock ? task : task * G + (uint32_t)(lane / L);
+    const bool has = pos < njobs && (kBlock || lane < G * L);
     uint32_t jid = 0;
     int m = 0, n = 0, lo = 0, w = 0, s0 = 0, nit = 0;
     const uint32_t* qrow = a.qrow;
@@ -99,11 +101,16 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
     i0 += kWaveAhead;
     c0 += 2 * J + kWaveAhead;
     uint32_t best = 0;
+    if (kBlock) {
+        if (lane == 31) xch[wib] = neg2;
+        __syncthreads();
+    }
     for (int it = 0; it < nmax; it += kWaveAhead) {
 #pragma unroll
         for (int t = 0; t < kWaveAhead; t++) {
             // even step: E, F come in from the odd band indices
             uint32_t left = __shfl_up_sync(0xffffffffu, E[J - 1], 1);
+            if (kBlock && lane == 0 && wib > 0) left = xch[wib - 1];
             if (gl == 0) left = neg2;
 #pragma unroll
             for (int j = 0; j < J; j++) {
@@ -119,8 +126,13 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
                 F[j] = __viaddmax_s16x2(Fin, nge2, Gv);
                 best = __vmaxs2(best, H);
             }
+            if (kBlock) {
+                if (lane == 0) xch[4 + wib] = F[0];
+                __syncthreads();
+            }
             // odd step: from the even ones
             uint32_t down = __shfl_down_sync(0xffffffffu, F[0], 1);
+            if (kBlock && lane == 31 && gl != L - 1) down = xch[5 + wib];
             if (gl == L - 1) down = neg2;
 #pragma unroll
             for (int j = 0; j < J; j++) {
@@ -133,6 +145,10 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
                 E[j] = __viaddmax_s16x2(Ein, nge2, Gv);
                 F[j] = __viaddmax_s16x2(Fin, nge2, Gv);
                 best = __vmaxs2(best, H);
+            }
+            if (kBlock) {
+                if (lane == 31) xch[wib] = E[J - 1];
+                __syncthreads();
             }
             // the windows advance by one row and one column
 #pragma unroll
@@ -158,6 +174,13 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
         const int v = __shfl_down_sync(0xffffffffu, sc, o);
         if (o < L && gl + o < L) sc = max(sc, v);
     }
+    if (kBlock) {
+        __syncthreads();  // (xch may still be read)
+        if (lane == 0) xch[wib] = (uint32_t)sc;
+        __syncthreads();
+        sc = (int)max(max(xch[0], xch[1]), max(xch[2], xch[3]));
+        __syncthreads();
+    }
     if (has && gl == 0) {
         if (sc >= kLimit16) a.rescue[atomicAdd(a.rescue_count, 1u)] = jid;
         else a.scores[jid] = sc;
@@ -168,6 +191,7 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
 // a class the list is largest first.
 __global__ void __launch_bounds__(kWaveThreads, 4) k_band_wave(WaveArgs a) {
     __shared__ __align__(4) int16_t tab[25 * kWaveRow / 2];
+    __shared__ uint32_t xch[8];
     wv_table(tab, a.matrix, a.go);
     __syncthreads();
     const uint8_t* tb = reinterpret_cast<const uint8_t*>(tab);
@@ -181,6 +205,18 @@ __global__ void __launch_bounds__(kWaveThreads, 4) k_band_wave(WaveArgs a) {
         total += tasks[c];
     }
     const uint32_t* list = a.order + (a.skip0 ? *a.skip0 : 0u) + (a.skip1 ? *a.skip1 : 0u);
+    // Few wide bands: one on a whole block (8 or 4 band indices a lane) instead
+    // of 32 or 16 a lane on one warp.  The longest job is then the launch: 40
+    // full windows of a 310-residue query 383 -> 257 us a call.  Many of them
+    // keep every warp busy by themselves, and a lane's sets share its overheads.
+    if (n[0] + n[1] <= 2 * gridDim.x) {
+        for (uint32_t p = blockIdx.x; p < n[0] + n[1]; p += gridDim.x) {
+            if (p < n[0]) wave_task<128, 2>(a, list, n[0], p, lane, tb, xch);
+            else wave_task<128, 1>(a, list + n[0], n[1], p - n[0], lane, tb, xch);
+        }
+        total -= tasks[0] + tasks[1];
+        tasks[0] = tasks[1] = 0;
+    }
     for (;;) {
         uint32_t t = 0;
         if (lane == 0) t = atomicAdd(a.task_counter, 1u);
@@ -188,42 +224,42 @@ __global__ void __launch_bounds__(kWaveThreads, 4) k_band_wave(WaveArgs a) {
         if (t >= total) break;
         const uint32_t* l = list;
         if (t < tasks[0]) {
-            wave_task<32, 8>(a, l, n[0], t, lane, tb);
+            wave_task<32, 8>(a, l, n[0], t, lane, tb, xch);
             continue;
         }
         t -= tasks[0];
         l += n[0];
         if (t < tasks[1]) {
-            wave_task<32, 4>(a, l, n[1], t, lane, tb);
+            wave_task<32, 4>(a, l, n[1], t, lane, tb, xch);
             continue;
         }
         t -= tasks[1];
         l += n[1];
         if (t < tasks[2]) {
-            wave_task<32, 2>(a, l, n[2], t, lane, tb);
+            wave_task<32, 2>(a, l, n[2], t, lane, tb, xch);
             continue;
         }
         t -= tasks[2];
         l += n[2];
         if (t < tasks[3]) {
-            wave_task<32, 1>(a, l, n[3], t, lane, tb);
+            wave_task<32, 1>(a, l, n[3], t, lane, tb, xch);
             continue;
         }
         t -= tasks[3];
         l += n[3];
         if (t < tasks[4]) {
-            wave_task<16, 1>(a, l, n[4], t, lane, tb);
+            wave_task<16, 1>(a, l, n[4], t, lane, tb, xch);
             continue;
         }
         t -= tasks[4];
         l += n[4];
         if (t < tasks[5]) {
-            wave_task<9, 1>(a, l, n[5], t, lane, tb);
+            wave_task<9, 1>(a, l, n[5], t, lane, tb, xch);
             continue;
         }
         t -= tasks[5];
         l += n[5];
-        wave_task<8, 1>(a, l, n[6], t, lane, tb);
+        wave_task<8, 1>(a, l, n[6], t, lane, tb, xch);
     }
 }
 

@@ -66,6 +66,35 @@ def test_class_edges_match_oracle(data, gaps, biased, graphs):
     assert st["banded_cells"] == cells
 
 
+@pytest.mark.parametrize("jobs_n", [1210, 1230])
+def test_wide_bands_on_blocks_and_on_warps(data, jobs_n):
+    """Wide bands below and above the count at which they go to single warps (two per block of the launch)."""
+    torch = pytest.importorskip("torch")
+    qs, ss = data
+    per_sm = 2 * 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    widths = [257, 400, 511, 512, 513, 700, 1023, 1024]
+    jobs = _jobs(np.random.default_rng(jobs_n), qs, ss, widths, (jobs_n * per_sm // 1216) // len(widths) + 1)
+    # bands that stay this wide when clipped to the query and the window
+    qlen = (qs.offsets[1:] - qs.offsets[:-1]).astype(np.int64)
+    long_q = int(np.argmax(qlen))
+    long_s = int(np.argmax((ss.offsets[1:] - ss.offsets[:-1]).astype(np.int64)))
+    for t in range(jobs.size):
+        w = widths[t % len(widths)]
+        jobs[t]["query"], jobs[t]["subject"] = long_q, long_s
+        jobs[t]["win_begin"] = int(ss.offsets[long_s]) + t % 7
+        jobs[t]["win_len"] = int(ss.offsets[long_s + 1] - ss.offsets[long_s]) - 7 - t % 11
+        jobs[t]["band_lo"] = -(w // 2) + t % 50
+        jobs[t]["band_hi"] = int(jobs[t]["band_lo"]) + w - 1
+    with Device(0) as dev:
+        dev.set_scheme(B62, 11, 1)
+        dev.load_db(ss.codes, ss.offsets)
+        dev.load_queries(qs.codes, qs.offsets, None)
+        dev.long_steps = 0
+        got, st = dev.score_band_jobs(jobs)
+    want, cells = orc.score_band_jobs(ss.codes, qs.codes, qs.offsets, None, jobs, B62, 11, 1, threads=4)
+    assert np.array_equal(got, want) and st["banded_cells"] == cells
+
+
 @pytest.mark.parametrize("width", [9, 36, 90, 200, 400, 1000])
 def test_scores_at_the_int16_limit(width):
     """Self-alignments whose scores lie on both sides of the limit at which a
