@@ -165,7 +165,7 @@ struct saber_gpu {
     uint64_t scan_table_bytes = 48ull << 20;  // tuning: seed-table bytes per scan pass (L2 budget)
     bool has_db_mask = false;
     // learned triage: installed model, per-call feature buffers, collection
-    saber::DevBuf tr_model, tr_wb, tr_sfeat, tr_qfeat, tr_reg, tr_rstat, tr_rq, tr_rrank, tr_qinfo, tr_X, tr_logit;
+    saber::DevBuf tr_model, tr_wb, tr_sfeat, tr_qfeat, tr_reg, tr_rstat, tr_rq, tr_rrank, tr_qinfo, tr_X, tr_logit, tr_err;
     saber::TriageScratch tg;
     bool tr_on = false, tr_sfeat_ok = false;
     uint64_t tr_sfeat_key = 0;

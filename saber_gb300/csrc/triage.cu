@@ -513,40 +513,6 @@ __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float
     }
 }
 
-// ---- fused inference on the tensor cores -------------------------------------
-// One warp per 16 regions, mma.sync m16n8k16 (bf16 operands, fp32
-// accumulation).  The weights are bf16 already; the activations (the
-// normalised inputs and the layer-1 outputs) are fp32 and enter as a
-// bf16 pair hi + lo (lo = the rounding residual), two products per tile, so
-// the result matches the fp32-activation forward pass of training to about
-// 2^-16 relative.  Layer 1 runs in chunks of 16 hidden units whose
-// accumulator tiles are, register for register, the A operand of layer 2;
-// layer 3 (256 -> 1) is a quad reduction of the layer-2 accumulators.
-constexpr size_t kPackOff = ((kModelFloats * 2 + 255) / 256) * 256;        // bytes into the bf16 buffer
-constexpr size_t kPackBytes = (size_t)(2 + 16) * 32 * 32 * sizeof(uint2);  // W1 and W2 fragments
-
-// B fragments of a row-major [K][256] bf16 weight, K = 16 kt: for tile (kt,
-// nt) and lane l, {W[k][n], W[k + 1][n]} and {W[k + 8][n], W[k + 9][n]} with
-// k = 16 kt + 2 (l % 4), n = 8 nt + l / 4.
-__global__ void k_pack_b(const __nv_bfloat16* __restrict__ W, int kt_n, uint2* __restrict__ out) {
-    const int total = kt_n * 32 * 32;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        const int lane = t & 31, nt = (t >> 5) & 31, kt = t >> 10;
-        const int k = kt * 16 + 2 * (lane & 3), n = nt * 8 + (lane >> 2);
-        auto u = [&](int kk) { return (uint32_t)__bfloat16_as_ushort(W[(size_t)kk * kTHid + n]); };
-        out[t] = make_uint2(u(k) | (u(k + 1) << 16), u(k + 8) | (u(k + 9) << 16));
-    }
-}
-
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint2 b) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-        "{%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y));
-}
-
 // (x, y) -> packed bf16 pairs hi and lo with x ~ hi.x + lo.x, y ~ hi.y + lo.y
 __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
@@ -555,95 +521,254 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
-__global__ void __launch_bounds__(128) k_mlp_infer(const float* __restrict__ X, uint64_t n,
-                                                   const float* __restrict__ model, const uint2* __restrict__ pk,
-                                                   const __nv_bfloat16* __restrict__ wb, float* __restrict__ logit) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t r0 = warp * 16;
-    if (r0 >= n) return;
-    const int qr = lane >> 2, qc = 2 * (lane & 3);
-    const uint64_t ra = r0 + qr, rb = r0 + qr + 8;
-    // layer-1 A operand: normalised inputs, 2 k-steps of 16, hi and lo
-    uint32_t xa[2][4], xl[2][4];
+// ---- fused inference on tcgen05 -------------------------------------------------
+// The weights are bf16 already; the activations (the normalised inputs and the
+// layer-1 outputs) are fp32 and enter as a bf16 pair hi + lo (lo = the rounding
+// residual), two products per tile with fp32 accumulation, so the result
+// matches the fp32-activation forward pass of training to about 2^-16 relative.
+// One persistent block per SM, tiles of 128 rows, the weights resident in
+// shared memory, both layers' accumulators (128 x 256 fp32 each) in the SM's
+// 512 TMEM columns.
+//   layer 1: A = [hi | lo] (128 x 64), B = [W1; W1]: four MMAs of K = 16
+//   layer 2: the hidden units in four chunks of 64; a chunk's accumulators are
+//            read back, biased, clamped and split into hi and lo operand tiles
+//            (two buffers, so that the next chunk is converted while eight
+//            MMAs of this one run)
+//   layer 3: each thread dots half a row of layer 2 with W3
+// Operand tiles are K-major with the 128-byte swizzle: row r, 16-byte piece j
+// at 128 r + 16 (j ^ (r & 7)), 64 values of K a row.
+//
+// One GB300, a call from host rows (an mma.sync m16n8k16 kernel, 16 rows a warp
+// with the weight fragments read from L1 -> this one): 200 rows 113 -> 69 us,
+// 20,000 153 -> 109, 1 M 1633 -> 1154 us, of which the rows' copy to the device
+// is about 750.
+//
+// Every wait on an mbarrier is bounded: when one runs out the block sets *err,
+// stops waiting, still finishes its loop and frees its TMEM, and the host
+// reports the error.
+constexpr int kMtRows = 128, kMtThreads = 256;
+constexpr uint32_t kMtTile = 128 * 128;          // bytes of a 128 x 64 bf16 operand tile
+constexpr uint32_t kMtW2 = 0;                    // four 256 x 64 tiles of W2^T
+constexpr uint32_t kMtW1 = kMtW2 + 4 * 2 * kMtTile;
+constexpr uint32_t kMtA = kMtW1 + 2 * kMtTile;   // two buffers of (hi, lo); the layer-1 operand uses the second
+constexpr size_t kMtSmem = kMtA + 4 * kMtTile + 1024;  // + room to align the base to 1024 bytes
+constexpr uint32_t kMtIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
+
+__device__ __forceinline__ uint32_t mt_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Shared-memory descriptor of a K-major tile, 128-byte swizzle, groups of eight
+// rows 1024 bytes apart.
+__device__ __forceinline__ uint64_t mt_desc(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+__device__ __forceinline__ void mt_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        :
+        : "r"(d), "l"(a), "l"(b), "r"(kMtIdesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void mt_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" : : "r"(bar) : "memory");
+}
+
+// Waits for the phase of parity `phase`; false when it does not come.
+__device__ __forceinline__ bool mt_wait(uint32_t bar, uint32_t phase) {
+    for (int i = 0; i < (1 << 15); i++) {  // (a try lasts two microseconds at most)
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(phase), "r"(2000u)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// 32 columns of this thread's TMEM lane.
+__device__ __forceinline__ void mt_ld32(uint32_t (&v)[32], uint32_t addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(addr)
+        : "memory");
+}
+__device__ __forceinline__ void mt_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void mt_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+__global__ void __launch_bounds__(kMtThreads, 1) k_mlp_tc(const float* __restrict__ X, uint64_t n,
+                                                          const float* __restrict__ model,
+                                                          const __nv_bfloat16* __restrict__ wb,
+                                                          float* __restrict__ logit, uint32_t* __restrict__ err) {
+    extern __shared__ uint8_t raw[];
+    __shared__ __align__(8) uint64_t bars[3];  // chunk buffers 0 and 1, layer 1
+    __shared__ uint32_t tmem_at;
+    __shared__ float norm[2 * kTIn], half_dot[kMtRows];
+    uint8_t* base = raw + ((1024u - (mt_smem(raw) & 1023u)) & 1023u);
+    const uint32_t sb = mt_smem(base);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const unsigned short* w = reinterpret_cast<const unsigned short*>(wb);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" : : "r"(mt_smem(&tmem_at)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 32)
+        for (int i = 0; i < 3; i++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" : : "r"(mt_smem(&bars[i])) : "memory");
+    if (tid < 2 * kTIn) norm[tid] = model[kOffMu + tid];  // mu, then isd
+    // weights, transposed to rows of the output unit: W2 in four tiles of 64
+    // inputs, W1 twice in one
+    for (int t = tid; t < 40 * kTHid; t += kMtThreads) {
+        const int o = t & (kTHid - 1), p = t >> 8;  // output unit, piece of eight inputs
+        const bool l2 = p < 32;
+        const unsigned short* src = w + (l2 ? kOffW2 + (size_t)p * 8 * kTHid : kOffW1 + (size_t)(p & 3) * 8 * kTHid) + o;
+        uint32_t v[4];
 #pragma unroll
-    for (int ks = 0; ks < 2; ks++) {
+        for (int i = 0; i < 4; i++) v[i] = (uint32_t)src[2 * i * kTHid] | ((uint32_t)src[(2 * i + 1) * kTHid] << 16);
+        const int j = p & 7;
+        uint8_t* dst = base + (l2 ? kMtW2 + (uint32_t)(p >> 3) * 2 * kMtTile : kMtW1) + 128 * o + 16 * (j ^ (o & 7));
+        *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mt_before_sync();
+    __syncthreads();
+    mt_after_sync();
+    const uint32_t tmem = tmem_at;
+    const uint32_t d1 = tmem, d2 = tmem + 256;
+    const uint32_t lanes = (uint32_t)(warp & 3) * 32u << 16;  // this warp's TMEM lanes
+    const int row = (warp & 3) * 32 + lane, hf = warp >> 2;   // its row of the tile, its half of the columns
+    const uint32_t bar0 = mt_smem(&bars[0]), bar1 = mt_smem(&bars[1]), barL = mt_smem(&bars[2]);
+    uint32_t ph0 = 0, ph1 = 0, phL = 0;
+    bool dead = false;
+    const uint64_t tiles = (n + kMtRows - 1) / kMtRows;
+    for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        // layer-1 operand: two threads per row, 16 features each
+        {
+            const int r = tid >> 1, h = tid & 1;
+            const uint64_t gr = tile * kMtRows + r;
+            uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int hf = 0; hf < 2; hf++) {  // k and k + 8
-            const int k = ks * 16 + hf * 8 + qc;
-            float v[2][2];
+            for (int q = 0; q < 4; q++) {
+                const float4 x = gr < n ? __ldg(reinterpret_cast<const float4*>(X + gr * kTIn + 16 * h) + q)
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+                const int k = 16 * h + 4 * q;
+                float v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-            for (int rr = 0; rr < 2; rr++) {
-                const uint64_t r = rr ? rb : ra;
+                for (int e = 0; e < 4; e++) v[e] = gr < n && k + e < kTFeat ? (v[e] - norm[k + e]) * norm[kTIn + k + e] : 0.f;
+                split2(v[0], v[1], hi[2 * q], lo[2 * q]);
+                split2(v[2], v[3], hi[2 * q + 1], lo[2 * q + 1]);
+            }
+            uint8_t* a1 = base + kMtA + 2 * kMtTile + 128 * r;
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int kk = k + e;
-                    v[rr][e] = (r < n && kk < kTFeat) ? (X[r * kTIn + kk] - model[kOffMu + kk]) * model[kOffIsd + kk]
-                                                      : 0.f;
+            for (int q = 0; q < 2; q++) {
+                *reinterpret_cast<uint4*>(a1 + 16 * ((2 * h + q) ^ (r & 7))) =
+                    make_uint4(hi[4 * q], hi[4 * q + 1], hi[4 * q + 2], hi[4 * q + 3]);
+                *reinterpret_cast<uint4*>(a1 + 16 * ((4 + 2 * h + q) ^ (r & 7))) =
+                    make_uint4(lo[4 * q], lo[4 * q + 1], lo[4 * q + 2], lo[4 * q + 3]);
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mt_before_sync();
+        __syncthreads();
+        if (tid == 0) {
+            mt_after_sync();
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                mt_mma(d1, mt_desc(sb + kMtA + 2 * kMtTile + 32 * k), mt_desc(sb + kMtW1 + 32 * k), k > 0);
+            mt_commit(barL);
+        }
+        if (!dead) dead = !mt_wait(barL, phL);
+        phL ^= 1u;
+        mt_after_sync();
+#pragma unroll 1
+        for (int c = 0; c < 4; c++) {
+            // the buffer's last MMAs (chunk c - 2) are done before it is written
+            if (c >= 2) {
+                if (c & 1) {
+                    if (!dead) dead = !mt_wait(bar1, ph1);
+                    ph1 ^= 1u;
+                } else {
+                    if (!dead) dead = !mt_wait(bar0, ph0);
+                    ph0 ^= 1u;
                 }
             }
-            split2(v[0][0], v[0][1], xa[ks][hf * 2 + 0], xl[ks][hf * 2 + 0]);
-            split2(v[1][0], v[1][1], xa[ks][hf * 2 + 1], xl[ks][hf * 2 + 1]);
-        }
-    }
-    const uint2* P1 = pk;
-    const uint2* P2 = pk + 2 * 32 * 32;
-    float acc[32][4];
+            uint32_t v[32];
+            const int col = 64 * c + 32 * hf;
+            mt_ld32(v, d1 + lanes + (uint32_t)col);
+            uint8_t* ah = base + kMtA + (uint32_t)(c & 1) * 2 * kMtTile + 128 * row;
+            uint8_t* al = ah + kMtTile;
 #pragma unroll
-    for (int nt = 0; nt < 32; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-#pragma unroll 1
-    for (int ch = 0; ch < 16; ch++) {
-        // layer 1, hidden units 16 ch .. 16 ch + 15 (n-tiles 2 ch, 2 ch + 1)
-        float h[2][4];
+            for (int q = 0; q < 4; q++) {  // eight units: one 16-byte piece of hi and of lo
+                const float4 b0 = __ldg(reinterpret_cast<const float4*>(model + kOffB1 + col + 8 * q));
+                const float4 b1 = __ldg(reinterpret_cast<const float4*>(model + kOffB1 + col + 8 * q + 4));
+                const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+                uint32_t hi[4], lo[4];
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            h[j][0] = h[j][1] = h[j][2] = h[j][3] = 0.f;
-            const int nt = 2 * ch + j;
-#pragma unroll
-            for (int ks = 0; ks < 2; ks++) {
-                const uint2 b = P1[(ks * 32 + nt) * 32 + lane];
-                mma_bf16(h[j], xa[ks][0], xa[ks][1], xa[ks][2], xa[ks][3], b);
-                mma_bf16(h[j], xl[ks][0], xl[ks][1], xl[ks][2], xl[ks][3], b);
+                for (int e = 0; e < 4; e++)
+                    split2(fmaxf(__uint_as_float(v[8 * q + 2 * e]) + bb[2 * e], 0.f),
+                           fmaxf(__uint_as_float(v[8 * q + 2 * e + 1]) + bb[2 * e + 1], 0.f), hi[e], lo[e]);
+                const int j = (4 * hf + q) ^ (row & 7);
+                *reinterpret_cast<uint4*>(ah + 16 * j) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(al + 16 * j) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
-            const float b0 = model[kOffB1 + nt * 8 + qc], b1 = model[kOffB1 + nt * 8 + qc + 1];
-            h[j][0] = fmaxf(h[j][0] + b0, 0.f);
-            h[j][1] = fmaxf(h[j][1] + b1, 0.f);
-            h[j][2] = fmaxf(h[j][2] + b0, 0.f);
-            h[j][3] = fmaxf(h[j][3] + b1, 0.f);
-        }
-        // the two accumulator tiles are the layer-2 A operand of k-step ch
-        uint32_t ah[4], al[4];
-        split2(h[0][0], h[0][1], ah[0], al[0]);
-        split2(h[0][2], h[0][3], ah[1], al[1]);
-        split2(h[1][0], h[1][1], ah[2], al[2]);
-        split2(h[1][2], h[1][3], ah[3], al[3]);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mt_before_sync();
+            __syncthreads();
+            if (tid == 0) {
+                mt_after_sync();
+                const uint32_t a0 = sb + kMtA + (uint32_t)(c & 1) * 2 * kMtTile, b0 = sb + kMtW2 + (uint32_t)c * 2 * kMtTile;
 #pragma unroll
-        for (int nt = 0; nt < 32; nt++) {
-            const uint2 b = P2[(ch * 32 + nt) * 32 + lane];
-            mma_bf16(acc[nt], ah[0], ah[1], ah[2], ah[3], b);
-            mma_bf16(acc[nt], al[0], al[1], al[2], al[3], b);
+                for (int k = 0; k < 4; k++) {
+                    mt_mma(d2, mt_desc(a0 + 32 * k), mt_desc(b0 + 32 * k), c > 0 || k > 0);
+                    mt_mma(d2, mt_desc(a0 + kMtTile + 32 * k), mt_desc(b0 + 32 * k), 1u);
+                }
+                mt_commit(c & 1 ? bar1 : bar0);
+            }
         }
-    }
-    // layer 3
-    const __nv_bfloat16* W3 = wb + kOffW3;
-    float sa = 0.f, sb = 0.f;
+        if (!dead) dead = !mt_wait(bar0, ph0);
+        ph0 ^= 1u;
+        if (!dead) dead = !mt_wait(bar1, ph1);
+        ph1 ^= 1u;
+        mt_after_sync();
+        // layer 3: this thread's 128 columns of its row
+        float sum = 0.f;
+#pragma unroll 1
+        for (int c = 0; c < 4; c++) {
+            uint32_t v[32];
+            const int col = 128 * hf + 32 * c;
+            mt_ld32(v, d2 + lanes + (uint32_t)col);
 #pragma unroll
-    for (int nt = 0; nt < 32; nt++) {
-        const int c = nt * 8 + qc;
-        const float b0 = model[kOffB2 + c], b1 = model[kOffB2 + c + 1];
-        const float w0 = __bfloat162float(W3[c]), w1 = __bfloat162float(W3[c + 1]);
-        sa = fmaf(fmaxf(acc[nt][0] + b0, 0.f), w0, sa);
-        sa = fmaf(fmaxf(acc[nt][1] + b1, 0.f), w1, sa);
-        sb = fmaf(fmaxf(acc[nt][2] + b0, 0.f), w0, sb);
-        sb = fmaf(fmaxf(acc[nt][3] + b1, 0.f), w1, sb);
+            for (int q = 0; q < 8; q++) {
+                const float4 b = __ldg(reinterpret_cast<const float4*>(model + kOffB2 + col + 4 * q));
+                const float4 w3 = bf4(__ldg(reinterpret_cast<const uint2*>(wb + kOffW3 + col + 4 * q)));
+                sum = fmaf(fmaxf(__uint_as_float(v[4 * q]) + b.x, 0.f), w3.x, sum);
+                sum = fmaf(fmaxf(__uint_as_float(v[4 * q + 1]) + b.y, 0.f), w3.y, sum);
+                sum = fmaf(fmaxf(__uint_as_float(v[4 * q + 2]) + b.z, 0.f), w3.z, sum);
+                sum = fmaf(fmaxf(__uint_as_float(v[4 * q + 3]) + b.w, 0.f), w3.w, sum);
+            }
+        }
+        if (hf) half_dot[row] = sum;
+        mt_before_sync();
+        __syncthreads();
+        mt_after_sync();
+        const uint64_t gr = tile * kMtRows + row;
+        if (!hf && gr < n) logit[gr] = sum + half_dot[row] + model[kOffB3];
     }
-    sa += __shfl_xor_sync(0xffffffffu, sa, 1);
-    sa += __shfl_xor_sync(0xffffffffu, sa, 2);
-    sb += __shfl_xor_sync(0xffffffffu, sb, 1);
-    sb += __shfl_xor_sync(0xffffffffu, sb, 2);
-    if ((lane & 3) == 0) {
-        if (ra < n) logit[ra] = sa + model[kOffB3];
-        if (rb < n) logit[rb] = sb + model[kOffB3];
+    if (dead) atomicExch(err, 1u);
+    mt_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        mt_after_sync();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" : : "r"(tmem) : "memory");
     }
 }
 
@@ -664,15 +789,10 @@ static int upload_model(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* ho
 
 int triage_upload_model(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* host_model) {
     CUALLOC(h, model, kModelFloats * 4);
-    CUALLOC(h, wb, kPackOff + kPackBytes);
+    CUALLOC(h, wb, kModelFloats * 2);
     CU(h, cudaMemcpyAsync(model.p, host_model, kModelFloats * 4, cudaMemcpyHostToDevice, h->stream));
     k_to_bf16<<<nblocks(kModelFloats, 256), 256, 0, h->stream>>>(model.as<float>(), kModelFloats,
                                                                  wb.as<__nv_bfloat16>());
-    // tensor-core fragments of W1 (2 x 32 tiles) and W2 (16 x 32 tiles)
-    const __nv_bfloat16* w = wb.as<__nv_bfloat16>();
-    uint2* pk = reinterpret_cast<uint2*>(wb.as<uint8_t>() + kPackOff);
-    k_pack_b<<<nblocks(2 * 32 * 32, 256), 256, 0, h->stream>>>(w + kOffW1, 2, pk);
-    k_pack_b<<<nblocks(16 * 32 * 32, 256), 256, 0, h->stream>>>(w + kOffW2, 16, pk + 2 * 32 * 32);
     CU(h, cudaGetLastError());
     return SABER_OK;
 }
@@ -815,11 +935,17 @@ int triage_train(saber_gpu* h, float* model, const float* X, const uint8_t* y, u
 // logits of n feature rows with the installed model or the given one
 int triage_predict(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* d_X, uint64_t n, float* d_logit) {
     if (n == 0) return SABER_OK;
-    const uint64_t warps = (n + 15) / 16;
-    k_mlp_infer<<<(unsigned)((warps + 3) / 4), 128, 0, h->stream>>>(
-        d_X, n, model.as<float>(), reinterpret_cast<const uint2*>(wb.as<uint8_t>() + kPackOff),
-        wb.as<__nv_bfloat16>(), d_logit);
+    CUALLOC(h, h->tr_err, 4);
+    CU(h, cudaMemsetAsync(h->tr_err.p, 0, 4, h->stream));
+    CU(h, cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMtSmem));
+    const unsigned grid = (unsigned)std::min<uint64_t>((n + kMtRows - 1) / kMtRows, (uint64_t)h->sm_count);
+    k_mlp_tc<<<grid, kMtThreads, kMtSmem, h->stream>>>(d_X, n, model.as<float>(), wb.as<__nv_bfloat16>(), d_logit,
+                                                       h->tr_err.as<uint32_t>());
     CU(h, cudaGetLastError());
+    uint32_t e = 0;
+    CU(h, cudaMemcpyAsync(&e, h->tr_err.p, 4, cudaMemcpyDeviceToHost, h->stream));
+    CU(h, cudaStreamSynchronize(h->stream));
+    if (e) return fail(h, SABER_ERR_DEVICE, "the triage network's matrix pipeline did not complete");
     return SABER_OK;
 }
 
