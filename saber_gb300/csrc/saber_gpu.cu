@@ -553,6 +553,12 @@ static uint64_t pow2_at_least(uint64_t v, uint64_t lo) {
     return p;
 }
 
+// Padded job count of a scoring graph: a power of two from 4,096 on, and 1,024
+// for the smallest batches, whose keys one block sorts (a search's one query
+// has a few hundred regions; the eight digit passes over 4,096 padded keys took
+// longer than scoring them).
+static uint64_t pad_jobs(uint64_t n) { return n <= 1024 ? 1024 : pow2_at_least(n, 1 << 12); }
+
 // The scoring pipeline as a CUDA graph: the same kernels as score_pipeline
 // with every count kept on the device (the real job count in a device word,
 // padded entries sorted last as empty jobs), scratch sized for a power-of-two
@@ -563,7 +569,7 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     if (!sch.has) return fail(h, SABER_ERR_STATE, "no scoring scheme set");
     if (!ds.has_db) return fail(h, SABER_ERR_STATE, "no database loaded");
     if (!ds.qs.has) return fail(h, SABER_ERR_STATE, "no query set loaded");
-    const uint64_t npad = pow2_at_least(njobs, 1 << 12);
+    const uint64_t npad = pad_jobs(njobs);
     const uint64_t wcap = pow2_at_least(wmax + 1, 64);
     if (npad >= (1ull << 31)) return fail(h, SABER_ERR_ARG, "too many jobs in one call");
     cudaStream_t s = h->stream;
@@ -732,7 +738,7 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
 }
 
 int reserve_resident_jobs(saber_gpu* h, uint64_t njobs) {
-    const uint64_t n = h->use_graphs ? pow2_at_least(njobs, 1 << 12) : njobs;
+    const uint64_t n = h->use_graphs ? pad_jobs(njobs) : njobs;
     CUALLOC(h, h->jobs_dev, n * sizeof(saber_band_job));
     CUALLOC(h, h->scores_dev, n * 4);
     return SABER_OK;

@@ -743,6 +743,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 1) k_scan_few(const __grid_con
             for (int k = 0; k < W; k++) win[k] = __funnelshift_r(x[k], x[k + 1], 4 * (lane & 7));
             uint32_t mine = 0;  // bit: this position passes shape s0 + bit
             const uint32_t* fs = fil;
+#pragma unroll 4
             for (uint32_t si = a.s0; si < a.s1; si++, fs += a.fil_words) {
                 uint32_t hsum = 0;
 #pragma unroll
