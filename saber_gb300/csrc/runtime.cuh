@@ -133,6 +133,8 @@ struct Scheme {
 struct saber_gpu {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t copy_stream = nullptr;  // host-to-device copies beside the stream's work (made on first use)
+    cudaEvent_t copy_event = nullptr;
     std::mutex mu;
     std::string err;
     int sm_count = 0;

@@ -1492,6 +1492,11 @@ int saber_gpu_close(saber_gpu* h) {
         cudaStreamSynchronize(h->stream);
         cudaStreamDestroy(h->stream);
     }
+    if (h->copy_stream) {
+        cudaStreamSynchronize(h->copy_stream);
+        cudaStreamDestroy(h->copy_stream);
+        if (h->copy_event) cudaEventDestroy(h->copy_event);
+    }
     for (auto& g : h->graphs) cudaGraphExecDestroy(g.second.exec);
     h->graphs.clear();
     delete h;

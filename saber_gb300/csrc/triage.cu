@@ -932,16 +932,20 @@ int triage_train(saber_gpu* h, float* model, const float* X, const uint8_t* y, u
     return SABER_OK;
 }
 
-// logits of n feature rows with the installed model or the given one
-int triage_predict(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* d_X, uint64_t n, float* d_logit) {
-    if (n == 0) return SABER_OK;
-    CUALLOC(h, h->tr_err, 4);
-    CU(h, cudaMemsetAsync(h->tr_err.p, 0, 4, h->stream));
+static int mlp_launch(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* d_X, uint64_t n, float* d_logit) {
     CU(h, cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMtSmem));
     const unsigned grid = (unsigned)std::min<uint64_t>((n + kMtRows - 1) / kMtRows, (uint64_t)h->sm_count);
     k_mlp_tc<<<grid, kMtThreads, kMtSmem, h->stream>>>(d_X, n, model.as<float>(), wb.as<__nv_bfloat16>(), d_logit,
                                                        h->tr_err.as<uint32_t>());
     CU(h, cudaGetLastError());
+    return SABER_OK;
+}
+static int mlp_begin(saber_gpu* h) {
+    CUALLOC(h, h->tr_err, 4);
+    CU(h, cudaMemsetAsync(h->tr_err.p, 0, 4, h->stream));
+    return SABER_OK;
+}
+static int mlp_end(saber_gpu* h) {
     uint32_t e = 0;
     CU(h, cudaMemcpyAsync(&e, h->tr_err.p, 4, cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
@@ -949,18 +953,48 @@ int triage_predict(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* d_X, ui
     return SABER_OK;
 }
 
+// logits of n feature rows with the installed model or the given one
+int triage_predict(saber_gpu* h, DevBuf& model, DevBuf& wb, const float* d_X, uint64_t n, float* d_logit) {
+    if (n == 0) return SABER_OK;
+    int rc = mlp_begin(h);
+    if (rc == SABER_OK) rc = mlp_launch(h, model, wb, d_X, n, d_logit);
+    return rc != SABER_OK ? rc : mlp_end(h);
+}
+
+// Rows of a chunk of a host call: a chunk's copy (16 MB) runs on the handle's
+// copy stream while the chunk before it is computed.  1 M rows on one GB300:
+// 1154 us in one piece, 921 in eight.
+constexpr uint64_t kPredictChunk = 128 << 10;
+
 int triage_predict_host(saber_gpu* h, const float* model, const float* X, uint64_t n, float* logits) {
     TriageScratch& d = h->tg;
     int rc = upload_model(h, d.model, d.wb, model);
     if (rc != SABER_OK) return rc;
     CUALLOC(h, d.X, std::max<uint64_t>(n, 1) * kTIn * 4);
     CUALLOC(h, d.z, std::max<uint64_t>(n, 1) * 4);
-    CU(h, cudaMemcpyAsync(d.X.p, X, n * kTIn * 4, cudaMemcpyHostToDevice, h->stream));
-    rc = triage_predict(h, d.model, d.wb, d.X.as<float>(), n, d.z.as<float>());
+    rc = mlp_begin(h);
     if (rc != SABER_OK) return rc;
+    if (!h->copy_stream) {
+        CU(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
+        CU(h, cudaEventCreateWithFlags(&h->copy_event, cudaEventDisableTiming));
+    }
+    // (the buffers are the handle's, and every earlier call has waited for its
+    // stream; no return leaves a copy from the caller's rows in flight)
+    struct Wait {
+        cudaStream_t s;
+        ~Wait() { cudaStreamSynchronize(s); }
+    } wait{h->copy_stream};
+    for (uint64_t r = 0; r < n; r += kPredictChunk) {
+        const uint64_t k = std::min<uint64_t>(kPredictChunk, n - r);
+        CU(h, cudaMemcpyAsync(d.X.as<float>() + r * kTIn, X + r * kTIn, k * kTIn * 4, cudaMemcpyHostToDevice,
+                              h->copy_stream));
+        CU(h, cudaEventRecord(h->copy_event, h->copy_stream));
+        CU(h, cudaStreamWaitEvent(h->stream, h->copy_event, 0));
+        rc = mlp_launch(h, d.model, d.wb, d.X.as<float>() + r * kTIn, k, d.z.as<float>() + r);
+        if (rc != SABER_OK) return rc;
+    }
     CU(h, cudaMemcpyAsync(logits, d.z.p, n * 4, cudaMemcpyDeviceToHost, h->stream));
-    CU(h, cudaStreamSynchronize(h->stream));
-    return SABER_OK;
+    return mlp_end(h);
 }
 
 // Region features for the engine: uploads the batch's regions and computes

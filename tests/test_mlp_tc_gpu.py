@@ -1,6 +1,6 @@
 """The triage network's tcgen05 inference against the float64 oracle, at the
-edges of its tiles of 128 rows and of its grid of one block per SM, and split
-into smaller calls.
+edges of its tiles of 128 rows, of its grid of one block per SM and of a host
+call's chunks, and split into smaller calls.
 
 Tolerance: activations enter as bf16 pairs (2^-16 of each value), accumulation
 is fp32 over 256 terms: 2e-5 of the largest logit leaves a factor of five over
@@ -20,7 +20,7 @@ def _rows(rng, n):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [1, 127, 128, 129, 1000, 16511, 16513, 152 * 128, 152 * 128 + 1, 40001])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 1000, 16511, 16513, 152 * 128, 152 * 128 + 1, 40001, 131072, 131073, 262145])
 def test_logits_match_oracle(n):
     rng = np.random.default_rng(n)
     x = _rows(rng, n)
