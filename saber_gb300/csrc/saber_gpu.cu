@@ -368,6 +368,11 @@ static WaveArgs wave_args(const Scheme& sch, const Dataset& ds, const saber_band
     return a;
 }
 
+// First key bit that the sort looks at.  Without strip classes (long_steps 0:
+// every job goes to the anti-diagonal kernel) only the class and the size in
+// steps of 512 cells matter: four digit passes instead of eight.
+static int sort_from(uint32_t long_steps) { return long_steps == 0 ? 36 : 0; }
+
 static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, const saber_band_job* d_jobs,
                           uint64_t njobs, int32_t* d_scores, saber_score_stats* st) {
     if (!sch.has) return fail(h, SABER_ERR_STATE, "no scoring scheme set");
@@ -399,6 +404,7 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     int rc0 = jobs_cells(h, qs, d_jobs, njobs, &job_cells);
     if (rc0 != SABER_OK) return rc0;
     const uint32_t long_steps = long_steps_for(h, job_cells);
+    const int key_from = sort_from(long_steps);
     cudaEvent_t ev[4];
     for (int i = 0; i < 4; i++) CU(h, cudaEventCreate(&ev[i]));
     struct EvGuard {
@@ -420,13 +426,13 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     size_t t_sort = 0;
     CU(h, cub::DeviceRadixSort::SortPairs(nullptr, t_sort, h->keys_in.as<uint64_t>(),
                                           h->keys_out.as<uint64_t>(), h->vals_in.as<uint32_t>(),
-                                          h->vals_out.as<uint32_t>(), (int)n, 0, 64, s));
+                                          h->vals_out.as<uint32_t>(), (int)n, key_from, 64, s));
     CUALLOC(h, h->cub_tmp, t_sort);
     size_t tb = h->cub_tmp.cap;
     CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, tb, h->keys_in.as<uint64_t>(),
                                           h->keys_out.as<uint64_t>(), h->vals_in.as<uint32_t>(),
-                                          h->vals_out.as<uint32_t>(), (int)n, 0, 64, s));
-    local.library_launches += 9;  // onesweep radix sort: histogram + 8 digit passes
+                                          h->vals_out.as<uint32_t>(), (int)n, key_from, 64, s));
+    local.library_launches += 1 + (64 - key_from) / 8;  // onesweep radix sort: histogram + digit passes
 
     // one small read-back: class counts and widths size the scratch
     uint32_t hc[20];
@@ -585,13 +591,17 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     const int rows0 = h->strip_rows;
     const unsigned grid0 = (unsigned)(h->sm_count * band_fast_blocks_per_sm(rows0, qs.p8));
     const unsigned grid8 = (unsigned)(h->sm_count * band_fast_blocks_per_sm(kStripRowsMin, qs.p8));
+    const uint32_t long_steps = long_steps_for(h, job_cells);
+    const int key_from = sort_from(long_steps);
+    const bool strips = long_steps != 0;  // the strip classes can hold jobs
     const uint64_t warps = (uint64_t)std::max(grid0, grid8) * 256 / 32;
-    CUALLOC(h, h->bufs, warps * wcap * 32 * sizeof(uint2));
+    if (strips) CUALLOC(h, h->bufs, warps * wcap * 32 * sizeof(uint2));
     const unsigned gT = 128, gGrid = (unsigned)(h->sm_count * 4);
     CUALLOC(h, h->slabs, (uint64_t)gGrid * (gT / 32) * wcap * 4 * sizeof(int32_t));
     size_t t_sort = 0;
     CU(h, cub::DeviceRadixSort::SortPairs(nullptr, t_sort, h->keys_in.as<uint64_t>(), h->keys_out.as<uint64_t>(),
-                                          h->vals_in.as<uint32_t>(), h->vals_out.as<uint32_t>(), (int)npad, 0, 64, s));
+                                          h->vals_in.as<uint32_t>(), h->vals_out.as<uint32_t>(), (int)npad, key_from, 64,
+                                          s));
     CUALLOC(h, h->cub_tmp, t_sort);
     GraphKey key;
     std::memset(&key, 0, sizeof(key));
@@ -601,7 +611,6 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     key.go = sch.go;
     key.ge = sch.ge;
     key.pair_steps = h->pair_steps;
-    const uint32_t long_steps = long_steps_for(h, job_cells);
     key.long_steps = long_steps;
     key.n_res = ds.n_res;  // scalar kernel parameters baked into the graph
     key.nq = qs.nq;
@@ -635,12 +644,12 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
         chk(cudaGetLastError());
         size_t tb = h->cub_tmp.cap;
         chk(cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, tb, h->keys_in.as<uint64_t>(), h->keys_out.as<uint64_t>(),
-                                            h->vals_in.as<uint32_t>(), h->vals_out.as<uint32_t>(), (int)npad, 0, 64,
+                                            h->vals_in.as<uint32_t>(), h->vals_out.as<uint32_t>(), (int)npad, key_from, 64,
                                             s));
         const uint32_t* order = h->vals_out.as<uint32_t>();
         k_copy_generic<<<h->sm_count * 4, 256, 0, s>>>(order, counts, h->list.as<uint32_t>());
         chk(cudaGetLastError());
-        for (int pass = 0; pass < 2; pass++) {
+        for (int pass = 0; pass < 2 && strips; pass++) {
             FastArgs a;
             a.res = ds.res.as<uint8_t>();
             a.prof = qs.prof.as<int16_t>();
@@ -728,8 +737,8 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
         local.generic_jobs = hc[1] + hc[19];
         local.empty_jobs = hc[4];
         local.i16_rescored = hc[5] - hc[1];
-        local.kernel_launches = 6;
-        local.library_launches = 9;
+        local.kernel_launches = strips ? 6 : 4;
+        local.library_launches = 1 + (64 - key_from) / 8;
         local.t_fast_ms = ms;
         local.prof8 = qs.p8 ? 1 : 0;
         *st = local;
