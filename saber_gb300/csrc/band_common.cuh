@@ -106,7 +106,7 @@ struct GenericArgs {
 // indices per lane, widest first.
 constexpr int kWaveClasses = 7;
 constexpr int kWaveMaxWidth = 1024;  // 32 lanes x 32 band indices
-constexpr int kWaveRowBytes = 52;    // row pitch of its score table (QuerySet::qrow holds row offsets)
+constexpr int kWaveRowBytes = 1250;  // row pitch of its score tables (25 x 25 pairs of bytes)
 // Class of a band of width w <= kWaveMaxWidth: 32 lanes of 32, 16, 8 and 4
 // band indices, then 16, 9 and 8 lanes of 4.  Nine lanes (three jobs per
 // warp) take the prefilter band of a seed hit, 2 x 16 + 1 wide, which sixteen
@@ -117,6 +117,7 @@ __host__ __device__ inline int wave_class(int64_t w) {
 struct WaveArgs {
     const uint8_t* res;
     const uint32_t* qrow;    // per batch position: table row offset | bias << 16
+    const uint8_t* pairs;    // the scheme's pair table, or null: the int16 table of the matrix
     const int32_t* matrix;   // 24 x 24
     const uint64_t* qoffs;
     const saber_band_job* jobs;

@@ -19,15 +19,21 @@
 // A lane's rows at one step are i0, i0 - 1, ..., i0 - 2J + 1 and its columns
 // c0 .. c0 + 2J; both windows advance by one per two steps, so one query
 // letter and one subject letter enter per lane and two steps (fetched four
-// pairs of steps ahead).  Scores come from the 24 x 24 matrix in shared
-// memory (int16, S + go) plus the packed query bias of the row pair.
+// pairs of steps ahead).  A row meets column c in an even step and column
+// c + 1 in the odd step after it, so the scores (S + go) are kept in shared
+// memory per code and pair of column codes, two bytes each: one 16-bit read
+// serves both steps, and a byte permute widens it (31 KB; schemes whose scores
+// do not fit in a byte read a 25 x 25 int16 table per step).  The packed query
+// bias of the row pair is added.
 //
-// Bound: L1 wavefronts of the score gathers (95 % busy at 100 k jobs, 2.75
-// wavefronts per gather; ALU pipe 68 %), 1.3e12 cells/s, half the strip
-// kernel's rate at a full device but reached from a few thousand jobs on.
-// One GB300: 3,001 host jobs (half-widths 4..64) 1.78 -> 0.28 ms a call, 40
-// full windows of a 310-residue query 0.86 -> 0.38 ms, 2 x 3,662 kilobase DNA
-// bands 16.5 -> 5.4 ms of scoring.
+// Bound: the ALU pipe (75 % busy at 100 k jobs; L1 80 %, issue slots 70 %).
+// With the int16 table alone it was L1 wavefronts of the gathers (95 %): 100 k
+// jobs 1.69 -> 1.41 ms, 300 k 4.77 -> 3.91, 1 M 15.5 -> 12.7, against 8.2 in
+// the strip kernel, whose rate needs a full device; this one reaches
+// 1.6e12 cells/s from a few thousand jobs on.
+// One GB300: 3,001 host jobs (half-widths 4..64) 1.78 -> 0.26 ms a call, 40
+// full windows of a 310-residue query 0.86 -> 0.26 ms, 2 x 3,662 kilobase DNA
+// bands 16.5 -> 4 ms of scoring.
 //
 // Cells left of column 0 or above row 0 hold H = 0 and E, F <= 0 from the
 // initial state on (their score is the sentinel), which is what the
@@ -41,10 +47,17 @@ namespace saber {
 
 constexpr unsigned kWaveThreads = 128;
 
+// Byte permute with sign replication (a selector nibble 8 | b: the sign of byte b).
+__device__ __forceinline__ uint32_t wv_sext(uint32_t x, uint32_t y, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(y), "r"(sel));
+    return d;
+}
+
 // Jobs [task * 32 / L, ...) of one (L, J) class of the sorted list, one per
 // group of L lanes.  L = 128: one job on the block's four warps, whose edge
 // lanes pass E and F through shared memory (xch), a barrier per step.
-template <int L, int J>
+template <int L, int J, bool P8>
 __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __restrict__ list, uint32_t njobs,
                                           uint32_t task, int lane, const uint8_t* tab, uint32_t* xch) {
     constexpr bool kBlock = L > 32;
@@ -76,7 +89,9 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
     int i0 = s0 / 2 - 2 * J * gl;
     int c0 = s0 / 2 + 2 * J * gl + lo;
 
-    uint32_t Ge[J], Go[J], E[J], F[J], keep_e[J], keep_o[J], R[2 * J], C[2 * J + 1], B[J];
+    // C: columns 0 .. 2J as offsets (int16 table), or column pairs 0 .. 2J - 1
+    // (pair table; `last` is the code of column 2J)
+    uint32_t Ge[J], Go[J], E[J], F[J], keep_e[J], keep_o[J], R[2 * J], C[2 * J + 1], B[J], last = 0;
 #pragma unroll
     for (int j = 0; j < J; j++) {
         Ge[j] = Go[j] = ngo2;
@@ -90,7 +105,15 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
         B[j] = wv_prmt(ra, rb, 0x7632);
     }
 #pragma unroll
-    for (int r = 0; r <= 2 * J; r++) C[r] = 2 * wv_col(win, c0 + r, n);
+    for (int r = 0; r <= 2 * J; r++) C[r] = wv_col(win, c0 + r, n);
+    if (P8) {
+        last = C[2 * J];
+#pragma unroll
+        for (int r = 0; r < 2 * J; r++) C[r] = 50 * C[r] + 2 * C[r + 1];
+    } else {
+#pragma unroll
+        for (int r = 0; r <= 2 * J; r++) C[r] *= 2;
+    }
     // letters of the next kWaveAhead pairs of steps
     uint32_t qn[kWaveAhead], sn[kWaveAhead];
 #pragma unroll
@@ -108,6 +131,14 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
     for (int it = 0; it < nmax; it += kWaveAhead) {
 #pragma unroll
         for (int t = 0; t < kWaveAhead; t++) {
+            uint32_t X[P8 ? J : 1], Y[P8 ? J : 1];  // both steps' scores of the rows 2j and 2j + 1
+            if (P8) {
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    X[P8 ? j : 0] = *reinterpret_cast<const uint16_t*>(tab + R[2 * j] + C[2 * j]);
+                    Y[P8 ? j : 0] = *reinterpret_cast<const uint16_t*>(tab + R[2 * j + 1] + C[2 * j + 1]);
+                }
+            }
             // even step: E, F come in from the odd band indices
             uint32_t left = __shfl_up_sync(0xffffffffu, E[J - 1], 1);
             if (kBlock && lane == 0 && wib > 0) left = xch[wib - 1];
@@ -118,7 +149,9 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
                 const uint32_t Ein = wv_prmt(left, own, 0x5432);
                 left = own;
                 const uint32_t Fin = F[j];
-                const uint32_t ds = __vadd2(Ge[j], wv_sub(tab, R[2 * j], C[2 * j], R[2 * j + 1], C[2 * j + 1], B[j]));
+                const uint32_t ds =
+                    __vadd2(Ge[j], P8 ? __vadd2(wv_sext(X[P8 ? j : 0], Y[P8 ? j : 0], 0xC480u), B[j])
+                                      : wv_sub(tab, R[2 * j], C[2 * j], R[2 * j + 1], C[2 * j + 1], B[j]));
                 const uint32_t H = __vimax3_s16x2_relu(Ein, Fin, ds) & keep_e[j];
                 const uint32_t Gv = __vadd2(H, ngo2);
                 Ge[j] = Gv;
@@ -138,7 +171,9 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
             for (int j = 0; j < J; j++) {
                 const uint32_t Ein = E[j];
                 const uint32_t Fin = wv_prmt(F[j], j + 1 < J ? F[j + 1 < J ? j + 1 : j] : down, 0x5432);
-                const uint32_t ds = __vadd2(Go[j], wv_sub(tab, R[2 * j], C[2 * j + 1], R[2 * j + 1], C[2 * j + 2], B[j]));
+                const uint32_t ds =
+                    __vadd2(Go[j], P8 ? __vadd2(wv_sext(X[P8 ? j : 0], Y[P8 ? j : 0], 0xD591u), B[j])
+                                      : wv_sub(tab, R[2 * j], C[2 * j + 1], R[2 * j + 1], C[2 * j + 2], B[j]));
                 const uint32_t H = __vimax3_s16x2_relu(Ein, Fin, ds) & keep_o[j];
                 const uint32_t Gv = __vadd2(H, ngo2);
                 Go[j] = Gv;
@@ -157,9 +192,16 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
 #pragma unroll
             for (int r = 2 * J - 1; r > 0; r--) R[r] = R[r - 1];
             R[0] = qn[t] & 0xFFFFu;
+            if (P8) {
 #pragma unroll
-            for (int r = 0; r < 2 * J; r++) C[r] = C[r + 1];
-            C[2 * J] = 2 * sn[t];
+                for (int r = 0; r < 2 * J - 1; r++) C[r] = C[r + 1];
+                C[2 * J - 1] = 50 * last + 2 * sn[t];
+                last = sn[t];
+            } else {
+#pragma unroll
+                for (int r = 0; r < 2 * J; r++) C[r] = C[r + 1];
+                C[2 * J] = 2 * sn[t];
+            }
             i0++;
             c0++;
             qn[t] = wv_row(qrow, i0, m);
@@ -189,12 +231,29 @@ __device__ __forceinline__ void wave_task(const WaveArgs& a, const uint32_t* __r
 
 // Persistent warps over warp tasks of the classes, widest bands first; within
 // a class the list is largest first.
+template <bool P8>
 __global__ void __launch_bounds__(kWaveThreads, 4) k_band_wave(WaveArgs a) {
-    __shared__ __align__(4) int16_t tab[25 * kWaveRow / 2];
+    __shared__ __align__(16) uint8_t tab[(kWavePairBytes + 15) / 16 * 16];
     __shared__ uint32_t xch[8];
-    wv_table(tab, a.matrix, a.go);
+    if (P8) {
+        // every load of the copy in flight at once: a batch of a few jobs waits for it
+        constexpr int kVec = (kWavePairBytes + 15) / 16, kPer = (kVec + kWaveThreads - 1) / kWaveThreads;
+        uint4 v[kPer];
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+            const int t = i * kWaveThreads + threadIdx.x;
+            if (t < kVec) v[i] = __ldg(reinterpret_cast<const uint4*>(a.pairs) + t);
+        }
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+            const int t = i * kWaveThreads + threadIdx.x;
+            if (t < kVec) reinterpret_cast<uint4*>(tab)[t] = v[i];
+        }
+    } else {
+        wv_table(reinterpret_cast<int16_t*>(tab), a.matrix, a.go);
+    }
     __syncthreads();
-    const uint8_t* tb = reinterpret_cast<const uint8_t*>(tab);
+    const uint8_t* tb = tab;
     const int lane = threadIdx.x & 31;
     uint32_t n[kWaveClasses], tasks[kWaveClasses], total = 0;
 #pragma unroll
@@ -211,8 +270,8 @@ __global__ void __launch_bounds__(kWaveThreads, 4) k_band_wave(WaveArgs a) {
     // keep every warp busy by themselves, and a lane's sets share its overheads.
     if (n[0] + n[1] <= 2 * gridDim.x) {
         for (uint32_t p = blockIdx.x; p < n[0] + n[1]; p += gridDim.x) {
-            if (p < n[0]) wave_task<128, 2>(a, list, n[0], p, lane, tb, xch);
-            else wave_task<128, 1>(a, list + n[0], n[1], p - n[0], lane, tb, xch);
+            if (p < n[0]) wave_task<128, 2, P8>(a, list, n[0], p, lane, tb, xch);
+            else wave_task<128, 1, P8>(a, list + n[0], n[1], p - n[0], lane, tb, xch);
         }
         total -= tasks[0] + tasks[1];
         tasks[0] = tasks[1] = 0;
@@ -224,47 +283,62 @@ __global__ void __launch_bounds__(kWaveThreads, 4) k_band_wave(WaveArgs a) {
         if (t >= total) break;
         const uint32_t* l = list;
         if (t < tasks[0]) {
-            wave_task<32, 8>(a, l, n[0], t, lane, tb, xch);
+            wave_task<32, 8, P8>(a, l, n[0], t, lane, tb, xch);
             continue;
         }
         t -= tasks[0];
         l += n[0];
         if (t < tasks[1]) {
-            wave_task<32, 4>(a, l, n[1], t, lane, tb, xch);
+            wave_task<32, 4, P8>(a, l, n[1], t, lane, tb, xch);
             continue;
         }
         t -= tasks[1];
         l += n[1];
         if (t < tasks[2]) {
-            wave_task<32, 2>(a, l, n[2], t, lane, tb, xch);
+            wave_task<32, 2, P8>(a, l, n[2], t, lane, tb, xch);
             continue;
         }
         t -= tasks[2];
         l += n[2];
         if (t < tasks[3]) {
-            wave_task<32, 1>(a, l, n[3], t, lane, tb, xch);
+            wave_task<32, 1, P8>(a, l, n[3], t, lane, tb, xch);
             continue;
         }
         t -= tasks[3];
         l += n[3];
         if (t < tasks[4]) {
-            wave_task<16, 1>(a, l, n[4], t, lane, tb, xch);
+            wave_task<16, 1, P8>(a, l, n[4], t, lane, tb, xch);
             continue;
         }
         t -= tasks[4];
         l += n[4];
         if (t < tasks[5]) {
-            wave_task<9, 1>(a, l, n[5], t, lane, tb, xch);
+            wave_task<9, 1, P8>(a, l, n[5], t, lane, tb, xch);
             continue;
         }
         t -= tasks[5];
         l += n[5];
-        wave_task<8, 1>(a, l, n[6], t, lane, tb, xch);
+        wave_task<8, 1, P8>(a, l, n[6], t, lane, tb, xch);
     }
 }
 
+// Pair table of a scheme (kWavePairBytes, 16-byte aligned).
+__global__ void k_wave_pairs(const int32_t* __restrict__ matrix, int go, uint8_t* __restrict__ pairs) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < kWavePairBytes / 2; t += gridDim.x * blockDim.x) {
+        const int q = t / 625, c = t / 25 % 25, d = t % 25;
+        const int x = q < 24 && c < 24 ? matrix[q * 24 + c] + go : -128, y = q < 24 && d < 24 ? matrix[q * 24 + d] + go : -128;
+        pairs[2 * t] = (uint8_t)(int8_t)x;
+        pairs[2 * t + 1] = (uint8_t)(int8_t)y;
+    }
+}
+cudaError_t launch_wave_pairs(cudaStream_t s, const int32_t* matrix, int go, uint8_t* pairs) {
+    k_wave_pairs<<<31, 256, 0, s>>>(matrix, go, pairs);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_band_wave(unsigned sm_count, cudaStream_t s, const WaveArgs& a) {
-    k_band_wave<<<sm_count * 4, kWaveThreads, 0, s>>>(a);
+    if (a.pairs) k_band_wave<true><<<sm_count * 4, kWaveThreads, 0, s>>>(a);
+    else k_band_wave<false><<<sm_count * 4, kWaveThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

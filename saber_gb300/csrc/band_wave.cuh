@@ -7,7 +7,7 @@
 
 namespace saber {
 
-constexpr int kWaveRow = kWaveRowBytes;   // bytes per row of the score table (26 entries)
+constexpr int kWaveRow = kWaveRowBytes;   // bytes per row of either score table
 constexpr int kWaveSent = 24;             // row / column of the sentinel score
 constexpr int kWaveAhead = 4;             // pairs of steps between a letter's load and its use
 
@@ -25,13 +25,24 @@ __device__ __forceinline__ uint32_t wv_col(const uint8_t* __restrict__ win, int 
 }
 
 // The score table: 24 x 24 matrix + gap open as int16, the sentinel in row and
-// column 24 (25 rows of kWaveRow bytes).
+// column 24, in 25 rows at the pitch of the pair table (a query's row words
+// serve both without a multiply between a letter and its score's read: 40
+// windows 257 -> 250 us).
 __device__ __forceinline__ void wv_table(int16_t* tab, const int32_t* __restrict__ matrix, int go) {
-    for (int t = threadIdx.x; t < 25 * (kWaveRow / 2); t += blockDim.x) {
-        const int r = t / (kWaveRow / 2), c = t - r * (kWaveRow / 2);
-        tab[t] = r < 24 && c < 24 ? (int16_t)(matrix[r * 24 + c] + go) : (int16_t)kSent16;
+    for (int t = threadIdx.x; t < 25 * 25; t += blockDim.x) {
+        const int r = t / 25, c = t - r * 25;
+        tab[r * (kWaveRow / 2) + c] =
+            r < 24 && c < 24 ? (int16_t)(matrix[r * 24 + c] + go) : (int16_t)kSent16;
     }
 }
+// The pair table of a scheme whose scores + gap open fit int8: for row code q
+// and two neighbouring column codes c, d the bytes S(q, c) + go, S(q, d) + go at
+// kWaveRow q + 50 c + 2 d (sentinel -128), so that one 16-bit read gives a
+// row's scores of an even and the following odd step.
+constexpr int kWavePairBytes = 25 * kWaveRow;
+static_assert(kWaveRow == 25 * 25 * 2, "a row holds every pair of column codes");
+cudaError_t launch_wave_pairs(cudaStream_t s, const int32_t* matrix, int go, uint8_t* pairs);  // band_wave.cu
+
 // Packed scores of two cells (low, high) plus the row pair's biases.
 __device__ __forceinline__ uint32_t wv_sub(const uint8_t* tab, uint32_t ra, uint32_t ca, uint32_t rb, uint32_t cb,
                                            uint32_t bias) {

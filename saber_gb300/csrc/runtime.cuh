@@ -126,6 +126,9 @@ struct Scheme {
     int32_t go = 11, ge = 1;
     bool has = false;
     DevBuf d_matrix;
+    bool pairs8 = false;               // every score + gap open fits in [-127, 127]: d_pairs is allocated,
+    mutable bool pairs_built = false;  // and filled by the scheme's first call that reads it
+    DevBuf d_pairs;
 };
 
 }  // namespace saber

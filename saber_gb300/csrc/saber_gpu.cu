@@ -76,7 +76,7 @@ __global__ void k_profile(const uint8_t* __restrict__ codes, const uint64_t* __r
         P[t] = (int16_t)(v + go);
         if (prof8) prof8[prof_off[q] + t] = real ? (int8_t)(v + go) : (int8_t)-128;
     }
-    // the anti-diagonal kernel's row words: table row offset | bias << 16
+    // the anti-diagonal kernels' row words: table row offset | bias << 16
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
         const int qc = codes[q0 + i];
         qrow[q0 + i] = (uint32_t)(kWaveRowBytes * (qc < 24 ? qc : 22)) |
@@ -185,7 +185,7 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
         }
         if (cls != 2 && (w >= (1 << 16) || ns >= (1 << 13))) cls = 2;
         // a sweep longer than long_steps column steps in one lane goes to the
-        // warp-per-job int32 kernel
+        // anti-diagonal kernel
         if (cls != 2) {
             // the sweep's steps per strip: the band's, or the window's when
             // the band is wider (the kernels sweep window columns only)
@@ -310,19 +310,39 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
 // and goes to the anti-diagonal kernel as a whole.  Scoring time on one GB300
 // by threshold 0 / 2048 / 4096 / 8192 / 16384 / none, bands half 8..128 wide,
 // by steps per lane:
-//      84 (10 k jobs)    0.28 / 1.13 / 1.79 / 3.24 / 3.30 / 3.35 ms
-//     883 (100 k)        1.69 / 2.05 / 2.34 / 3.24 / 3.85 / 3.89
-//    1751 (200 k)        3.21 / 2.85 / 2.66 / 3.56 / 4.06 / 4.19
-//    2641 (300 k)        4.77 / 3.87 / 3.58 / 3.89 / 4.59 / 4.50
-//    4374 (500 k)        7.82 / 5.87 / 4.94 / 4.84 / 5.29 / 5.27
-//    8750 (1 M)         15.48 / 10.8 / 8.80 / 8.59 / 8.16 / 8.21
+//      84 (10 k jobs)    0.25 / 1.10 / 1.71 / 3.22 / 3.30 / 3.27 ms
+//     883 (100 k)        1.41 / 1.99 / 2.09 / 3.15 / 3.79 / 3.80
+//    1751 (200 k)        2.67 / 2.78 / 2.61 / 3.50 / 4.14 / 4.04
+//    2641 (300 k)        3.91 / 3.54 / 3.36 / 3.98 / 4.56 / 4.51
+//    4374 (500 k)        6.41 / 5.27 / 4.80 / 4.86 / 5.30 / 5.18
+//    8750 (1 M)         12.71 / 9.63 / 8.57 / 8.40 / 8.22 / 8.21
 // and 11,000-query searches (30 k steps per lane) 131 / 65.0 / 64.1 / 64.1 /
 // 63.7 / 63.8 ms.
-constexpr uint64_t kLoadSmall = 1500;
+constexpr uint64_t kLoadSmall = 1650;
+// Below kLoadPairs steps per lane the anti-diagonal kernel reads the small
+// int16 score table instead of the pair table: a batch of a few jobs is one
+// job's chain of steps long, and building the pair table (a launch per scheme,
+// which a call on a query's windows sets anew) and copying it into every
+// block only add to it.  A call on 40 windows (2 steps per lane) 250 us with
+// the int16 table, 255 with the pair table; 3,001 bands (24 steps) 268 and 250.
+constexpr uint64_t kLoadPairs = 12;
+static uint64_t steps_per_lane(const saber_gpu* h, uint64_t cells) {
+    const uint64_t lanes = (uint64_t)h->sm_count * band_fast_blocks_per_sm(h->strip_rows, false) * 256;
+    return cells / 32 / (lanes ? lanes : 1);
+}
+static bool use_pairs(const saber_gpu* h, const Scheme& sch, uint64_t cells) {
+    return sch.pairs8 && (h->long_steps != kLongStepsAuto || steps_per_lane(h, cells) >= kLoadPairs);
+}
+// Builds the scheme's pair table if this is its first use.
+static cudaError_t ensure_pairs(saber_gpu* h, const Scheme& sch) {
+    if (sch.pairs_built) return cudaSuccess;
+    const cudaError_t e = launch_wave_pairs(h->stream, sch.d_matrix.as<int32_t>(), sch.go, sch.d_pairs.as<uint8_t>());
+    sch.pairs_built = e == cudaSuccess;
+    return e;
+}
 static uint32_t long_steps_for(const saber_gpu* h, uint64_t cells) {
     if (h->long_steps != kLongStepsAuto) return h->long_steps;
-    const uint64_t lanes = (uint64_t)h->sm_count * band_fast_blocks_per_sm(h->strip_rows, false) * 256;
-    const uint64_t load = cells / 32 / (lanes ? lanes : 1);
+    const uint64_t load = steps_per_lane(h, cells);
     if (load < kLoadSmall) return 0;
     uint64_t t = kLongStepsSmall;
     while (t < load + load / 4 && t < (1ull << 30)) t <<= 1;
@@ -348,11 +368,12 @@ static int jobs_cells(saber_gpu* h, const QuerySet& qs, const saber_band_job* d_
 }
 
 static WaveArgs wave_args(const Scheme& sch, const Dataset& ds, const saber_band_job* d_jobs, const uint32_t* order,
-                          uint32_t* counts, int32_t* d_scores, uint32_t* list) {
+                          uint32_t* counts, int32_t* d_scores, uint32_t* list, bool pairs) {
     WaveArgs a;
     a.res = ds.res.as<uint8_t>();
     a.qrow = ds.qs.qrow.as<uint32_t>();
     a.matrix = sch.d_matrix.as<int32_t>();
+    a.pairs = pairs ? sch.d_pairs.as<uint8_t>() : nullptr;
     a.qoffs = ds.qs.offsets.as<uint64_t>();
     a.jobs = d_jobs;
     a.order = order;
@@ -405,6 +426,8 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     if (rc0 != SABER_OK) return rc0;
     const uint32_t long_steps = long_steps_for(h, job_cells);
     const int key_from = sort_from(long_steps);
+    const bool pairs = use_pairs(h, sch, job_cells);
+    if (pairs) CU(h, ensure_pairs(h, sch));
     cudaEvent_t ev[4];
     for (int i = 0; i < 4; i++) CU(h, cudaEventCreate(&ev[i]));
     struct EvGuard {
@@ -497,7 +520,7 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
         local.kernel_launches++;
     }
     if (n_wave) {
-        WaveArgs wa = wave_args(sch, ds, d_jobs, order, counts, d_scores, h->list.as<uint32_t>());
+        WaveArgs wa = wave_args(sch, ds, d_jobs, order, counts, d_scores, h->list.as<uint32_t>(), pairs);
         CU(h, launch_band_wave((unsigned)h->sm_count, s, wa));
         local.kernel_launches++;
     }
@@ -593,6 +616,8 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     const unsigned grid8 = (unsigned)(h->sm_count * band_fast_blocks_per_sm(kStripRowsMin, qs.p8));
     const uint32_t long_steps = long_steps_for(h, job_cells);
     const int key_from = sort_from(long_steps);
+    const bool pairs = use_pairs(h, sch, job_cells);
+    if (pairs) CU(h, ensure_pairs(h, sch));
     const bool strips = long_steps != 0;  // the strip classes can hold jobs
     const uint64_t warps = (uint64_t)std::max(grid0, grid8) * 256 / 32;
     if (strips) CUALLOC(h, h->bufs, warps * wcap * 32 * sizeof(uint2));
@@ -620,7 +645,7 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
                             h->cub_tmp.p, ds.res.p, qs.prof.p, qs.offsets.p, qs.prof_off.p};
     std::memcpy(key.ptrs, ptrs, sizeof(ptrs));
     key.qrow = qs.qrow.p;
-    key.matrix = sch.d_matrix.p;
+    key.matrix = pairs ? sch.d_pairs.p : sch.d_matrix.p;  // which anti-diagonal kernel, too
     const void* extra = qs.prof_mpad.p;  // (pointer identity of the last profile table)
     cudaGraphExec_t exec = nullptr;
     for (auto& e : h->graphs)
@@ -674,7 +699,7 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
             chk(launch_band_fast(pass == 0 ? grid0 : grid8, s, a));
         }
         chk(launch_band_wave((unsigned)h->sm_count, s,
-                             wave_args(sch, ds, d_jobs, order, counts, d_scores, h->list.as<uint32_t>())));
+                             wave_args(sch, ds, d_jobs, order, counts, d_scores, h->list.as<uint32_t>(), pairs)));
         GenericArgs g;
         g.res = ds.res.as<uint8_t>();
         g.prof = qs.prof.as<int16_t>();
@@ -900,6 +925,12 @@ static int set_scheme(saber_gpu* h, Scheme& sch, const int32_t* matrix, int32_t 
     sch.has = false;
     CUALLOC(h, sch.d_matrix, 576 * 4);
     CU(h, cudaMemcpyAsync(sch.d_matrix.p, sch.matrix, 576 * 4, cudaMemcpyHostToDevice, h->stream));
+    const auto mm = std::minmax_element(sch.matrix, sch.matrix + 576);
+    sch.pairs8 = *mm.first + go >= -127 && *mm.second + go <= 127;
+    if (sch.pairs8) {
+        CUALLOC(h, sch.d_pairs, kWavePairBytes + 64);
+        sch.pairs_built = false;
+    }
     CU(h, cudaStreamSynchronize(h->stream));
     sch.has = true;
     return SABER_OK;
