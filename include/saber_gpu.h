@@ -61,15 +61,15 @@ typedef struct {
 typedef struct {
     uint64_t jobs;            /* jobs scored */
     uint64_t banded_cells;    /* in-band cells, counted as banded.rs:123-131 */
-    uint64_t fast_cells;      /* the part of banded_cells in jobs of the packed int16 kernel */
-    uint64_t fast_jobs;       /* jobs taken by the packed int16 kernel */
-    uint64_t generic_jobs;    /* jobs scored directly in int32 (narrow bands) */
+    uint64_t fast_cells;      /* the part of banded_cells in jobs of the packed int16 kernels */
+    uint64_t fast_jobs;       /* jobs taken by the packed int16 kernels (strips and anti-diagonals) */
+    uint64_t generic_jobs;    /* the other jobs: narrow bands, and bands scored directly in int32 */
     uint64_t i16_rescored;    /* int16 results at the overflow limit, rescored in int32 */
     uint64_t empty_jobs;      /* empty band / window / query: score 0 */
     uint64_t kernel_launches; /* this library's own kernels launched by the call */
     uint64_t library_launches;/* CUB sort / scan / select kernels launched by the call */
     double t_prep_ms;         /* device time: classify, sort, pairing (CUDA events) */
-    double t_fast_ms;         /* device time of the packed int16 kernel */
+    double t_fast_ms;         /* device time of the packed int16 kernels */
     double t_generic_ms;      /* device time of the int32 kernel */
     uint64_t prof8;           /* 1: the packed kernel read the int8 copy of the query profiles (every
                                  S + bias + go of the query set in [-127, 127]), 0: the int16 profiles */
@@ -483,13 +483,13 @@ uint32_t saber_gpu_get_pair_steps(saber_gpu* h);
 
 /* Tuning: a job whose sweep in one lane would take more than `steps` column
  * steps (strips x the steps of a strip, window columns only) is scored by
- * the int32 kernel instead, which pipelines a long job's strips over a
- * warp's lanes, so one long job does not set the launch's length.
- * 0xFFFFFFFF keeps every job on the int16 lanes; 0xFFFFFFFE (the default)
- * picks, per call, the power of two at or above four times the sweep steps
- * of one int16 lane if the batch's in-band cells were spread evenly over
- * the lanes (32 cells per step), and at least 2048.  Results do not depend
- * on it.
+ * the anti-diagonal int16 kernel instead, which spreads a job over 8 to 128
+ * lanes, so one long job does not set the launch's length.
+ * 0 sends every job there; 0xFFFFFFFF keeps every job on the one-lane
+ * strips; 0xFFFFFFFE (the default) picks, per call, the power of two at or
+ * above 1.25 times the sweep steps of one lane if the batch's in-band cells
+ * were spread evenly over the lanes (32 cells per step), and at least 2048,
+ * or 0 when that is under 1,650 steps.  Results do not depend on it.
  * No reference counterpart. */
 int saber_gpu_set_long_steps(saber_gpu* h, uint32_t steps);
 uint32_t saber_gpu_get_long_steps(saber_gpu* h);

@@ -11,11 +11,11 @@ never results:
   critical path) instead of half a lane; the threshold is the bin edge
   between the two classes;
 * the long-job bin edge (`Device.long_steps`): a job whose one-lane sweep is
-  longer than this goes to the warp-per-job int32 kernel's pipelined strips
-  (a whole warp on one job) instead of a lane of the int16 kernel; the
-  default picks it per call from the batch's in-band cells per lane (the
-  power of two at or above four times a lane's even share of the sweep
-  steps, at least 2048).
+  longer than this goes to the anti-diagonal int16 kernel (8 to 128 lanes on
+  one job) instead of a lane of the strip kernel; the default picks it per
+  call from the batch's in-band cells per lane (the power of two at or above
+  1.25 times a lane's even share of the sweep steps, at least 2048; a batch
+  of less than 1,650 steps per lane goes there as a whole).
 
 `autotune_scoring` times settings on the caller's own batch (the
 device-resident entry point, same stream) by coordinate descent: starting
