@@ -172,8 +172,8 @@ struct saber_gpu {
     // learned triage: installed model, per-call feature buffers, collection
     saber::DevBuf tr_model, tr_wb, tr_sfeat, tr_qfeat, tr_reg, tr_rstat, tr_rq, tr_rrank, tr_qinfo, tr_X, tr_logit, tr_err;
     saber::TriageScratch tg;
-    bool tr_on = false, tr_sfeat_ok = false;
-    uint64_t tr_sfeat_key = 0;
+    bool tr_on = false;
+    bool tr_sfeat_ok = false;  // tr_sfeat holds the loaded database's features
     float tr_threshold = 0.f;
     bool tr_collect = false;
     std::vector<float> tr_rows, tr_logits;

@@ -907,7 +907,9 @@ static int load_db(saber_gpu* h, Dataset& ds, const uint8_t* residues, uint64_t 
     ds.max_len = max_len;
     ds.has_db = true;
     if (&ds == &h->main) {
+        // what is kept of the database loaded before (its buffers may stay where they are)
         h->sc_key = 0;
+        h->tr_sfeat_ok = false;
         h->has_db_mask = false;
     }
     return SABER_OK;

@@ -1005,14 +1005,13 @@ int triage_region_features(saber_gpu* h, const saber_region* d_reg, const uint4*
     const Dataset& ds = h->main;
     const QuerySet& qs = ds.qs;
     cudaStream_t s = h->stream;
-    if (!h->tr_sfeat_ok || h->tr_sfeat_key != (uint64_t)(uintptr_t)ds.res.p + ds.n_res) {
+    if (!h->tr_sfeat_ok) {
         CUALLOC(h, h->tr_sfeat, std::max<uint64_t>(ds.nsub, 1) * sizeof(float4));
         if (ds.nsub)
             k_seq_feats<<<(unsigned)std::min<uint64_t>((ds.nsub + 7) / 8, 65535u * 8), 256, 0, s>>>(
                 ds.res.as<uint8_t>(), ds.soff.as<uint64_t>(), ds.nsub, h->tr_sfeat.as<float4>());
         CU(h, cudaGetLastError());
         h->tr_sfeat_ok = true;
-        h->tr_sfeat_key = (uint64_t)(uintptr_t)ds.res.p + ds.n_res;
     }
     CUALLOC(h, h->tr_qfeat, std::max<uint64_t>(qs.nq, 1) * sizeof(float4));
     if (qs.nq)
