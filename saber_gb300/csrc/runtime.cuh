@@ -41,6 +41,7 @@ struct DevBuf {
         size_t want = bytes < 256 ? 256 : bytes;
         cudaError_t e = cudaMalloc(&p, want);
         if (e == cudaSuccess) cap = want;
+        else p = nullptr, cudaGetLastError();  // the caller has the error: the next launch's check must not find it
         return e;
     }
     template <class T>
@@ -67,6 +68,7 @@ struct HostBuf {
         const size_t want = std::max<size_t>(bytes + bytes / 4, 4096);
         cudaError_t e = cudaHostAlloc(&p, want, cudaHostAllocDefault);
         if (e == cudaSuccess) cap = want;
+        else p = nullptr, cudaGetLastError();
         return e;
     }
     template <class T>
