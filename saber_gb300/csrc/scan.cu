@@ -1665,6 +1665,7 @@ int scan_build_db(saber_gpu* h, const saber_scan_params* p) {
     const uint64_t N = ds.n_res;
     AlphaMap am;
     memcpy(am.m, p->alpha_map, 24);
+    h->sc_key = 0;  // a build that fails on the way must not be taken for the one before it
     {
         CombTab ct;
         h->sc_comb = comb_table(p, ct.t);

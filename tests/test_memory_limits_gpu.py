@@ -6,9 +6,10 @@ import numpy as np
 import pytest
 
 from oracle import oracle as orc
-from saber_gb300 import synth
-from saber_gb300.gpu import Device, SaberGpuError
+from saber_gb300 import presets, synth
+from saber_gb300.gpu import Device, SaberGpuError, scan_params
 from saber_gb300.scoring import matrix
+from tests.test_scan_gpu import _check
 
 pytestmark = pytest.mark.gpu
 B62 = matrix("BLOSUM62")
@@ -43,3 +44,28 @@ def test_a_refused_allocation_does_not_fail_the_next_call():
         got, _ = dev.score_band_jobs(jobs)
     want, _ = orc.score_band_jobs(ss.codes, qs.codes, qs.offsets, None, jobs, B62, 11, 1, threads=4)
     assert np.array_equal(got, want)
+
+
+def test_scan_after_parameters_whose_tables_did_not_fit():
+    """The database state of the parameters before is built anew, not taken
+    from what the refused call left of it."""
+    qs, ss, _ = synth.protein_db(7, 12, 800)
+    amap, asz = presets.alphabet_map()
+    full, fsz = presets.full_alphabet()
+    n = int(ss.codes.size)
+    kw = dict(min_ids=27, exact_weight=2, db_length=n)
+    gp, op = scan_params(amap, asz, presets.DS16, **kw), orc.make_scan_params(amap, asz, presets.DS16, **kw)
+    # 20^7 codes: 5 GB of counts
+    wide = scan_params(full, fsz, ["1111111"], min_ids=12, exact_weight=1, db_length=n)
+    with Device(0) as dev:
+        dev.set_scheme(B62, 11, 1)
+        dev.load_db(ss.codes, ss.offsets)
+        dev.load_queries(qs.codes, qs.offsets, None)
+        dev.scan(gp, None, None)
+        with memory_left(3 * GIB):
+            with pytest.raises(SaberGpuError, match="allocation"):
+                dev.scan(wide, None, None)
+        got, gst = dev.scan(gp, None, None)
+    want, ost = orc.scan_regions(ss.codes, ss.offsets, None, qs.codes, qs.offsets, None, None, None, B62, op)
+    assert want.size > 0
+    _check(got, gst, want, ost)
