@@ -484,12 +484,15 @@ uint32_t saber_gpu_get_pair_steps(saber_gpu* h);
 /* Tuning: a job whose sweep in one lane would take more than `steps` column
  * steps (strips x the steps of a strip, window columns only) is scored by
  * the anti-diagonal int16 kernel instead, which spreads a job over 8 to 128
- * lanes, so one long job does not set the launch's length.
+ * lanes (bands wider than 1,024: the int32 kernel, a warp per job), so one
+ * long job does not set the launch's length.
  * 0 sends every job there; 0xFFFFFFFF keeps every job on the one-lane
  * strips; 0xFFFFFFFE (the default) picks, per call, the power of two at or
  * above 1.25 times the sweep steps of one lane if the batch's in-band cells
  * were spread evenly over the lanes (32 cells per step), and at least 2048,
- * or 0 when that is under 1,650 steps.  Results do not depend on it.
+ * or 0 when that is under 1,650 steps; a batch whose bands are wide for their
+ * queries' lengths, or mostly wider than 1,024, takes 4 times those steps, and
+ * at least 2048.  Results do not depend on it.
  * No reference counterpart. */
 int saber_gpu_set_long_steps(saber_gpu* h, uint32_t steps);
 uint32_t saber_gpu_get_long_steps(saber_gpu* h);

@@ -114,6 +114,13 @@ constexpr int kWaveRowBytes = 1250;  // row pitch of its score tables (25 x 25 p
 __host__ __device__ inline int wave_class(int64_t w) {
     return w > 512 ? 0 : w > 256 ? 1 : w > 128 ? 2 : w > 64 ? 3 : w > 36 ? 4 : w > 32 ? 5 : 6;
 }
+// Band indices that a job of the class is swept over.
+__host__ __device__ inline uint32_t wave_slots(int c) { return c < 5 ? 1024u >> c : c == 5 ? 36u : 32u; }
+// Longest one-lane sweeps (column steps) that stay on the strip kernel: of bands
+// that the anti-diagonal kernel takes, and of wider ones.
+struct LongSteps {
+    uint32_t narrow, wide;
+};
 struct WaveArgs {
     const uint8_t* res;
     const uint32_t* qrow;    // per batch position: table row offset | bias << 16

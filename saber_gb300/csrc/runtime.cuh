@@ -106,7 +106,9 @@ struct Dataset {
 struct GraphKey {
     uint64_t npad, wcap, n_res;
     int32_t rows, go, ge;
-    uint32_t pair_steps, nq, long_steps;
+    uint32_t pair_steps, nq;
+    LongSteps longest;
+    bool strips;
     const void* ptrs[16];
     const void* prof8;
     const void *qrow, *matrix;
@@ -149,7 +151,7 @@ struct saber_gpu {
     // captured scoring graphs (saber_gpu_score_band_jobs with graphs on)
     bool use_graphs = true;
     uint64_t graph_captures = 0;
-    saber::DevBuf g_nreal, g_wmax;
+    saber::DevBuf g_nreal, g_load;
     std::vector<std::pair<saber::GraphKey, saber::GraphEntry>> graphs;
     // the handle's scheme and dataset (set_scheme / load_db / load_queries)
     saber::Scheme scheme;

@@ -84,28 +84,97 @@ __global__ void k_profile(const uint8_t* __restrict__ codes, const uint64_t* __r
     }
 }
 
-// Widest clipped band (out[0]) and in-band cell total (out[1]) of the jobs
-// that reference a loaded query.
-__global__ void k_job_wmax(const saber_band_job* __restrict__ jobs, uint64_t njobs,
-                           const uint64_t* __restrict__ qoffs, uint32_t nq, unsigned long long* __restrict__ out) {
-    unsigned long long wm = 0, cells = 0;
+// A band's sweep on the strip kernel: rows of a strip (R, or 8 where R = 16 is
+// wider than the band), strips that hold window rows, and the column steps of
+// one lane.  Sweeps longer than pair_steps go to paired strips (one job per lane,
+// 2 R rows).  A strip's steps are the band's, or the window's when the band is
+// wider (the kernels sweep window columns only).  For w >= kStripRowsMin.
+struct LaneSweep {
+    int rows;
+    bool pair;
+    int64_t strips;
+    uint64_t steps;
+};
+__device__ __forceinline__ LaneSweep lane_sweep(int64_t n, int64_t w, int64_t first, int64_t last, int R,
+                                                uint32_t pair_steps) {
+    LaneSweep s;
+    int sh = w >= R && R == kStripRows ? 4 : 3;
+    s.rows = 1 << sh;
+    s.strips = (last >> sh) - (first >> sh) + 1;
+    s.pair = w >= R && R == kStripRows && w >= 2 * R + 1 && (uint64_t)s.strips * (uint64_t)(w + R - 1) > pair_steps;
+    if (s.pair) {
+        sh++;
+        s.rows = 2 * R;
+        s.strips = (last >> sh) - (first >> sh) + 1;
+    }
+    s.steps = (uint64_t)s.strips * (uint64_t)(min(w - 1, n) + s.rows);
+    return s;
+}
+static_assert(kStripRows == 16 && kStripRowsMin == 8, "strips of 8, 16 and 32 rows");
+
+// What a batch's jobs that reference a loaded query come to (long_steps_for).
+struct JobLoad {
+    unsigned long long wmax;        // widest clipped band
+    unsigned long long sweep;       // longest lane sweep of a band of 8 .. kWaveMaxWidth
+    unsigned long long wide_sweep;  // and of a wider one
+    unsigned long long cells;       // in-band cells
+    unsigned long long wave;        // cells that the anti-diagonal kernel steps through for the bands of 8 .. kWaveMaxWidth
+    unsigned long long wide;        // in-band cells of the wider ones
+};
+
+// Sum over a warp, 22 bits at a time.
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+    constexpr unsigned kLow = (1u << 22) - 1u;
+    const unsigned long long a = __reduce_add_sync(0xffffffffu, (unsigned)v & kLow);
+    const unsigned long long b = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 22) & kLow);
+    const unsigned long long c = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 44));
+    return a + (b << 22) + (c << 44);
+}
+
+__global__ void k_job_load(const saber_band_job* __restrict__ jobs, uint64_t njobs,
+                           const uint64_t* __restrict__ qoffs, uint32_t nq, int R, uint32_t pair_steps,
+                           unsigned long long* __restrict__ out) {
+    uint32_t mx[3] = {};
+    unsigned long long sum[3] = {};
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < njobs; t += (uint64_t)gridDim.x * blockDim.x) {
         const saber_band_job j = jobs[t];
         if (j.query >= nq) continue;
-        const int64_t m = (int64_t)(qoffs[j.query + 1] - qoffs[j.query]);
+        const int64_t m = (int64_t)(qoffs[j.query + 1] - qoffs[j.query]), n = j.win_len;
         int64_t lo = j.band_lo, hi = j.band_hi;
-        const int64_t w = clip_band(m, j.win_len, lo, hi);
-        wm = max(wm, (unsigned long long)w);
-        if (w > 0) cells += band_cells(m, j.win_len, lo, hi);
+        const int64_t w = clip_band(m, n, lo, hi);
+        if (w <= 0) continue;
+        mx[0] = max(mx[0], (uint32_t)min(w, (int64_t)UINT32_MAX));
+        const uint64_t jc = band_cells(m, n, lo, hi);
+        sum[0] += jc;
+        if (w < kStripRowsMin || m >= (1 << 28) || n >= (1 << 28)) continue;
+        const LaneSweep ls = lane_sweep(n, w, hi < 0 ? -hi : 0, min(n - 1 - lo, m - 1), R, pair_steps);
+        const uint32_t steps = (uint32_t)min(ls.steps, (uint64_t)UINT32_MAX);
+        if (w > kWaveMaxWidth) {
+            mx[2] = max(mx[2], steps);
+            sum[2] += jc;
+        } else {
+            int s0, nit;
+            wv_span((int)m, (int)n, (int)lo, (int)w, s0, nit);
+            mx[1] = max(mx[1], steps);
+            sum[1] += (uint64_t)nit * wave_slots(wave_class(w));
+        }
     }
+    __shared__ unsigned long long b[6];
+    if (threadIdx.x < 6) b[threadIdx.x] = 0;
+    __syncthreads();
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        wm = max(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-        cells += __shfl_xor_sync(0xffffffffu, cells, o);
+    for (int k = 0; k < 3; k++) {
+        const uint32_t most = __reduce_max_sync(0xffffffffu, mx[k]);
+        const unsigned long long total = warp_sum(sum[k]);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMax(&b[k], (unsigned long long)most);
+            atomicAdd(&b[3 + k], total);
+        }
     }
-    if ((threadIdx.x & 31) == 0) {
-        if (wm) atomicMax(out, wm);
-        if (cells) atomicAdd(out + 1, cells);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        atomicMax(out + threadIdx.x, b[threadIdx.x]);
+        atomicAdd(out + 3 + threadIdx.x, b[3 + threadIdx.x]);
     }
 }
 
@@ -133,7 +202,7 @@ constexpr int kCounts = 32;  // words of the counts buffer
 // consecutive jobs of a warp task share their loop counts and widths; within
 // class 0 the paired jobs (bit 61; their strips counted in 2R rows) sort last.
 __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njobs, const uint32_t* __restrict__ n_real,
-                           int R, uint32_t pair_steps, uint32_t long_steps, const uint64_t* __restrict__ qoffs,
+                           int R, uint32_t pair_steps, LongSteps longest, const uint64_t* __restrict__ qoffs,
                            uint32_t nq, uint64_t n_res,
                            uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
                            int32_t* __restrict__ scores, uint32_t* __restrict__ counts,
@@ -169,29 +238,15 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
         const int64_t first = hi < 0 ? -hi : 0;
         int64_t last = (int64_t)j.win_len - 1 - lo;
         if (last > m - 1) last = m - 1;
+        // narrow bands and sizes that a strip key cannot hold leave the strips,
+        // and so does a sweep of more than `longest` steps
+        LaneSweep ls{};
         int cls = 2;
-        int rows = R;
-        if (w >= R) cls = 0;
-        else if (R > kStripRowsMin && w >= kStripRowsMin) {
-            cls = 1;
-            rows = kStripRowsMin;
-        }
-        int64_t ns = last / rows - first / rows + 1;
-        // long R-row sweeps go to paired strips (one job per lane, 2R rows)
-        uint64_t pair = 0;
-        if (cls == 0 && R == kStripRows && w >= 2 * R + 1 && (uint64_t)ns * (uint64_t)(w + R - 1) > pair_steps) {
-            pair = 1;
-            ns = last / (2 * R) - first / (2 * R) + 1;
-        }
-        if (cls != 2 && (w >= (1 << 16) || ns >= (1 << 13))) cls = 2;
-        // a sweep longer than long_steps column steps in one lane goes to the
-        // anti-diagonal kernel
-        if (cls != 2) {
-            // the sweep's steps per strip: the band's, or the window's when
-            // the band is wider (the kernels sweep window columns only)
-            const int64_t srw = pair ? 2 * R : rows;
-            const int64_t span = w + srw - 1 < (int64_t)j.win_len + srw ? w + srw - 1 : (int64_t)j.win_len + srw;
-            if ((uint64_t)ns * (uint64_t)span > long_steps) cls = 2;
+        if (w >= kStripRowsMin) {
+            ls = lane_sweep(j.win_len, w, first, last, R, pair_steps);
+            if (w < (1 << 16) && ls.strips < (1 << 13) &&
+                ls.steps <= (w <= kWaveMaxWidth ? longest.narrow : longest.wide))
+                cls = w >= R ? 0 : 1;
         }
         if (cls == 2) {
             const uint64_t sz = jc >> 4 < 0x7FFFFFFull ? jc >> 4 : 0x7FFFFFFull;
@@ -212,14 +267,14 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
             // within (strips, width): jobs ordered by the first strip's
             // window geometry (steps before column -1, steps to the last
             // column), so that a warp's jobs share the step range it sweeps
-            const int64_t srows = pair ? 2 * R : rows;
-            const int64_t col0 = lo + (first / srows) * srows;
+            const int64_t col0 = lo + first / ls.rows * ls.rows;
             const int64_t left = col0 < -1 ? -col0 - 1 : 0;
-            const int64_t right = (int64_t)j.win_len - (pair ? 0 : 1) - col0;
+            const int64_t right = (int64_t)j.win_len - (ls.pair ? 0 : 1) - col0;
             const uint64_t low = ((uint64_t)(left < 65535 ? left : 65535) << 16) |
                                  (uint64_t)(right < 0 ? 0 : (right < 65535 ? right : 65535));
-            keys[t] = ((uint64_t)cls << 62) | (pair << 61) | ((uint64_t)ns << 48) | ((uint64_t)w << 32) | low;
-            cp += (uint32_t)pair;
+            keys[t] = ((uint64_t)cls << 62) | ((uint64_t)ls.pair << 61) | ((uint64_t)ls.strips << 48) | ((uint64_t)w << 32) |
+                      low;
+            cp += (uint32_t)ls.pair;
             fcells += jc;
             if (cls == 0) {
                 c0++;
@@ -296,7 +351,6 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
     }
 }
 
-
 // ---------------------------------------------------------------------------
 // the scoring pipeline (device-resident jobs and scores)
 // ---------------------------------------------------------------------------
@@ -340,30 +394,59 @@ static cudaError_t ensure_pairs(saber_gpu* h, const Scheme& sch) {
     sch.pairs_built = e == cudaSuccess;
     return e;
 }
-static uint32_t long_steps_for(const saber_gpu* h, uint64_t cells) {
-    if (h->long_steps != kLongStepsAuto) return h->long_steps;
-    const uint64_t load = steps_per_lane(h, cells);
-    if (load < kLoadSmall) return 0;
-    uint64_t t = kLongStepsSmall;
-    while (t < load + load / 4 && t < (1ull << 30)) t <<= 1;
-    return (uint32_t)t;
+// Those are bands of the usual proportions.  The anti-diagonal kernel sweeps 2
+// rows + w steps over a width rounded up to its classes, so bands that are wide
+// for their queries' lengths cost it many times their cells, and bands wider than
+// it takes go to the int32 kernel.  Such a batch keeps sweeps of up to four times
+// the even share on the strips, where the other kernel's work, spread evenly,
+// takes longer than the batch's longest lane sweep (a lane's step is about 0.6 us
+// on its own, 32 cells a lane about 0.7 us of the anti-diagonal kernel).  One
+// GB300, a call by the anti-diagonal kernel / the strips:
+//   30 rows x 401,   50 k jobs (share 2,370, sweep 832)     1.65 / 0.77 ms
+//                   300 k      (14,200)                     9.16 / 1.45
+//   60 x 257,        20 k      (773, 1,088)                 0.49 / 0.72
+//                    50 k      (1,932)                      1.04 / 0.73
+//   120 x 161,       50 k      (1,025, 1,408)               0.87 / 1.20
+//                   100 k      (2,050)                      1.61 / 1.22
+//   500 x 257,       20 k      (2,582, 4,608)               1.64 / 1.67
+//                    50 k      (6,456)                      3.97 / 2.82
+// and by the int32 kernel / the strips, 1,201-wide bands (a cell of the int32
+// kernel as kWideCell ones):
+//   30 rows,         200 jobs  (139, 1,232)                 0.32 / 0.49 ms
+//                  5,000       (3,470)                      1.20 / 0.81
+//                 50,000       (34,700)                     8.8 / 1.02
+//   300 rows,     30,000       (208,000, 12,320)            20.7 / 7.9
+constexpr uint64_t kWideCell = 48;
+static LongSteps long_steps_for(const saber_gpu* h, const JobLoad& l) {
+    if (h->long_steps != kLongStepsAuto) return {h->long_steps, h->long_steps};
+    const uint64_t load = steps_per_lane(h, l.cells);
+    auto power = [](uint64_t least) {
+        uint64_t t = kLongStepsSmall;
+        while (t < least && t < (1ull << 30)) t <<= 1;
+        return t;
+    };
+    const uint64_t most = power(4 * load), usual = load < kLoadSmall ? 0 : power(load + load / 4);
+    const bool narrow = steps_per_lane(h, l.wave) > std::min<uint64_t>(l.sweep, most);
+    const bool wide = steps_per_lane(h, l.wide * kWideCell) > std::min<uint64_t>(l.wide_sweep, most);
+    return {(uint32_t)(narrow ? most : usual), (uint32_t)(wide ? most : usual)};
+}
+// The strip classes can hold jobs.
+static bool has_strips(const LongSteps& t, const JobLoad& l) {
+    return t.narrow != 0 || (t.wide != 0 && l.wide != 0);
 }
 
-// In-band cells of the device jobs (for the automatic long-job threshold):
-// one reduction and an 8-byte read-back, only in the automatic mode.
-static int jobs_cells(saber_gpu* h, const QuerySet& qs, const saber_band_job* d_jobs, uint64_t njobs,
-                      uint64_t* cells) {
-    *cells = 0;
-    if (h->long_steps != kLongStepsAuto || !qs.has || njobs == 0) return SABER_OK;
-    CUALLOC(h, h->g_wmax, 16);
-    CU(h, cudaMemsetAsync(h->g_wmax.p, 0, 16, h->stream));
-    k_job_wmax<<<nblocks(njobs, 256, h->sm_count * 8), 256, 0, h->stream>>>(
-        d_jobs, njobs, qs.offsets.as<uint64_t>(), qs.nq, h->g_wmax.as<unsigned long long>());
+// One reduction over the device jobs and a read-back of 48 bytes.
+static int job_load(saber_gpu* h, const QuerySet& qs, const saber_band_job* d_jobs, uint64_t njobs, JobLoad* l) {
+    *l = JobLoad{};
+    if (!qs.has || njobs == 0) return SABER_OK;
+    CUALLOC(h, h->g_load, sizeof(JobLoad));
+    CU(h, cudaMemsetAsync(h->g_load.p, 0, sizeof(JobLoad), h->stream));
+    k_job_load<<<nblocks(njobs, 256, h->sm_count * 8), 256, 0, h->stream>>>(
+        d_jobs, njobs, qs.offsets.as<uint64_t>(), qs.nq, h->strip_rows, h->pair_steps,
+        h->g_load.as<unsigned long long>());
     CU(h, cudaGetLastError());
-    unsigned long long r[2] = {0, 0};
-    CU(h, cudaMemcpyAsync(r, h->g_wmax.p, 16, cudaMemcpyDeviceToHost, h->stream));
+    CU(h, cudaMemcpyAsync(l, h->g_load.p, sizeof(JobLoad), cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
-    *cells = r[1];
     return SABER_OK;
 }
 
@@ -389,10 +472,9 @@ static WaveArgs wave_args(const Scheme& sch, const Dataset& ds, const saber_band
     return a;
 }
 
-// First key bit that the sort looks at.  Without strip classes (long_steps 0:
-// every job goes to the anti-diagonal kernel) only the class and the size in
-// steps of 512 cells matter: four digit passes instead of eight.
-static int sort_from(uint32_t long_steps) { return long_steps == 0 ? 36 : 0; }
+// First key bit that the sort looks at.  Without strip classes only the class
+// and the size in steps of 512 cells matter: four digit passes instead of eight.
+static int sort_from(bool strips) { return strips ? 0 : 36; }
 
 static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, const saber_band_job* d_jobs,
                           uint64_t njobs, int32_t* d_scores, saber_score_stats* st) {
@@ -421,12 +503,14 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     CU(h, cudaMemsetAsync(stats, 0, 8 * 8, s));
 
     const QuerySet& qs = ds.qs;
-    uint64_t job_cells = 0;
-    int rc0 = jobs_cells(h, qs, d_jobs, njobs, &job_cells);
-    if (rc0 != SABER_OK) return rc0;
-    const uint32_t long_steps = long_steps_for(h, job_cells);
-    const int key_from = sort_from(long_steps);
-    const bool pairs = use_pairs(h, sch, job_cells);
+    JobLoad jl{};
+    if (h->long_steps == kLongStepsAuto) {
+        int rc0 = job_load(h, qs, d_jobs, njobs, &jl);
+        if (rc0 != SABER_OK) return rc0;
+    }
+    const LongSteps longest = long_steps_for(h, jl);
+    const int key_from = sort_from(has_strips(longest, jl));
+    const bool pairs = use_pairs(h, sch, jl.cells);
     if (pairs) CU(h, ensure_pairs(h, sch));
     cudaEvent_t ev[4];
     for (int i = 0; i < 4; i++) CU(h, cudaEventCreate(&ev[i]));
@@ -438,7 +522,7 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     } evg{ev};
     CU(h, cudaEventRecord(ev[0], s));
     k_classify<<<nblocks(njobs, 256, h->sm_count * 8), 256, 0, s>>>(
-        d_jobs, njobs, nullptr, h->strip_rows, h->pair_steps, long_steps, qs.offsets.as<uint64_t>(), qs.nq,
+        d_jobs, njobs, nullptr, h->strip_rows, h->pair_steps, longest, qs.offsets.as<uint64_t>(), qs.nq,
         ds.n_res,
         h->keys_in.as<uint64_t>(),
         h->vals_in.as<uint32_t>(), d_scores, counts, stats);
@@ -593,13 +677,13 @@ static uint64_t pad_jobs(uint64_t n) { return n <= 1024 ? 1024 : pow2_at_least(n
 // padded entries sorted last as empty jobs), scratch sized for a power-of-two
 // job count and band width, captured once per (size bucket, buffers,
 // settings) and replayed.  Jobs and scores live in the handle's buffers.
-static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& ds, uint64_t njobs, uint64_t wmax,
-                                uint64_t job_cells, saber_score_stats* st) {
+static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& ds, uint64_t njobs, const JobLoad& jl,
+                                saber_score_stats* st) {
     if (!sch.has) return fail(h, SABER_ERR_STATE, "no scoring scheme set");
     if (!ds.has_db) return fail(h, SABER_ERR_STATE, "no database loaded");
     if (!ds.qs.has) return fail(h, SABER_ERR_STATE, "no query set loaded");
     const uint64_t npad = pad_jobs(njobs);
-    const uint64_t wcap = pow2_at_least(wmax + 1, 64);
+    const uint64_t wcap = pow2_at_least(jl.wmax + 1, 64);
     if (npad >= (1ull << 31)) return fail(h, SABER_ERR_ARG, "too many jobs in one call");
     cudaStream_t s = h->stream;
     const QuerySet& qs = ds.qs;
@@ -614,11 +698,11 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     const int rows0 = h->strip_rows;
     const unsigned grid0 = (unsigned)(h->sm_count * band_fast_blocks_per_sm(rows0, qs.p8));
     const unsigned grid8 = (unsigned)(h->sm_count * band_fast_blocks_per_sm(kStripRowsMin, qs.p8));
-    const uint32_t long_steps = long_steps_for(h, job_cells);
-    const int key_from = sort_from(long_steps);
-    const bool pairs = use_pairs(h, sch, job_cells);
+    const LongSteps longest = long_steps_for(h, jl);
+    const bool strips = has_strips(longest, jl);
+    const int key_from = sort_from(strips);
+    const bool pairs = use_pairs(h, sch, jl.cells);
     if (pairs) CU(h, ensure_pairs(h, sch));
-    const bool strips = long_steps != 0;  // the strip classes can hold jobs
     const uint64_t warps = (uint64_t)std::max(grid0, grid8) * 256 / 32;
     if (strips) CUALLOC(h, h->bufs, warps * wcap * 32 * sizeof(uint2));
     const unsigned gT = 128, gGrid = (unsigned)(h->sm_count * 4);
@@ -636,7 +720,8 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
     key.go = sch.go;
     key.ge = sch.ge;
     key.pair_steps = h->pair_steps;
-    key.long_steps = long_steps;
+    key.longest = longest;
+    key.strips = strips;
     key.n_res = ds.n_res;  // scalar kernel parameters baked into the graph
     key.nq = qs.nq;
     key.prof8 = qs.p8 ? qs.prof8.p : nullptr;  // which packed kernel the graph launches
@@ -663,7 +748,7 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
         chk(cudaMemsetAsync(counts, 0, kCounts * 4, s));
         chk(cudaMemsetAsync(stats, 0, 8 * 8, s));
         k_classify<<<nblocks(npad, 256, h->sm_count * 8), 256, 0, s>>>(
-            d_jobs, npad, h->g_nreal.as<uint32_t>(), rows0, h->pair_steps, long_steps,
+            d_jobs, npad, h->g_nreal.as<uint32_t>(), rows0, h->pair_steps, longest,
             qs.offsets.as<uint64_t>(), qs.nq,
             ds.n_res, h->keys_in.as<uint64_t>(), h->vals_in.as<uint32_t>(), d_scores, counts, stats);
         chk(cudaGetLastError());
@@ -782,21 +867,12 @@ int score_resident_jobs(saber_gpu* h, uint64_t njobs, saber_score_stats* st) {
     if (!h->use_graphs)
         return score_pipeline(h, h->scheme, h->main, h->jobs_dev.as<saber_band_job>(), njobs,
                               h->scores_dev.as<int32_t>(), st);
-    // the widest clipped band sizes the graph's scratch and the cell total sets
-    // the automatic long-job threshold: one reduction on the device, 16 bytes
-    // read back
-    const QuerySet& qs = h->main.qs;
-    CUALLOC(h, h->g_wmax, 16);
-    CU(h, cudaMemsetAsync(h->g_wmax.p, 0, 16, h->stream));
-    if (qs.has)
-        k_job_wmax<<<nblocks(njobs, 256, h->sm_count * 8), 256, 0, h->stream>>>(
-            h->jobs_dev.as<saber_band_job>(), njobs, qs.offsets.as<uint64_t>(), qs.nq,
-            h->g_wmax.as<unsigned long long>());
-    CU(h, cudaGetLastError());
-    unsigned long long r[2] = {0, 0};
-    CU(h, cudaMemcpyAsync(r, h->g_wmax.p, 16, cudaMemcpyDeviceToHost, h->stream));
-    CU(h, cudaStreamSynchronize(h->stream));
-    return score_pipeline_graph(h, h->scheme, h->main, njobs, r[0], r[1], st);
+    // the widest clipped band sizes the graph's scratch, the sums set the
+    // automatic long-job thresholds
+    JobLoad jl;
+    int rc = job_load(h, h->main.qs, h->jobs_dev.as<saber_band_job>(), njobs, &jl);
+    if (rc != SABER_OK) return rc;
+    return score_pipeline_graph(h, h->scheme, h->main, njobs, jl, st);
 }
 
 static int build_profiles(saber_gpu* h, const Scheme& sch, QuerySet& q) {
