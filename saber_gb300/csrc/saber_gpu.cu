@@ -1123,8 +1123,18 @@ using RunPools = std::vector<std::vector<uint32_t>>;
 // 6.6 GB of direction bytes) fits one launch.
 constexpr uint64_t kDirPoolBudget = 8ull << 30;
 constexpr uint64_t kAlignSlabBudget = 512ull << 20;
-// Widest band of the anti-diagonal kernel: 32 lanes x 16 band indices.
+// The anti-diagonal kernel's jobs: bands of at most 32 lanes x 16 band indices,
+// on queries that are not too short for them.  It sweeps rows + w / 2 pairs of
+// steps where the row kernel takes a scan a row, so a few rows on a wide band are
+// the row kernel's.  Calls of 5,000 jobs (rows x clipped width) on one GB300, row
+// kernel / this one: 5 x 21 0.236 / 0.274 ms, 5 x 133 0.266 / 0.325; 8 x 73 0.266 /
+// 0.278, x 136 0.281 / 0.314, x 263 0.316 / 0.482; 12 x 77 0.287 / 0.275, x 211
+// 0.338 / 0.349, x 267 0.367 / 0.498; 16 x 215 0.373 / 0.365, x 271 0.403 / 0.495;
+// 20 x 219 0.402 / 0.373, x 275 0.448 / 0.501; 25 x 280 0.511 / 0.514; 300 x 129
+// 2.28 / 0.55.
 constexpr int64_t kAlignWaveWidth = 512;
+constexpr int64_t kAlignWaveRows = 8;      // at least
+constexpr int64_t kAlignWaveAspect = 16;   // band indices a row, at most
 
 static int align_batch(saber_gpu* h, const Scheme& sch, const Dataset& ds, const std::vector<AlignHostReq>& in,
                        uint64_t max_dir_bytes, std::vector<AlignResult>& out, RunPools& pools) {
@@ -1182,7 +1192,8 @@ static int align_batch(saber_gpu* h, const Scheme& sch, const Dataset& ds, const
         int64_t lo = r.lo, hi = r.hi;
         const int64_t m = (int64_t)(qs.offs[r.query + 1] - qs.offs[r.query]);
         const int64_t w = clip_band(m, r.win_len, lo, hi);
-        return r.want_dir && r.stop_at >= 1 && w <= kAlignWaveWidth && m < (1 << 28) && r.win_len < (1u << 28);
+        return r.want_dir && r.stop_at >= 1 && w <= kAlignWaveWidth && m >= kAlignWaveRows && w <= kAlignWaveAspect * m &&
+               m < (1 << 28) && r.win_len < (1u << 28);
     };
     const size_t n_wave = (size_t)(std::stable_partition(todo.begin(), todo.end(), by_wave) - todo.begin());
     cudaStream_t s = h->stream;
