@@ -506,6 +506,13 @@ uint32_t saber_gpu_get_long_steps(saber_gpu* h);
 int saber_gpu_set_scan_table_bytes(saber_gpu* h, uint64_t bytes);
 uint64_t saber_gpu_get_scan_table_bytes(saber_gpu* h);
 
+/* Tuning: batch positions whose seed tables saber_gpu_scan builds at a time; a
+ * larger batch goes in blocks of equal length, each with its own tables and
+ * passes over the database.  0 (the default): as many as tables of 16 GB hold.
+ * Results do not depend on it.  No reference counterpart. */
+int saber_gpu_set_scan_block(saber_gpu* h, uint64_t positions);
+uint64_t saber_gpu_get_scan_block(saber_gpu* h);
+
 /* Captured scoring graphs (default on): saber_gpu_score_band_jobs (and so
  * the batch engine's scoring stages) runs classify -> radix sort -> int16
  * kernels -> int32 kernel as one CUDA graph with every count kept on the

@@ -171,6 +171,7 @@ struct saber_gpu {
         sc_rk64a, sc_rk64b, sc_rk64c, sc_rk32a, sc_rk32b, sc_ridxa, sc_ridxb, sc_regions2, sc_rstat, sc_rstat2,
         sc_flags, sc_nib, sc_fil, sc_qwin, sc_qwinx, sc_surv2, sc_qrng, sc_ewin, sc_pl, sc_combtab;
     bool sc_comb = false;  // the database's bit planes (sc_pl) are built
+    uint64_t scan_block = 0;  // tuning: batch positions per block of a scan (0: scan_block_len's)
     uint64_t scan_table_bytes = 48ull << 20;  // tuning: seed-table bytes per scan pass (L2 budget)
     bool has_db_mask = false;
     // learned triage: installed model, per-call feature buffers, collection

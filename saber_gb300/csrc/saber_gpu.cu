@@ -1838,6 +1838,14 @@ int saber_gpu_set_long_steps(saber_gpu* h, uint32_t steps) {
 
 uint32_t saber_gpu_get_long_steps(saber_gpu* h) { return h ? h->long_steps : 0u; }
 
+int saber_gpu_set_scan_block(saber_gpu* h, uint64_t positions) {
+    ENTER(h);
+    h->scan_block = positions;
+    return SABER_OK;
+}
+
+uint64_t saber_gpu_get_scan_block(saber_gpu* h) { return h ? h->scan_block : 0u; }
+
 int saber_gpu_set_scan_table_bytes(saber_gpu* h, uint64_t bytes) {
     ENTER(h);
     h->scan_table_bytes = bytes;

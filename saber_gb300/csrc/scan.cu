@@ -1615,8 +1615,9 @@ constexpr uint64_t kEntryWindowBytes = 64ull << 20;
 // reads the database again, 18 ms for 150 M residues and 16 shapes, and
 // smaller blocks that would keep the windows in L2 lost more to that (11,000
 // queries in 1 / 2 / 3 / 6 blocks: 113 / 117 / 126 / 166 ms).
-static uint64_t scan_block_len(uint64_t QN, uint32_t nshapes) {
-    const uint64_t most = (16ull << 30) / 48 / nshapes;
+static uint64_t scan_block_len(const saber_gpu* h, uint64_t QN, uint32_t nshapes) {
+    uint64_t most = (16ull << 30) / 48 / nshapes;
+    if (h->scan_block) most = std::min(most, h->scan_block);
     const uint64_t blocks = std::max<uint64_t>(1, (QN + most - 1) / most);
     return std::max<uint64_t>(1, (QN + blocks - 1) / blocks);
 }
@@ -2013,7 +2014,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     const bool windows = comb && p->hit_filter_min_ids > 0 && QN * 32 > kEntryWindowBytes;  // copied to the entries
     // a large batch goes in blocks of positions (scan_block_len), each with its
     // own tables and its own passes over the database
-    const uint64_t block_len = scan_block_len(QN, nsh);
+    const uint64_t block_len = scan_block_len(h, QN, nsh);
     const uint64_t ngroups = gbase[nsh], nranks = (uint64_t)nsh * block_len;
     CUALLOC(h, h->sc_qpres, ngroups * 8 + 8);
     CUALLOC(h, h->sc_qslot, nranks * 4 + 4);

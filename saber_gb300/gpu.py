@@ -235,6 +235,8 @@ def load_library():
         "saber_gpu_collected_regions": (ctypes.c_int, [P, P, P, P, U64, P]),
         "saber_gpu_get_pair_steps": (U32, [P]),
         "saber_gpu_set_scan_table_bytes": (ctypes.c_int, [P, U64]),
+        "saber_gpu_set_scan_block": (ctypes.c_int, [P, U64]),
+        "saber_gpu_get_scan_block": (U64, [P]),
         "saber_gpu_set_long_steps": (ctypes.c_int, [P, U32]),
         "saber_gpu_get_long_steps": (U32, [P]),
         "saber_gpu_get_scan_table_bytes": (U64, [P]),
@@ -600,6 +602,15 @@ class Device:
     @scan_table_bytes.setter
     def scan_table_bytes(self, v):
         self._check(self.lib.saber_gpu_set_scan_table_bytes(self.h, int(v)), "set_scan_table_bytes")
+
+    @property
+    def scan_block(self):
+        """Batch positions whose seed tables a scan builds at a time (0: as many as 16 GB of tables hold)."""
+        return int(self.lib.saber_gpu_get_scan_block(self.h))
+
+    @scan_block.setter
+    def scan_block(self, v):
+        self._check(self.lib.saber_gpu_set_scan_block(self.h, int(v)), "set_scan_block")
 
     def probe_int_peak(self):
         """(DPX s16x2 lane-instructions/s, int32 max lane-instructions/s) of this GPU."""
