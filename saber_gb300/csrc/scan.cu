@@ -1607,7 +1607,8 @@ static bool comb_table(const saber_scan_params* p, uint8_t* tab /* 256 */) {
 // copy per shape).  Scan stage without / with the copies on one GB300: 105 MB
 // of records (11,000 queries x 150 M residues) 112.0 / 90.2 ms; 49 MB (5,000 x
 // 100 M) 35.5 / 34.7 and the tables 2.1 / 2.7; 14 MB (1,500 x 60 M) 10.5 / 10.8,
-// with the shorter seeds of the sensitive preset 12.9 / 15.2.
+// with the shorter seeds of the sensitive preset 12.9 / 15.2.  The copies only
+// save time: where they do not fit (reserve_spare) the scan reads by position.
 constexpr uint64_t kEntryWindowBytes = 64ull << 20;
 
 // Positions per block of a batch's scan.  Blocks bound the tables' memory (48
@@ -2011,7 +2012,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
         k_query_windows<<<nblocks(QN * 32, 256), 256, 0, s>>>(
             h->sc_qsb.as<uint8_t>(), h->sc_qfull.as<uint8_t>(), h->sc_qrem.as<uint8_t>(), h->sc_qdst.as<uint8_t>(),
             QN, cfil, h->sc_qwin.as<uint8_t>(), h->sc_qwinx.as<uint8_t>());
-    const bool windows = comb && p->hit_filter_min_ids > 0 && QN * 32 > kEntryWindowBytes;  // copied to the entries
+    bool windows = comb && p->hit_filter_min_ids > 0 && QN * 32 > kEntryWindowBytes;  // copied to the entries
     // a large batch goes in blocks of positions (scan_block_len), each with its
     // own tables and its own passes over the database
     const uint64_t block_len = scan_block_len(h, QN, nsh);
@@ -2020,7 +2021,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     CUALLOC(h, h->sc_qslot, nranks * 4 + 4);
     CUALLOC(h, h->sc_qent, nranks * 4 + 4);
     CUALLOC(h, h->sc_qrng, nranks * 8 + 8);
-    if (windows) CUALLOC(h, h->sc_ewin, nranks * 32 + 32);
+    windows = windows && reserve_spare(h->sc_ewin, nranks * 32 + 32);
     if (few) CUALLOC(h, h->sc_fil, ((uint64_t)nsh << few_bits) / 8);
     SeedArgs sa;
     sa.qsb = h->sc_qsb.as<uint8_t>();

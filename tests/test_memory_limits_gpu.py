@@ -10,6 +10,7 @@ from saber_gb300 import presets, synth
 from saber_gb300.gpu import Device, SaberGpuError, scan_params
 from saber_gb300.scoring import matrix
 from tests.test_scan_gpu import _check
+from tests.test_scan_small_batch_gpu import _sets
 
 pytestmark = pytest.mark.gpu
 B62 = matrix("BLOSUM62")
@@ -69,3 +70,24 @@ def test_scan_after_parameters_whose_tables_did_not_fit():
     want, ost = orc.scan_regions(ss.codes, ss.offsets, None, qs.codes, qs.offsets, None, None, None, B62, op)
     assert want.size > 0
     _check(got, gst, want, ost)
+
+
+def test_scan_without_room_for_its_entries_windows():
+    """A batch whose window records are copied to its seed entries (1 GB of
+    copies) is scanned without the copies where they do not fit."""
+    qn = (64 << 20) // 32 + 1
+    qs, ss, _ = _sets(11, qn, 3000)
+    amap, asz = presets.alphabet_map()
+    kw = dict(min_ids=27, exact_weight=2, db_length=int(ss.codes.size))
+    gp, op = scan_params(amap, asz, presets.DS16, **kw), orc.make_scan_params(amap, asz, presets.DS16, **kw)
+    with Device(0) as dev:
+        dev.set_scheme(B62, 11, 1)
+        dev.load_db(ss.codes, ss.offsets)
+        dev.load_queries(qs.codes, qs.offsets, None)
+        with memory_left(3 * GIB // 2):
+            got, gst = dev.scan(gp, None, None)
+        again, ast = dev.scan(gp, None, None)  # with them
+    want, ost = orc.scan_regions(ss.codes, ss.offsets, None, qs.codes, qs.offsets, None, None, None, B62, op)
+    assert ost["hits"] > 0
+    _check(got, gst, want, ost)
+    _check(again, ast, want, ost)
