@@ -232,17 +232,21 @@ static int fail(saber_gpu* h, int code, const char* fmt, ...) {
     } while (0)
 
 
-// Reserves a buffer that a call is faster with and can do without: no more than
-// a quarter of the free memory (what the buffer holds counted), so that what the
-// call needs, and other handles, still fit.  False: not reserved.
-static inline bool reserve_spare(DevBuf& b, size_t bytes) {
-    if (b.p && bytes <= b.cap) return true;
+// Memory that a call is faster with and can do without: up to a quarter of what
+// is free (`held` bytes that would be given back for it counted), so that what the
+// call needs, and other handles, still fit.
+static inline bool spare_memory(size_t bytes, size_t held) {
     size_t free = 0, total = 0;
     if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return bytes <= (free + b.cap) / 4 && b.reserve(bytes) == cudaSuccess;
+    return bytes <= (free + held) / 4;
+}
+// Reserves such a buffer; false: not reserved.
+static inline bool reserve_spare(DevBuf& b, size_t bytes) {
+    if (b.p && bytes <= b.cap) return true;
+    return spare_memory(bytes, b.cap) && b.reserve(bytes) == cudaSuccess;
 }
 
 int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask, const int32_t* region_thr,

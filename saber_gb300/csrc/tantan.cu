@@ -599,9 +599,26 @@ __global__ void __launch_bounds__(THREADS, MINB) k_tantan8(const __grid_constant
 
 // ---- host driver ------------------------------------------------------------------
 
-// Scratch rows (positions) per launch: 64 F floats + one float2 each (8.9 GB;
-// 30 M residues are one launch, which ends once instead of four times).
+// Scratch rows (positions) per launch: 64 F floats + one float2 each, 8.9 GB at
+// most.  A launch ends with its last sequences' chains while most of the GPU is
+// idle, so a large call takes few (30 M residues: 7.3 ms in four launches of 8 M
+// rows, 4.0 in one).  Above kTtRowsLeast (2.2 GB) the rows may take a quarter of
+// the free memory; what does not fit is halved.
 constexpr uint64_t kTtRowsPerLaunch = 32ull << 20;
+constexpr uint64_t kTtRowsLeast = 8ull << 20;
+constexpr size_t kTtRowBytes = kTtMaxW * sizeof(float) + sizeof(float2);
+
+static bool tt_reserve(saber_gpu* h, uint64_t rows) {
+    const size_t held = h->tt_F.cap + h->tt_BS.cap;
+    if (rows > kTtRowsLeast && rows * kTtRowBytes > held && !spare_memory(rows * kTtRowBytes, held)) return false;
+    rows = std::max<uint64_t>(rows, 1);
+    if (h->tt_F.reserve(rows * kTtMaxW * sizeof(float)) == cudaSuccess &&
+        h->tt_BS.reserve(rows * sizeof(float2)) == cudaSuccess)
+        return true;
+    h->tt_F.release();
+    h->tt_BS.release();
+    return false;
+}
 
 // Masks the sequences [offs[i], offs[i+1]) of the device residues d_codes
 // (offsets on the host: h_offs; on the device: d_offs) into d_mask (one byte
@@ -626,32 +643,45 @@ int tantan_run(saber_gpu* h, const TantanModel& M, const uint8_t* d_codes, const
         bucket[b] = (uint32_t)acc;
         acc += c;
     }
-    const uint64_t cap = std::max<uint64_t>(kTtRowsPerLaunch, maxn);
     std::vector<uint32_t> ord(nseq);
     std::vector<uint64_t> base(nseq);
     for (uint64_t i = 0; i < nseq; i++)
         ord[bucket[nb - 1 - std::min<uint64_t>(h_offs[i + 1] - h_offs[i], nb - 1)]++] = (uint32_t)i;
-    std::vector<uint64_t> cuts{0};
-    uint64_t rows = 0;
-    for (uint64_t k = 0; k < nseq; k++) {
-        const uint64_t n = h_offs[ord[k] + 1] - h_offs[ord[k]];
-        if (rows + n > cap) {
-            cuts.push_back(k);
-            rows = 0;
-        }
-        base[k] = rows;
-        rows += n;
-    }
-    cuts.push_back(nseq);
+    // launches of about the same rows, as few as the limit allows
+    const uint64_t total = h_offs[nseq] - h_offs[0];
+    std::vector<uint64_t> cuts;
     uint64_t rows_max = 0;
-    for (size_t c = 0; c + 1 < cuts.size(); c++) {
-        const uint64_t k = cuts[c + 1] - 1;
-        rows_max = std::max(rows_max, base[k] + (h_offs[ord[k] + 1] - h_offs[ord[k]]));
+    auto cut = [&](uint64_t limit) {
+        uint64_t cap = std::max(limit, maxn);
+        if (total > limit && maxn < limit / 2) {
+            const uint64_t launches = (total + limit - maxn - 1) / (limit - maxn);
+            cap = (total + launches - 1) / launches + maxn;
+        }
+        cuts.assign(1, 0);
+        rows_max = 0;
+        uint64_t rows = 0;
+        for (uint64_t k = 0; k < nseq; k++) {
+            const uint64_t n = h_offs[ord[k] + 1] - h_offs[ord[k]];
+            if (rows + n > cap) {
+                cuts.push_back(k);
+                rows = 0;
+            }
+            base[k] = rows;
+            rows += n;
+            rows_max = std::max(rows_max, rows);
+        }
+        cuts.push_back(nseq);
+    };
+    uint64_t limit = kTtRowsPerLaunch;
+    cut(limit);
+    while (!tt_reserve(h, rows_max)) {
+        if (rows_max <= maxn)
+            return fail(h, SABER_ERR_NOMEM, "device allocation of %zu bytes of tantan rows", (size_t)(rows_max * kTtRowBytes));
+        limit = rows_max / 2;
+        cut(limit);
     }
     CUALLOC(h, h->tt_ord, nseq * sizeof(uint32_t));
     CUALLOC(h, h->tt_base, nseq * sizeof(uint64_t));
-    CUALLOC(h, h->tt_F, std::max<uint64_t>(rows_max, 1) * kTtMaxW * sizeof(float));
-    CUALLOC(h, h->tt_BS, std::max<uint64_t>(rows_max, 1) * sizeof(float2));
     CUALLOC(h, h->tt_count, sizeof(unsigned long long));
     CU(h, cudaMemcpyAsync(h->tt_ord.p, ord.data(), nseq * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
     CU(h, cudaMemcpyAsync(h->tt_base.p, base.data(), nseq * sizeof(uint64_t), cudaMemcpyHostToDevice, h->stream));
@@ -689,10 +719,10 @@ int tantan_run(saber_gpu* h, const TantanModel& M, const uint8_t* d_codes, const
             (float*)h->tt_F.p, (float2*)h->tt_BS.p, d_mask, d_probs, (unsigned long long*)h->tt_count.p);
         CU(h, cudaGetLastError());
     }
-    unsigned long long total = 0;
-    CU(h, cudaMemcpyAsync(&total, h->tt_count.p, sizeof(total), cudaMemcpyDeviceToHost, h->stream));
+    unsigned long long masked = 0;
+    CU(h, cudaMemcpyAsync(&masked, h->tt_count.p, sizeof(masked), cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
-    *n_masked = total;
+    *n_masked = masked;
     return SABER_OK;
 }
 

@@ -8,6 +8,7 @@ import pytest
 from oracle import oracle as orc
 from saber_gb300 import presets, synth
 from saber_gb300.gpu import Device, SaberGpuError, scan_params
+from saber_gb300.masking import TantanParams
 from saber_gb300.scoring import matrix
 from tests.test_scan_gpu import _check
 from tests.test_scan_small_batch_gpu import _sets
@@ -91,3 +92,22 @@ def test_scan_without_room_for_its_entries_windows():
     assert ost["hits"] > 0
     _check(got, gst, want, ost)
     _check(again, ast, want, ost)
+
+
+@pytest.mark.parametrize("left", [2600 << 20, 600 << 20])
+@pytest.mark.parametrize("longest", [900, 700_000])
+def test_tantan_rows_in_less_memory(left, longest):
+    """12 M residues want 3.2 GB of rows; with less they go in smaller launches."""
+    rng = np.random.default_rng(4)
+    lens = np.append(rng.integers(1, 900, size=26_700), longest)
+    off = np.zeros(lens.size + 1, np.uint64)
+    off[1:] = np.cumsum(lens)
+    codes = rng.integers(0, 24, size=int(off[-1])).astype(np.uint8)
+    for s in range(0, codes.size - 40, 997):
+        codes[s:s + 30] = np.resize(codes[s:s + 3], 30)
+    with Device(0) as dev:
+        with memory_left(left):
+            m, p, n, _ = dev.tantan_mask(TantanParams(), B62, codes, off, want_probs=True)
+    with Device(0) as dev:
+        wm, wp, wn, _ = dev.tantan_mask(TantanParams(), B62, codes, off, want_probs=True)
+    assert n == wn > 0 and np.array_equal(m, wm) and np.array_equal(p.view(np.uint32), wp.view(np.uint32))
