@@ -120,9 +120,23 @@ struct GraphEntry {
 };
 
 // Work buffers of the triage network's host entry points (gradients, training,
-// prediction): kept with the handle, sized by the largest call so far.
+// prediction), kept with the handle up to kTriageKeep bytes of rows: allocating
+// them took longer than a call on a few thousand rows, and takes a small part of
+// one on two million (prediction, 132 bytes a row) or 80,000 (gradients, 3.3 KB).
+constexpr size_t kTriageKeep = 256u << 20;
 struct TriageScratch {
     DevBuf model, wb, X, Xn, y, H1, H2, z, dz, dH1, part, grad, m, v, loss;
+    // At the end of a call: what is above that is given back.
+    struct Trim {
+        TriageScratch& t;
+        ~Trim() {
+            DevBuf* rows[] = {&t.X, &t.Xn, &t.y, &t.H1, &t.H2, &t.z, &t.dz, &t.dH1};
+            size_t held = 0;
+            for (const DevBuf* b : rows) held += b->cap;
+            if (held <= kTriageKeep) return;
+            for (DevBuf* b : rows) b->release();
+        }
+    };
 };
 
 struct Scheme {
