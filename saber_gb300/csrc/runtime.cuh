@@ -126,17 +126,14 @@ struct GraphEntry {
 constexpr size_t kTriageKeep = 256u << 20;
 struct TriageScratch {
     DevBuf model, wb, X, Xn, y, H1, H2, z, dz, dH1, part, grad, m, v, loss;
-    // At the end of a call: what is above that is given back.
-    struct Trim {
-        TriageScratch& t;
-        ~Trim() {
-            DevBuf* rows[] = {&t.X, &t.Xn, &t.y, &t.H1, &t.H2, &t.z, &t.dz, &t.dH1};
-            size_t held = 0;
-            for (const DevBuf* b : rows) held += b->cap;
-            if (held <= kTriageKeep) return;
-            for (DevBuf* b : rows) b->release();
-        }
-    };
+    // gives the rows' buffers back, those above `keep` bytes only
+    void trim(size_t keep) {
+        DevBuf* rows[] = {&X, &Xn, &y, &H1, &H2, &z, &dz, &dH1};
+        size_t held = 0;
+        for (const DevBuf* b : rows) held += b->cap;
+        if (held <= keep) return;
+        for (DevBuf* b : rows) b->release();
+    }
 };
 
 struct Scheme {
@@ -152,6 +149,7 @@ struct Scheme {
 }  // namespace saber
 
 struct saber_gpu {
+    unsigned spare_used = 0;  // kSpare bits of the scratch that the running call works in
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // host-to-device copies beside the stream's work (made on first use)
@@ -230,6 +228,32 @@ static int fail(saber_gpu* h, int code, const char* fmt, ...) {
     return code;
 }
 
+// Scratch that a handle keeps between calls for speed alone.  An allocation that
+// does not fit takes back what the running call does not work in (SpareUse).
+enum : unsigned { kSpareRows = 1, kSpareWindows = 2, kSpareTriage = 4 };
+struct SpareUse {
+    saber_gpu* h;
+    unsigned bit;
+    SpareUse(saber_gpu* h_, unsigned bit_) : h(h_), bit(bit_) { h->spare_used |= bit; }
+    ~SpareUse() {
+        h->spare_used &= ~bit;
+        if (bit == kSpareTriage) h->tg.trim(kTriageKeep);
+    }
+    SpareUse(const SpareUse&) = delete;
+    SpareUse& operator=(const SpareUse&) = delete;
+};
+static bool give_back(saber_gpu* h) {
+    const size_t held = h->tt_F.cap + h->tt_BS.cap + h->sc_ewin.cap;
+    if (!(h->spare_used & kSpareRows)) {
+        h->tt_F.release();
+        h->tt_BS.release();
+    }
+    if (!(h->spare_used & kSpareWindows)) h->sc_ewin.release();
+    const bool rows = h->tg.X.cap + h->tg.H1.cap > 0 && !(h->spare_used & kSpareTriage);
+    if (rows) h->tg.trim(0);
+    return rows || h->tt_F.cap + h->tt_BS.cap + h->sc_ewin.cap < held;
+}
+
 #define CU(h, call)                                                                       \
     do {                                                                                  \
         cudaError_t e_ = (call);                                                          \
@@ -240,6 +264,7 @@ static int fail(saber_gpu* h, int code, const char* fmt, ...) {
 #define CUALLOC(h, buf, bytes)                                                            \
     do {                                                                                  \
         cudaError_t e_ = (buf).reserve(bytes);                                            \
+        if (e_ != cudaSuccess && ::saber::give_back(h)) e_ = (buf).reserve(bytes);        \
         if (e_ != cudaSuccess)                                                            \
             return ::saber::fail((h), SABER_ERR_NOMEM, "device allocation of %zu bytes: %s", \
                                  (size_t)(bytes), cudaGetErrorString(e_));                \

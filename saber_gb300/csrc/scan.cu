@@ -1942,6 +1942,7 @@ int scan_regions(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask
     for (uint32_t q = 0; q < qs.nq; q++)
         if (qs.offs[q + 1] - qs.offs[q] >= (uint64_t)kDBias) return fail(h, SABER_ERR_ARG, "query too long");
     cudaStream_t s = h->stream;
+    const SpareUse use(h, kSpareWindows);
     if (h->sc_key != fingerprint(h, p)) {
         int rc = scan_build_db(h, p);
         if (rc != SABER_OK) return rc;

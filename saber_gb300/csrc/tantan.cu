@@ -612,9 +612,10 @@ static bool tt_reserve(saber_gpu* h, uint64_t rows) {
     const size_t held = h->tt_F.cap + h->tt_BS.cap;
     if (rows > kTtRowsLeast && rows * kTtRowBytes > held && !spare_memory(rows * kTtRowBytes, held)) return false;
     rows = std::max<uint64_t>(rows, 1);
-    if (h->tt_F.reserve(rows * kTtMaxW * sizeof(float)) == cudaSuccess &&
-        h->tt_BS.reserve(rows * sizeof(float2)) == cudaSuccess)
-        return true;
+    for (bool more = true; more; more = give_back(h))
+        if (h->tt_F.reserve(rows * kTtMaxW * sizeof(float)) == cudaSuccess &&
+            h->tt_BS.reserve(rows * sizeof(float2)) == cudaSuccess)
+            return true;
     h->tt_F.release();
     h->tt_BS.release();
     return false;
@@ -672,6 +673,7 @@ int tantan_run(saber_gpu* h, const TantanModel& M, const uint8_t* d_codes, const
         }
         cuts.push_back(nseq);
     };
+    const SpareUse use(h, kSpareRows);
     uint64_t limit = kTtRowsPerLaunch;
     cut(limit);
     while (!tt_reserve(h, rows_max)) {

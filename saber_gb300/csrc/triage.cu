@@ -844,7 +844,7 @@ int triage_grads(saber_gpu* h, const float* model, const float* X, const uint8_t
                  float* grads, double* loss) {
     if (n == 0) return fail(h, SABER_ERR_CUDA, "no rows: invalid launch configuration");
     TriageScratch& d = h->tg;
-    const TriageScratch::Trim trim{d};
+    const SpareUse use(h, kSpareTriage);
     int rc = upload_model(h, d.model, d.wb, model);
     if (rc != SABER_OK) return rc;
     rc = reserve_batch(h, d, n);
@@ -872,7 +872,7 @@ int triage_train(saber_gpu* h, float* model, const float* X, const uint8_t* y, u
     cudaStream_t s = h->stream;
     const int B = (int)std::max<uint32_t>(32, cfg->batch);
     TriageScratch& d = h->tg;
-    const TriageScratch::Trim trim{d};
+    const SpareUse use(h, kSpareTriage);
     int rc = upload_model(h, d.model, d.wb, model);
     if (rc != SABER_OK) return rc;
     rc = reserve_batch(h, d, (uint64_t)B);
@@ -970,7 +970,7 @@ constexpr uint64_t kPredictChunk = 128 << 10;
 
 int triage_predict_host(saber_gpu* h, const float* model, const float* X, uint64_t n, float* logits) {
     TriageScratch& d = h->tg;
-    const TriageScratch::Trim trim{d};
+    const SpareUse use(h, kSpareTriage);
     int rc = upload_model(h, d.model, d.wb, model);
     if (rc != SABER_OK) return rc;
     CUALLOC(h, d.X, std::max<uint64_t>(n, 1) * kTIn * 4);

@@ -111,3 +111,27 @@ def test_tantan_rows_in_less_memory(left, longest):
     with Device(0) as dev:
         wm, wp, wn, _ = dev.tantan_mask(TantanParams(), B62, codes, off, want_probs=True)
     assert n == wn > 0 and np.array_equal(m, wm) and np.array_equal(p.view(np.uint32), wp.view(np.uint32))
+
+
+@pytest.mark.parametrize("held", ["tantan rows", "entry windows"])
+def test_scratch_kept_for_speed_is_given_back_for_a_database(held):
+    """A database that fits only without what the call before kept."""
+    with Device(0) as dev:
+        dev.set_scheme(B62, 11, 1)
+        if held == "tantan rows":
+            left, size = 3 * GIB, 5 * GIB // 2
+            off = np.arange(0, 12_000_001, 400, dtype=np.uint64)
+            codes = np.resize(np.arange(20, dtype=np.uint8), int(off[-1]))
+        else:
+            left, size = 6 * GIB, 4900 << 20
+            qs, ss, _ = _sets(11, (64 << 20) // 32 + 1, 3000)
+            amap, asz = presets.alphabet_map()
+            gp = scan_params(amap, asz, presets.DS16, min_ids=27, exact_weight=2, db_length=int(ss.codes.size))
+        with memory_left(left):
+            if held == "tantan rows":
+                dev.tantan_mask(TantanParams(), B62, codes, off)
+            else:
+                dev.load_db(ss.codes, ss.offsets)
+                dev.load_queries(qs.codes, qs.offsets, None)
+                dev.scan(gp, None, None)
+            dev.load_db(np.zeros(size, np.uint8), np.array([0, size], np.uint64))
