@@ -14,9 +14,10 @@
 //
 // Whole-number work is the host's.  The f64 thresholds (the score that sends a
 // region to the second stage, the E-value cut) are logarithms and exponentials
-// whose last bit may differ from the host's libm: a stage-two decision closer
-// to its threshold than kTie is left to the host, and the cut keeps a margin
-// (the host applies the exact rule to what it gets).
+// whose last bits may differ from the host's libm: a stage-two decision within
+// kTie of its threshold, or one that a length adjustment within kTie of a whole
+// number could turn, is left to the host (all of a batch's in one exchange), and
+// the cut keeps a margin (the host applies the exact rule to what it gets).
 #include <cub/cub.cuh>
 #include <cuda_runtime.h>
 #include <thrust/iterator/counting_iterator.h>
@@ -28,7 +29,8 @@
 
 namespace saber {
 
-constexpr double kTie = 1e-7;
+constexpr double kTie = 1e-10;        // relative to the terms summed; the two libms differ by about 1e-15 of them
+constexpr double kCutMargin = 1e-7;
 constexpr int64_t kBandScoreMinCells = 1 << 20;  // engine.rs:401
 constexpr int64_t kBandCostRatio = 12;           // engine.rs:402
 constexpr int64_t kBandBridge = 1024;            // engine.rs:404
@@ -210,13 +212,16 @@ __global__ void k_plan_jobs(const saber_region* __restrict__ reg, const int2* __
     if ((threadIdx.x & 31) == 0 && nb) atomicAdd(banded, nb);
 }
 
-// QueryStatistics::space_lower_bound (stats.rs) in f64; `more` is added to the
-// length adjustment, `tie` set when its rounding up is in doubt.
-__device__ __forceinline__ double pl_space(const PlanParams& P, int64_t qlen, int64_t sl, double more, bool& tie) {
+// QueryStatistics::space_lower_bound (stats.rs) in f64: the length adjustment
+// before it is rounded up, and how far it may be off; the space for one.
+__device__ __forceinline__ double pl_adjustment(const PlanParams& P, int64_t qlen, int64_t sl, double& eps) {
     const double m = (double)max(qlen, (int64_t)1), n = (double)max(sl, (int64_t)1);
-    const double v = fmax(P.adl * (P.log_k + log(m * n)) + P.beta, 0.0);
-    tie = fabs(v - rint(v)) < kTie * (v + 1.0) && v > 0.0;
-    const double up = ceil(v) + more;
+    const double l = log(m * n);
+    eps = kTie * (fabs(P.adl) * (fabs(P.log_k) + l) + fabs(P.beta) + 1.0);
+    return P.adl * (P.log_k + l) + P.beta;
+}
+__device__ __forceinline__ double pl_space(const PlanParams& P, int64_t qlen, int64_t sl, double up) {
+    const double m = (double)max(qlen, (int64_t)1), n = (double)max(sl, (int64_t)1);
     return P.num_seqs * fmax(m - up, 1.0) * fmax(n - up, 1.0);
 }
 
@@ -235,25 +240,57 @@ __global__ void k_plan_again(const saber_region* __restrict__ reg, const DevPlan
         if (plan[i].kind == 1) {
             const saber_region r = reg[i];
             bool tie = false;
-            double f;
             if (P.database_model) {
-                f = (double)region_floor[r.query];
+                ag = (double)s >= P.prefilter_frac * (double)region_floor[r.query];
             } else {
-                f = 1.0;
+                // reaches the threshold of a bound of 1, or of the search space's
+                const double wide = kTie * fabs(P.prefilter_frac) * (1.0 + 1.0 / P.lambda);
+                auto reaches = [&](double f) {
+                    if (P.even) f -= 1.0;
+                    const double thr = P.prefilter_frac * f;
+                    tie |= !(fabs((double)s - thr) > kTie * (fabs(thr) + 1.0) + wide);
+                    return (double)s >= thr;
+                };
                 if (P.region_evalue > 0.0 && isfinite(P.region_evalue)) {
                     const int64_t qlen = (int64_t)(qoffs[r.query + 1] - qoffs[r.query]);
                     const int64_t sl = (int64_t)(soffs[r.subject + 1] - soffs[r.subject]);
-                    f = fmax(f, log(P.k * pl_space(P, qlen, sl, 0.0, tie) / P.region_evalue) / P.lambda);
+                    double eps;
+                    const double v = pl_adjustment(P, qlen, sl, eps), whole = rint(v);
+                    auto with = [&](double up) {
+                        return reaches(fmax(1.0, log(P.k * pl_space(P, qlen, sl, up) / P.region_evalue) / P.lambda));
+                    };
+                    if (fabs(v - whole) > eps || whole < 0.0) {
+                        ag = with(ceil(fmax(v, 0.0)));
+                    } else {  // the host may round it up to either
+                        ag = with(whole);
+                        tie |= !isfinite(v) || with(whole + 1.0) != ag;
+                    }
+                } else {
+                    ag = reaches(1.0);
                 }
-                if (P.even) f -= 1.0;
+                if (tie) ties[atomicAdd(nties, 1u)] = i;
             }
-            const double thr = P.prefilter_frac * f;
-            ag = (double)s >= thr;
-            if (!P.database_model && (tie || fabs((double)s - thr) <= kTie * (fabs(thr) + 1.0)))
-                ties[atomicAdd(nties, 1u)] = i;
         }
         again[i] = ag;
     }
+}
+
+// What the host needs to decide a tie, and its answers.
+struct TieRec {
+    uint32_t query, slen;
+    int32_t score;
+};
+__global__ void k_plan_ties(const saber_region* __restrict__ reg, const int32_t* __restrict__ score,
+                            const uint64_t* __restrict__ soffs, const uint32_t* __restrict__ ties, uint32_t n,
+                            TieRec* __restrict__ out) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const saber_region r = reg[ties[t]];
+        out[t] = {r.query, (uint32_t)(soffs[r.subject + 1] - soffs[r.subject]), score[ties[t]]};
+    }
+}
+__global__ void k_plan_untie(const uint32_t* __restrict__ ties, uint32_t n, const uint8_t* __restrict__ answers,
+                             uint8_t* __restrict__ again) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) again[ties[t]] = answers[t];
 }
 
 __global__ void k_plan_jobs2(const saber_region* __restrict__ reg, const DevPlan* __restrict__ plan,
@@ -287,13 +324,14 @@ __global__ void k_plan_keep(const saber_region* __restrict__ reg, const int32_t*
             const double adj = (double)(P.even && (s & 1) ? s - 1 : s);
             if (k && P.has_bits) {
                 const double bits = (P.lambda * adj - P.log_k) / 0.69314718055994530942;
-                k = bits >= P.min_bitscore - kTie * (fabs(P.min_bitscore) + 1.0);
+                k = !(bits < P.min_bitscore - kCutMargin * (fabs(P.min_bitscore) + 1.0));
             }
             if (k && isfinite(P.evalue_cut)) {
                 const int64_t qlen = (int64_t)(qoffs[r.query + 1] - qoffs[r.query]);
                 const int64_t sl = (int64_t)(soffs[r.subject + 1] - soffs[r.subject]);
-                bool tie;
-                k = P.k * pl_space(P, qlen, sl, 1.0, tie) * exp(-P.lambda * adj) <= P.evalue_cut * (1.0 + kTie);
+                double eps;
+                const double up = ceil(fmax(pl_adjustment(P, qlen, sl, eps), 0.0)) + 1.0;  // (the host's, or one more)
+                k = !(P.k * pl_space(P, qlen, sl, up) * exp(-P.lambda * adj) > P.evalue_cut * (1.0 + kCutMargin));
             }
         }
         keep[i] = k;
@@ -409,22 +447,21 @@ int plan_and_score(saber_gpu* h, const RegionSink& sk, const PlanParams& P, cons
     out.banded = ((uint64_t)hc[3] << 32) | hc[2];
     if (hc[1]) {
         // decisions too close for the device: the host's libm decides
-        std::vector<uint32_t> at(hc[1]);
-        CU(h, cudaMemcpyAsync(at.data(), ties, (uint64_t)hc[1] * 4, cudaMemcpyDeviceToHost, s));
+        const uint32_t nt = hc[1];
+        CUALLOC(h, h->pl_ties, (uint64_t)nt * (sizeof(TieRec) + 1));
+        TieRec* d_rec = h->pl_ties.as<TieRec>();
+        uint8_t* d_answer = reinterpret_cast<uint8_t*>(d_rec + nt);
+        std::vector<TieRec> rec(nt);
+        std::vector<uint8_t> answer(nt);
+        k_plan_ties<<<nblocks(nt, 256, h->sm_count * 32), 256, 0, s>>>(reg, score, soffs, ties, nt, d_rec);
+        CU(h, cudaGetLastError());
+        CU(h, cudaMemcpyAsync(rec.data(), d_rec, nt * sizeof(TieRec), cudaMemcpyDeviceToHost, s));
         CU(h, cudaStreamSynchronize(s));
-        for (uint32_t i : at) {
-            saber_region r;
-            int32_t v;
-            uint64_t so[2];
-            CU(h, cudaMemcpyAsync(&r, reg + i, sizeof(r), cudaMemcpyDeviceToHost, s));
-            CU(h, cudaMemcpyAsync(&v, score + i, 4, cudaMemcpyDeviceToHost, s));
-            CU(h, cudaStreamSynchronize(s));
-            CU(h, cudaMemcpyAsync(so, soffs + r.subject, 16, cudaMemcpyDeviceToHost, s));
-            CU(h, cudaStreamSynchronize(s));
-            const uint8_t ag = tie(r.query, (int64_t)(so[1] - so[0]), v) ? 1 : 0;
-            CU(h, cudaMemcpyAsync(flag + i, &ag, 1, cudaMemcpyHostToDevice, s));
-            CU(h, cudaStreamSynchronize(s));
-        }
+        for (uint32_t t = 0; t < nt; t++) answer[t] = tie(rec[t].query, (int64_t)rec[t].slen, rec[t].score) ? 1 : 0;
+        CU(h, cudaMemcpyAsync(d_answer, answer.data(), nt, cudaMemcpyHostToDevice, s));
+        k_plan_untie<<<nblocks(nt, 256, h->sm_count * 32), 256, 0, s>>>(ties, nt, d_answer, flag);
+        CU(h, cudaGetLastError());
+        CU(h, cudaStreamSynchronize(s));  // (answer is this block's)
         rc = select();
         if (rc != SABER_OK) return rc;
         CU(h, cudaMemcpyAsync(hc, ctr, 4, cudaMemcpyDeviceToHost, s));

@@ -202,7 +202,7 @@ struct saber_gpu {
     saber::DevBuf rg_qcnt, rg_qstart, rg_rank, rg_flag, rg_idx, rg_idx2, rg_out;
     // window plans and scoring of the regions (plan.cu)
     saber::DevBuf pl_key, pl_keyo, pl_idx, pl_by, pl_flag, pl_list, pl_span, pl_plan, pl_score, pl_floor, pl_ctr, pl_tmp,
-        pl_kept;
+        pl_kept, pl_ties;
     saber::HostBuf pin_kept;
     saber::HostBuf pin_scratch[4];  // the batch engine's staging (pinned_scratch)
     saber::DevBuf mask_runs;  // database mask runs being expanded
