@@ -390,17 +390,20 @@ typedef struct {
     uint64_t triage_dropped;      /* regions dropped by the learned triage */
     uint64_t band_scored_regions, band_rescored, banded_cells, score_launches;
     uint64_t alignments;
-    double t_prep_ms, t_scan_ms, t_triage_ms, t_plan_ms, t_score_ms, t_finish_ms, t_total_ms;  /* host wall clock */
-    /* inside t_score_ms: wall clock of the scoring calls (copies, kernels,
+    /* the parts of t_total_ms, host wall clock: scan to the capped regions, the
+     * learned triage (its features, network, cut and collection), the window
+     * plans' spans (device time), plans and scoring, E-values and tracebacks */
+    double t_prep_ms, t_scan_ms, t_triage_ms, t_plan_ms, t_score_ms, t_finish_ms, t_total_ms;
+    /* inside t_score_ms: wall clock of the scoring calls (kernels,
      * synchronisation) and the device time of their kernels */
     double t_score_calls_ms, t_score_device_ms;
     /* inside t_finish_ms: wall clock of the traceback calls */
     double t_finish_tb_ms;
     /* the scoring calls' device time by part (saber_score_stats) */
     double t_score_prep_ms, t_score_fast_ms, t_score_generic_ms;
-    /* host parts: inside t_score_ms, building the first-stage jobs and the
-     * second-stage decisions and jobs; inside t_finish_ms, the per-query
-     * E-value order */
+    /* inside t_score_ms, building the plans and first-stage jobs (device time;
+     * host wall clock in the exhaustive mode) and the second-stage decisions and
+     * jobs (host wall clock); inside t_finish_ms, the per-query E-value order */
     double t_score_build_ms, t_score_stage2_ms, t_finish_order_ms;
 } saber_search_stats;
 

@@ -390,6 +390,7 @@ struct Engine {
     int score_exhaustive(const std::vector<std::vector<Region>>& per_q, const std::vector<int64_t>& qlens,
                          std::vector<std::vector<Plan>>& plans, std::vector<std::vector<int64_t>>& scores) {
         const size_t nq = per_q.size();
+        const double t0 = now_ms();
         std::vector<size_t> base(nq + 1, 0);
         for (size_t qi = 0; qi < nq; qi++) base[qi + 1] = base[qi] + per_q[qi].size();
         const size_t n = base[nq];
@@ -407,6 +408,7 @@ struct Engine {
                 jobs[base[q] + ri] = job((uint32_t)q, r, lo, hi, -m, hi - lo);
             }
         });
+        st.t_score_build_ms += now_ms() - t0;
         const int32_t* sc = nullptr;
         int rc = score(jobs, n, 2, &sc);
         if (rc != SABER_OK) return rc;
@@ -812,7 +814,12 @@ extern "C" int saber_gpu_search(saber_gpu* h, const saber_search_params* params,
         rc = saber::scan_plan_score(h, &P.scan, q_mask, thr.data(), sink, &E.st.scan, E.plan_params(preps),
                                     floors.data(), rfloors.data(), tie, kept, &scan_ms);
         if (rc != SABER_OK) return rc;
-        t2 = t1 + scan_ms;
+        t2 = t1 + scan_ms + sink.triage_ms + kept.spans_ms;
+        E.st.t_triage_ms = sink.triage_ms;
+        E.st.t_plan_ms = kept.spans_ms;
+        E.st.t_score_build_ms = kept.jobs_ms;
+        E.st.t_score_stage2_ms = kept.stage2_ms;
+        E.st.t_score_calls_ms = kept.calls_ms;
         collecting = sink.collecting;
         if (sink.triaged) E.st.triage_dropped += sink.ncap - sink.n;
         E.st.regions += sink.n;
@@ -820,7 +827,6 @@ extern "C" int saber_gpu_search(saber_gpu* h, const saber_search_params* params,
         E.st.band_rescored += kept.n2;
         E.add_score_stats(kept.stage1);
         E.add_score_stats(kept.stage2);
-        E.st.t_score_calls_ms += now_ms() - t2;
         for (uint64_t t = 0; t < kept.n; t++) {
             const saber::KeptRegion& r = kept.kept[t];
             per_q[r.query].push_back({r.subject, r.d_min, r.d_max, r.best, r.src, r.sbase, (int64_t)r.slen});
@@ -845,7 +851,7 @@ extern "C" int saber_gpu_search(saber_gpu* h, const saber_search_params* params,
     *n_hits = nh;
     *n_ops = no;
     E.st.t_prep_ms = t1 - t0;
-    E.st.t_scan_ms = t2 - t1;
+    E.st.t_scan_ms = t2 - t1 - E.st.t_triage_ms - E.st.t_plan_ms;
     E.st.t_score_ms = t4 - t2;
     E.st.t_finish_ms = t5 - t4;
     E.st.t_total_ms = t5 - t0;

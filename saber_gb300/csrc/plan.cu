@@ -371,6 +371,8 @@ int plan_and_score(saber_gpu* h, const RegionSink& sk, const PlanParams& P, cons
                    const int64_t* region_floors, const PlanTie& tie, PlanResult& out) {
     out = PlanResult{};
     if (!sk.n) return SABER_OK;
+    for (cudaEvent_t& e : h->pl_ev)
+        if (!e) CU(h, cudaEventCreate(&e));
     const Dataset& ds = h->main;
     const QuerySet& qs = ds.qs;
     cudaStream_t s = h->stream;
@@ -418,6 +420,7 @@ int plan_and_score(saber_gpu* h, const RegionSink& sk, const PlanParams& P, cons
         return SABER_OK;
     };
     // spans of the pairs
+    CU(h, cudaEventRecord(h->pl_ev[0], s));
     k_plan_keys<<<grid, 256, 0, s>>>(reg, n, bs, key, idx);
     size_t tb = h->pl_tmp.cap;
     CU(h, cub::DeviceRadixSort::SortPairs(h->pl_tmp.p, tb, key, keyo, idx, by, (int)n, 0, bs + bq, s));
@@ -426,14 +429,23 @@ int plan_and_score(saber_gpu* h, const RegionSink& sk, const PlanParams& P, cons
     if (rc != SABER_OK) return rc;
     k_plan_spans<<<nblocks(n, 128, h->sm_count * 32), 128, 0, s>>>(reg, by, list, ctr, n, P.hsp_threshold,
                                                                    h->pl_span.as<int2>());
+    CU(h, cudaEventRecord(h->pl_ev[1], s));
     // stage 1
     rc = reserve_resident_jobs(h, n);
     if (rc != SABER_OK) return rc;
     k_plan_jobs<<<grid, 256, 0, s>>>(reg, h->pl_span.as<int2>(), n, qoffs, soffs, P, plan,
                                      h->jobs_dev.as<saber_band_job>(), reinterpret_cast<unsigned long long*>(ctr + 2));
     CU(h, cudaGetLastError());
+    CU(h, cudaEventRecord(h->pl_ev[2], s));
+    const double w0 = wall_ms();
     rc = score_resident_jobs(h, n, &out.stage1);
     if (rc != SABER_OK) return rc;
+    const double w1 = wall_ms();
+    float ms[2] = {0.f, 0.f};
+    for (int i = 0; i < 2; i++) CU(h, cudaEventElapsedTime(&ms[i], h->pl_ev[i], h->pl_ev[i + 1]));
+    out.spans_ms = ms[0];
+    out.jobs_ms = ms[1];
+    out.calls_ms = std::max(0.0, w1 - w0 - ms[0] - ms[1]);  // (the call's first wait is for the plans)
     // stage 2
     uint32_t* ties = by;  // (the group order is done with)
     k_plan_again<<<grid, 256, 0, s>>>(reg, plan, h->scores_dev.as<int32_t>(), n, qoffs, soffs, d_rfloor, P, score, flag,
@@ -469,12 +481,16 @@ int plan_and_score(saber_gpu* h, const RegionSink& sk, const PlanParams& P, cons
     }
     const uint32_t n2 = hc[0];
     out.n2 = n2;
+    out.stage2_ms = wall_ms() - w1;
     if (n2) {
         k_plan_jobs2<<<nblocks(n2, 256, h->sm_count * 32), 256, 0, s>>>(reg, plan, list, n2, soffs,
                                                                         h->jobs_dev.as<saber_band_job>());
         CU(h, cudaGetLastError());
+        const double w2 = wall_ms();
+        out.stage2_ms = w2 - w1;
         rc = score_resident_jobs(h, n2, &out.stage2);
         if (rc != SABER_OK) return rc;
+        out.calls_ms += wall_ms() - w2;
         k_plan_put<<<nblocks(n2, 256, h->sm_count * 32), 256, 0, s>>>(list, n2, h->scores_dev.as<int32_t>(), score);
     }
     // what finish may report

@@ -20,6 +20,7 @@ struct RegionSink {
     uint64_t ncap = 0;               // regions after the per-query cap
     bool triaged = false;            // a model dropped regions
     bool collecting = false;         // feature rows were collected
+    double triage_ms = 0;            // wall clock of the features, the network and its cut
 };
 
 // What planning and scoring the regions needs of the search's parameters and
@@ -54,6 +55,8 @@ struct PlanResult {
     uint64_t banded = 0;  // regions with a banded plan
     uint64_t n2 = 0;      // regions scored again
     saber_score_stats stage1{}, stage2{};
+    double spans_ms = 0, jobs_ms = 0;    // device time: the pairs' spans; plans and first-stage jobs
+    double calls_ms = 0, stage2_ms = 0;  // wall clock: the scoring calls; second-stage decisions and jobs
 };
 
 }  // namespace saber

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -203,6 +204,7 @@ struct saber_gpu {
     // window plans and scoring of the regions (plan.cu)
     saber::DevBuf pl_key, pl_keyo, pl_idx, pl_by, pl_flag, pl_list, pl_span, pl_plan, pl_score, pl_floor, pl_ctr, pl_tmp,
         pl_kept, pl_ties;
+    cudaEvent_t pl_ev[3] = {nullptr, nullptr, nullptr};  // start, spans, jobs (made on first use)
     saber::HostBuf pin_kept;
     saber::HostBuf pin_scratch[4];  // the batch engine's staging (pinned_scratch)
     saber::DevBuf mask_runs;  // database mask runs being expanded
@@ -298,6 +300,10 @@ int reserve_resident_jobs(saber_gpu* h, uint64_t njobs);
 int score_resident_jobs(saber_gpu* h, uint64_t njobs, saber_score_stats* st);
 int plan_and_score(saber_gpu* h, const RegionSink& sk, const PlanParams& P, const int64_t* floors,
                    const int64_t* region_floors, const PlanTie& tie, PlanResult& out);
+
+static inline double wall_ms() {
+    return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now().time_since_epoch()).count();
+}
 
 static inline unsigned nblocks(uint64_t n, unsigned t, unsigned cap = 65535u * 16u) {
     uint64_t b = (n + t - 1) / t;

@@ -8,7 +8,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <chrono>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -1556,15 +1555,16 @@ void* pinned_scratch(saber_gpu* h, int slot, size_t bytes) {
 
 // The batch's candidate regions for the host engine (engine.cpp): scanned,
 // capped per query, triaged, planned and scored on the device; those that may
-// be reported come back in pinned memory.  *scan_ms: the scan's share.
+// be reported come back in pinned memory.  *scan_ms: the scan's share, without
+// the triage's.
 int scan_plan_score(saber_gpu* h, const saber_scan_params* p, const uint8_t* q_mask, const int32_t* region_thr,
                     RegionSink& sink, saber_scan_stats* st, const PlanParams& pp, const int64_t* floors,
                     const int64_t* region_floors, const PlanTie& tie, PlanResult& out, double* scan_ms) {
     ENTER(h);
     uint64_t n = 0;
-    const auto t0 = std::chrono::steady_clock::now();
+    const double t0 = wall_ms();
     int rc = scan_regions(h, p, q_mask, region_thr, nullptr, 0, &n, st, &sink);
-    *scan_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    *scan_ms = wall_ms() - t0 - sink.triage_ms;
     if (rc != SABER_OK) return rc;
     return plan_and_score(h, sink, pp, floors, region_floors, tie, out);
 }
@@ -1626,6 +1626,8 @@ int saber_gpu_close(saber_gpu* h) {
         cudaStreamDestroy(h->copy_stream);
         if (h->copy_event) cudaEventDestroy(h->copy_event);
     }
+    for (cudaEvent_t e : h->pl_ev)
+        if (e) cudaEventDestroy(e);
     for (auto& g : h->graphs) cudaGraphExecDestroy(g.second.exec);
     h->graphs.clear();
     delete h;

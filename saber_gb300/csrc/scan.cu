@@ -1866,6 +1866,7 @@ static int region_sink(saber_gpu* h, const saber_scan_params* p, bool has_thr, u
     uint32_t nout = ncap;
     uint32_t* osrc = h->rg_idx2.as<uint32_t>();
     bool have_src = false;
+    const double triage0 = wall_ms();
     if (h->tr_on || h->tr_collect) {
         CUALLOC(h, h->tr_qinfo, std::max<uint64_t>(nq, 1) * sizeof(float4));
         if (nq)
@@ -1907,6 +1908,7 @@ static int region_sink(saber_gpu* h, const saber_scan_params* p, bool has_thr, u
             have_src = true;
             sk.triaged = true;
         }
+        sk.triage_ms = wall_ms() - triage0;
     }
     if (!have_src) k_iota<<<nblocks(nout, 256), 256, 0, s>>>(osrc, nout);
     CU(h, cudaGetLastError());
