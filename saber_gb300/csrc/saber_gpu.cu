@@ -474,6 +474,12 @@ static WaveArgs wave_args(const Scheme& sch, const Dataset& ds, const saber_band
 // First key bit that the sort looks at.  Without strip classes only the class
 // and the size in steps of 512 cells matter: four digit passes instead of eight.
 static int sort_from(bool strips) { return strips ? 0 : 36; }
+// Kernels of the sort of n keys from that bit on: one block's, which needs no
+// second copy of the keys among its `temp` bytes, or histogram, sum and digit
+// passes.
+static uint64_t sort_launches(uint64_t n, int key_from, size_t temp) {
+    return temp < n * 8 ? 1 : 2 + (64 - key_from + 7) / 8;
+}
 
 static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, const saber_band_job* d_jobs,
                           uint64_t njobs, int32_t* d_scores, saber_score_stats* st) {
@@ -538,7 +544,7 @@ static int score_pipeline(saber_gpu* h, const Scheme& sch, const Dataset& ds, co
     CU(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, tb, h->keys_in.as<uint64_t>(),
                                           h->keys_out.as<uint64_t>(), h->vals_in.as<uint32_t>(),
                                           h->vals_out.as<uint32_t>(), (int)n, key_from, 64, s));
-    local.library_launches += 1 + (64 - key_from) / 8;  // onesweep radix sort: histogram + digit passes
+    local.library_launches += sort_launches(n, key_from, t_sort);
 
     // one small read-back: class counts and widths size the scratch
     uint32_t hc[20];
@@ -847,7 +853,7 @@ static int score_pipeline_graph(saber_gpu* h, const Scheme& sch, const Dataset& 
         local.empty_jobs = hc[4];
         local.i16_rescored = hc[5] - hc[1];
         local.kernel_launches = strips ? 6 : 4;
-        local.library_launches = 1 + (64 - key_from) / 8;
+        local.library_launches = sort_launches(npad, key_from, t_sort);
         local.t_fast_ms = ms;
         local.prof8 = qs.p8 ? 1 : 0;
         *st = local;
