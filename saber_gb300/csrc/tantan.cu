@@ -694,10 +694,11 @@ int tantan_run(saber_gpu* h, const TantanModel& M, const uint8_t* d_codes, const
             // Shape by sequences per SM: two warps per block and eight rows in
             // flight while latency rules (one sequence's serial chain is the
             // launch), more warps and fewer rows in flight as the memory
-            // traffic takes over.  Calls of 2,400 / 20,000 / 40,000 / 100,000
-            // sequences on one GB300: two warps 0.86 / 1.42 / 2.75 / 6.8 ms,
-            // eight warps 1.06 / 1.49 / 1.84 / 4.2, twelve 1.31 / 1.82 / 2.18
-            // / 4.0.
+            // traffic takes over.  Resident databases of 16 / 116 / 131 / 145 /
+            // 180 / 380 / 420 / 658 sequences an SM on one GB300: two warps
+            // 0.82 / 1.19 / 1.31 / 1.46 / 1.79 / 3.70 / 4.08 / 6.39 ms, eight
+            // 1.03 / 1.37 / 1.38 / 1.42 / 1.49 / 2.20 / 2.40 / 3.75, twelve 1.28 /
+            // 1.72 / 1.74 / 1.75 / 1.83 / 2.28 / 2.37 / 3.58.
             auto go = [&](auto kern, unsigned warps) -> int {
                 const uint64_t per_block = (uint64_t)warps * kTgSeqs;
                 const unsigned blocks = (unsigned)((k1 - k0 + per_block - 1) / per_block);
@@ -708,7 +709,7 @@ int tantan_run(saber_gpu* h, const TantanModel& M, const uint8_t* d_codes, const
                 return SABER_OK;
             };
             const uint64_t per_sm = (k1 - k0) / (uint64_t)h->sm_count;
-            const int rc = per_sm < 128   ? go(k_tantan8<50, 8, 64, 2>, 2)
+            const int rc = per_sm < 140   ? go(k_tantan8<50, 8, 64, 2>, 2)
                            : per_sm < 400 ? go(k_tantan8<50, 4, 256, 2>, 8)
                                           : go(k_tantan8<50, 1, 384, 2>, 12);
             if (rc) return rc;
