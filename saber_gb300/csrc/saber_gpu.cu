@@ -372,19 +372,23 @@ __global__ void k_classify(const saber_band_job* __restrict__ jobs, uint64_t njo
 // and 11,000-query searches (30 k steps per lane) 131 / 65.0 / 64.1 / 64.1 /
 // 63.7 / 63.8 ms.
 constexpr uint64_t kLoadSmall = 1650;
-// Below kLoadPairs steps per lane the anti-diagonal kernel reads the small
-// int16 score table instead of the pair table: a batch of a few jobs is one
-// job's chain of steps long, and building the pair table (a launch per scheme,
-// which a call on a query's windows sets anew) and copying it into every
-// block only add to it.  A call on 40 windows (2 steps per lane) 250 us with
-// the int16 table, 255 with the pair table; 3,001 bands (24 steps) 268 and 250.
+// The anti-diagonal kernel reads the pair table where the scheme has one: a call
+// on 100 / 1,000 / 3,001 / 6,000 bands of half-widths 4..64 takes 147 / 186 / 230 /
+// 254 us with it and 160 / 187 / 239 / 262 with the int16 table, of 4..128 164 /
+// 181 / 244 / 282 and 191 / 227 / 307 / 326.  But score_windows sets its scheme
+// anew on every call, and the launch that builds the table adds to a small batch's
+// chain: 5 / 20 windows of 310 rows 231 / 817 us with the pair table, 228 / 811 with
+// the other, 400 of 100 rows 333 / 327.  Such a call takes it from kLoadPairs steps
+// per lane on, where the two are alike (200 and 400 windows of 310 rows, 16 and 32
+// steps: 1,228 / 1,217 us, 1,226 / 1,228).
 constexpr uint64_t kLoadPairs = 12;
 static uint64_t steps_per_lane(const saber_gpu* h, uint64_t cells) {
     const uint64_t lanes = (uint64_t)h->sm_count * band_fast_blocks_per_sm(h->strip_rows, false) * 256;
     return cells / 32 / (lanes ? lanes : 1);
 }
 static bool use_pairs(const saber_gpu* h, const Scheme& sch, uint64_t cells) {
-    return sch.pairs8 && (h->long_steps != kLongStepsAuto || steps_per_lane(h, cells) >= kLoadPairs);
+    const bool set_anew = &sch == &h->eph_scheme;
+    return sch.pairs8 && (!set_anew || h->long_steps != kLongStepsAuto || steps_per_lane(h, cells) >= kLoadPairs);
 }
 // Builds the scheme's pair table if this is its first use.
 static cudaError_t ensure_pairs(saber_gpu* h, const Scheme& sch) {
