@@ -1,6 +1,7 @@
-// Banded affine-gap Smith-Waterman, one job on 8, 9, 16 or 32 lanes (int16
-// pairs): the jobs whose sweep in one lane of k_band_fast would outlast the
-// rest of the batch, and narrow bands.  Semantics as in band_kernels.cu.
+// Banded affine-gap Smith-Waterman, one job on 8, 9, 16 or 32 lanes, or on a
+// block's 128 (int16 pairs): the jobs whose sweep in one lane of k_band_fast
+// would outlast the rest of the batch, and narrow bands.  Semantics as in
+// band_kernels.cu.
 //
 // The band is swept along anti-diagonals s = 2 i + k of its (row i, band
 // index k = j - i - lo) coordinates.  A lane holds 4 J consecutive band

@@ -285,13 +285,6 @@ struct HitRec {
     std::vector<uint32_t> runs;
 };
 
-inline void band_clip(int64_t& lo, int64_t& hi, int64_t m, int64_t n) {
-    lo = std::max(lo, -(m - 1));
-    hi = std::min(hi, n - 1);
-}
-inline bool band_covers(int64_t lo, int64_t hi, int64_t m, int64_t n) { return lo <= -(m - 1) && hi >= n - 1; }
-inline int64_t band_width(int64_t lo, int64_t hi) { return std::max<int64_t>(hi - lo + 1, 0); }
-
 struct Engine {
     saber_gpu* h;
     const saber_search_params& P;
@@ -410,7 +403,7 @@ struct Engine {
         });
         st.t_score_build_ms += now_ms() - t0;
         const int32_t* sc = nullptr;
-        int rc = score(jobs, n, 2, &sc);
+        int rc = score(jobs, n, 1, &sc);
         if (rc != SABER_OK) return rc;
         for (size_t q = 0; q < nq; q++) scores[q].assign(sc + base[q], sc + base[q + 1]);
         return SABER_OK;

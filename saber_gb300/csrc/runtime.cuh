@@ -206,7 +206,7 @@ struct saber_gpu {
         pl_kept, pl_ties;
     cudaEvent_t pl_ev[3] = {nullptr, nullptr, nullptr};  // start, spans, jobs (made on first use)
     saber::HostBuf pin_kept;
-    saber::HostBuf pin_scratch[4];  // the batch engine's staging (pinned_scratch)
+    saber::HostBuf pin_scratch[2];  // the batch engine's staging (pinned_scratch)
     saber::DevBuf mask_runs;  // database mask runs being expanded
     // six-frame translation scratch
     saber::DevBuf tr_nt, tr_offs, tr_out_offs, tr_chunks, tr_aa, tr_out;

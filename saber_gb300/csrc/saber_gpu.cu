@@ -1558,7 +1558,7 @@ int translate6_host(saber_gpu* h, const uint8_t* nt, const uint64_t* nt_offsets,
                     const uint8_t* codon64, uint8_t* out, uint64_t out_cap, uint64_t* out_offsets);
 // Pinned host staging for the host engine (engine.cpp).
 void* pinned_scratch(saber_gpu* h, int slot, size_t bytes) {
-    if (!h || slot < 0 || slot >= 4) return nullptr;
+    if (!h || slot < 0 || slot >= 2) return nullptr;
     cudaSetDevice(h->device);
     return h->pin_scratch[slot].reserve(std::max<size_t>(bytes, 64)) == cudaSuccess ? h->pin_scratch[slot].p : nullptr;
 }

@@ -195,9 +195,7 @@ static int tantan_model(saber_gpu* h, const int32_t* m, const saber_tantan_param
 // ((a0+a1)+(a2+a3))+((a4+a5)+(a6+a7)) in lane 0 (IEEE addition commutes, so
 // the partner order within each pair does not matter), then the remaining
 // w mod 8 states are added one at a time.  Every lane returns the sum.
-template <int WC>
-__device__ __forceinline__ float tt_sum8(float v0, float v1, int wrt) {
-    const int w = WC ? WC : wrt;
+__device__ __forceinline__ float tt_sum8(float v0, float v1, int w) {
     const int chunks = w >> 3;
     float acc = 0.f;
     if (chunks > 0) {
@@ -226,7 +224,6 @@ __device__ __forceinline__ float tt_sum8(float v0, float v1, int wrt) {
 // One warp per sequence (ord[k] for k in [k0, k1)); base[k] is the sequence's
 // first scratch row.  Writes mask[offs[sid] + p] (and probs when non-null) and
 // adds the masked positions to *n_masked.
-template <int WC>  // repeat states when fixed at compile time (0: M.w)
 __global__ void __launch_bounds__(kTtWarps * 32, 4) k_tantan(const __grid_constant__ TantanModel M,
                                                           const uint8_t* __restrict__ codes,
                                                           const uint64_t* __restrict__ offs,
@@ -248,7 +245,7 @@ __global__ void __launch_bounds__(kTtWarps * 32, 4) k_tantan(const __grid_consta
     const uint8_t* x = codes + st;
     float* F = fwdF + base[k] * (uint64_t)kTtMaxW;
     float2* BS = fwdBS + base[k];
-    const int w = WC ? WC : M.w;
+    const int w = M.w;
     const float b2f0 = M.b2f[lane], b2f1 = M.b2f[lane + 32];
     const float b2b = M.b2b, f2f = M.f2f, f2b = M.f2b;
 
@@ -265,11 +262,11 @@ __global__ void __launch_bounds__(kTtWarps * 32, 4) k_tantan(const __grid_consta
         }
         const int xp = __shfl_sync(kFull, cw, j);
         const float e0 = lr[xp * 32 + h0], e1 = lr[xp * 32 + h1];
-        const float sum_f = tt_sum8<WC>(pf0, pf1, w);
+        const float sum_f = tt_sum8(pf0, pf1, w);
         const float c0 = __fmul_rn(__fadd_rn(__fmul_rn(pb, b2f0), __fmul_rn(pf0, f2f)), e0);
         const float c1 = __fmul_rn(__fadd_rn(__fmul_rn(pb, b2f1), __fmul_rn(pf1, f2f)), e1);
         const float cb = __fadd_rn(__fmul_rn(pb, b2b), __fmul_rn(sum_f, f2b));
-        const float tot = __fadd_rn(cb, tt_sum8<WC>(c0, c1, w));
+        const float tot = __fadd_rn(cb, tt_sum8(c0, c1, w));
         const float s = tot > 0.f ? __fdiv_rn(1.f, tot) : 1.f;
         pb = __fmul_rn(cb, s);
         pf0 = __fmul_rn(c0, s);
@@ -325,14 +322,14 @@ __global__ void __launch_bounds__(kTtWarps * 32, 4) k_tantan(const __grid_consta
         const float onb = nb, onf0 = nf0, onf1 = nf1;
         if (p > 0) {
             const float be0 = __fmul_rn(lr[xp * 32 + g0], onf0), be1 = __fmul_rn(lr[xp * 32 + g1], onf1);
-            const float to_fg = tt_sum8<WC>(__fmul_rn(b2f0, be0), __fmul_rn(b2f1, be1), w);
+            const float to_fg = tt_sum8(__fmul_rn(b2f0, be0), __fmul_rn(b2f1, be1), w);
             const float fb = __fmul_rn(f2b, onb);
             nf0 = __fmul_rn(__fadd_rn(__fmul_rn(f2f, be0), fb), s);
             nf1 = __fmul_rn(__fadd_rn(__fmul_rn(f2f, be1), fb), s);
             nb = __fmul_rn(__fadd_rn(__fmul_rn(b2b, onb), to_fg), s);
         }
         const float pbv = __fmul_rn(rb, onb);
-        const float pfv = tt_sum8<WC>(__fmul_rn(r0, onf0), __fmul_rn(r1, onf1), w);
+        const float pfv = tt_sum8(__fmul_rn(r0, onf0), __fmul_rn(r1, onf1), w);
         const float z = __fadd_rn(pbv, pfv);
         const float post = z > 0.f ? __fdiv_rn(pfv, z) : 0.f;
         if (lane == j) keep = post;
@@ -717,7 +714,7 @@ int tantan_run(saber_gpu* h, const TantanModel& M, const uint8_t* d_codes, const
             continue;
         }
         const unsigned blocks = (unsigned)((k1 - k0 + kTtWarps - 1) / kTtWarps);
-        k_tantan<0><<<blocks, kTtWarps * 32, 0, h->stream>>>(
+        k_tantan<<<blocks, kTtWarps * 32, 0, h->stream>>>(
             M, d_codes, d_offs, (const uint32_t*)h->tt_ord.p, (const uint64_t*)h->tt_base.p, k0, k1,
             (float*)h->tt_F.p, (float2*)h->tt_BS.p, d_mask, d_probs, (unsigned long long*)h->tt_count.p);
         CU(h, cudaGetLastError());
