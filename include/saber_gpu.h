@@ -62,8 +62,9 @@ typedef struct {
     uint64_t jobs;            /* jobs scored */
     uint64_t banded_cells;    /* in-band cells, counted as banded.rs:123-131 */
     uint64_t fast_cells;      /* the part of banded_cells in jobs of the packed int16 kernels */
-    uint64_t fast_jobs;       /* jobs taken by the packed int16 kernels (strips and anti-diagonals) */
-    uint64_t generic_jobs;    /* the other jobs: narrow bands, and bands scored directly in int32 */
+    uint64_t fast_jobs;       /* bands of 8 and more taken by the packed int16 kernels (strips and anti-diagonals) */
+    uint64_t generic_jobs;    /* the other jobs: narrower bands (scored by the anti-diagonal kernel), and
+                                 bands scored directly in int32 */
     uint64_t i16_rescored;    /* int16 results at the overflow limit, rescored in int32 */
     uint64_t empty_jobs;      /* empty band / window / query: score 0 */
     uint64_t kernel_launches; /* this library's own kernels launched by the call */

@@ -146,8 +146,8 @@ __global__ void k_region_feats(RegionFeatArgs a) {
 // matrix.  The weight gradients contract over the batch's rows: the rows are
 // split over blockIdx.z, each split writes its own partial gradient, and
 // k_sum_splits adds them (2,048 rows: 16 splits x 16 tiles instead of 16
-// blocks walking all rows).  A call of 2,048 rows takes six launches and 154
-// us on one GB300 (fourteen launches and 1.49 ms with one block per output
+// blocks walking all rows).  A call of 2,048 rows takes eight launches and 141
+// us on one GB300 (sixteen launches and 1.49 ms with one block per output
 // tile, separate column sums and buffers allocated per call); its error
 // against 64 bits fell from 6e-7 to 8e-8.
 constexpr int kBT = 64, kBK = 32, kPitch = kBT + 4;

@@ -587,7 +587,7 @@ class Device:
 
     @property
     def long_steps(self):
-        """Lane-sweep length (column steps) above which a job goes to the warp-per-job kernel."""
+        """Lane-sweep length (column steps) above which a job leaves the strip kernel's lanes."""
         return int(self.lib.saber_gpu_get_long_steps(self.h))
 
     @long_steps.setter

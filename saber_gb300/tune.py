@@ -15,7 +15,8 @@ never results:
   one job) instead of a lane of the strip kernel; the default picks it per
   call from the batch's in-band cells per lane (the power of two at or above
   1.25 times a lane's even share of the sweep steps, at least 2048; a batch
-  of less than 1,650 steps per lane goes there as a whole).
+  of less than 1,650 steps per lane goes there as a whole, and one of bands
+  wide for their queries' lengths takes 4 times the share).
 
 `autotune_scoring` times settings on the caller's own batch (the
 device-resident entry point, same stream) by coordinate descent: starting
