@@ -130,7 +130,7 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
     return a + (b << 22) + (c << 44);
 }
 
-__global__ void k_job_load(const saber_band_job* __restrict__ jobs, uint64_t njobs,
+__global__ void __launch_bounds__(256) k_job_load(const saber_band_job* __restrict__ jobs, uint64_t njobs,
                            const uint64_t* __restrict__ qoffs, uint32_t nq, int R, uint32_t pair_steps,
                            unsigned long long* __restrict__ out) {
     uint32_t mx[3] = {};
@@ -158,22 +158,25 @@ __global__ void k_job_load(const saber_band_job* __restrict__ jobs, uint64_t njo
             sum[1] += (uint64_t)nit * wave_slots(wave_class(w));
         }
     }
-    __shared__ unsigned long long b[6];
-    if (threadIdx.x < 6) b[threadIdx.x] = 0;
-    __syncthreads();
+    // block totals by way of a row per warp (64-bit atomics in shared memory are
+    // loops), then one global atomic per member and block
+    __shared__ unsigned long long b[8][6];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         const uint32_t most = __reduce_max_sync(0xffffffffu, mx[k]);
         const unsigned long long total = warp_sum(sum[k]);
         if ((threadIdx.x & 31) == 0) {
-            atomicMax(&b[k], (unsigned long long)most);
-            atomicAdd(&b[3 + k], total);
+            b[threadIdx.x >> 5][k] = most;
+            b[threadIdx.x >> 5][3 + k] = total;
         }
     }
     __syncthreads();
-    if (threadIdx.x < 3) {
-        atomicMax(out + threadIdx.x, b[threadIdx.x]);
-        atomicAdd(out + 3 + threadIdx.x, b[3 + threadIdx.x]);
+    if (threadIdx.x < 6) {
+        unsigned long long v = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) v = threadIdx.x < 3 ? max(v, b[w][threadIdx.x]) : v + b[w][threadIdx.x];
+        if (threadIdx.x < 3) atomicMax(out + threadIdx.x, v);
+        else atomicAdd(out + threadIdx.x, v);
     }
 }
 
