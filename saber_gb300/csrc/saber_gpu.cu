@@ -385,10 +385,10 @@ constexpr uint64_t kLoadSmall = 1650;
 // per lane on, where the two are alike (200 and 400 windows of 310 rows, 16 and 32
 // steps: 1,228 / 1,217 us, 1,226 / 1,228).
 constexpr uint64_t kLoadPairs = 12;
-static uint64_t steps_per_lane(const saber_gpu* h, uint64_t cells) {
-    const uint64_t lanes = (uint64_t)h->sm_count * band_fast_blocks_per_sm(h->strip_rows, false) * 256;
-    return cells / 32 / (lanes ? lanes : 1);
+static uint64_t strip_lanes(const saber_gpu* h) {
+    return std::max<uint64_t>(1, (uint64_t)h->sm_count * band_fast_blocks_per_sm(h->strip_rows, false) * 256);
 }
+static uint64_t steps_per_lane(const saber_gpu* h, uint64_t cells) { return cells / 32 / strip_lanes(h); }
 static bool use_pairs(const saber_gpu* h, const Scheme& sch, uint64_t cells) {
     const bool set_anew = &sch == &h->eph_scheme;
     return sch.pairs8 && (!set_anew || h->long_steps != kLongStepsAuto || steps_per_lane(h, cells) >= kLoadPairs);
@@ -425,15 +425,15 @@ static cudaError_t ensure_pairs(saber_gpu* h, const Scheme& sch) {
 constexpr uint64_t kWideCell = 48;
 static LongSteps long_steps_for(const saber_gpu* h, const JobLoad& l) {
     if (h->long_steps != kLongStepsAuto) return {h->long_steps, h->long_steps};
-    const uint64_t load = steps_per_lane(h, l.cells);
+    const uint64_t step = 32 * strip_lanes(h), load = l.cells / step;  // (step: cells of a step of all lanes)
     auto power = [](uint64_t least) {
         uint64_t t = kLongStepsSmall;
         while (t < least && t < (1ull << 30)) t <<= 1;
         return t;
     };
     const uint64_t most = power(4 * load), usual = load < kLoadSmall ? 0 : power(load + load / 4);
-    const bool narrow = steps_per_lane(h, l.wave) > std::min<uint64_t>(l.sweep, most);
-    const bool wide = steps_per_lane(h, l.wide * kWideCell) > std::min<uint64_t>(l.wide_sweep, most);
+    const bool narrow = l.wave / step > std::min<uint64_t>(l.sweep, most);
+    const bool wide = l.wide * kWideCell / step > std::min<uint64_t>(l.wide_sweep, most);
     return {(uint32_t)(narrow ? most : usual), (uint32_t)(wide ? most : usual)};
 }
 // The strip classes can hold jobs.
